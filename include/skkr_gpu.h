@@ -66,8 +66,7 @@ typedef struct {
   int precision;                  /* skkr_precision */
   int nk_chunk;                   /* k points per device batch (0: automatic) */
   int slices;                     /* SKKR_MIXED: BF16 slices per product operand, 3..8 (0: 6).
-                                     Digits are 8-bit for a product depth K <= 128 (8 slices act
-                                     as 7), 7-bit above.  SKKR_BDG splits every product into its
+                                     Digits are 8-bit for a product depth K <= 128, 7-bit above.  SKKR_BDG splits every product into its
                                      electron and hole K halves, each with its own scales */
 } skkr_sizes;
 
@@ -125,9 +124,8 @@ int skkr_gpu_destroy(skkr_ctx *ctx);
 /* Split-precision policy near the real axis, where the lead and slab
  * matrices become ill-conditioned and rounding of the products is amplified
  * by their condition number: decimation runs in FP64 when |Im E| < dec_fp64_im
- * (default 2e-4 Ry); the products use slices_near BF16 slices on the
- * exact-level tile when |Im E| < near_im (defaults 7 slices below 1e-3 Ry;
- * 3..8, 0 = off);
+ * (default 2e-4 Ry); the products use slices_near BF16 slices when
+ * |Im E| < near_im (defaults 7 slices below 1e-3 Ry; 3..8, 0 = off);
  * every k point whose contribution exceeds dominant_frac (default 1e-2) of
  * the norm of the k-summed tau, and ten times the mean contribution of a k
  * point (an isolated peak), is recomputed in FP64 (0 = off).  Inverses
@@ -153,7 +151,7 @@ int skkr_gpu_set_newton(skkr_ctx *ctx, int steps);
  * Newton steps, their acceptance test and the FP64 redo are the same. */
 int skkr_gpu_set_inverse_start(skkr_ctx *ctx, int blocked);
 
-/* The B operand of every split-precision product on the default tile: on
+/* The B operand of every split-precision product: on
  * != 0 (the default) the product reads B in FP64 and forms its BF16 slices in
  * shared memory, tile by tile, with the warps that later run the epilogue; 0
  * splits B into a staging buffer first and loads its tiles by TMA.  Both give

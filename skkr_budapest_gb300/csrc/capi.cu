@@ -1587,7 +1587,6 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
   }
   if (c->mw) {
     CKR(mixed_resid_reset(c->mw, st));
-    mixed_set_precise(c->mw, c->slices_near > 0 && std::fabs(c->ce.y) < c->near_im);
     mixed_set_fused(c->mw, c->fused_b != 0);
   }
   plan_pack(c);
@@ -1616,7 +1615,7 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
     double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + (5.0 * c->nprc + 1) * ng) +
                    (double)nc * ni * ni * lk2 * sizeof(zd);
     if (c->sz.precision == SKKR_MIXED) {
-      const double Mp = 128.0 * ((n + 127) / 128), Np = 96.0 * ((2 * n + 95) / 96), Kp = 32.0 * ((2 * n + 31) / 32);
+      const double Mp = 128.0 * ((n + 127) / 128), Np = 64.0 * ((2 * n + 63) / 64), Kp = 32.0 * ((2 * n + 31) / 32);
       per_k += (double)ncmax * MIXED_SLOTS * c->slices_res * (Mp + Np) * Kp * 2.0;
     }
     kc = c->sz.nk_chunk > 0 ? c->sz.nk_chunk : (int)std::max(1.0, std::floor(32.0e9 / per_k));
@@ -1834,8 +1833,6 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   }
   if (c->mw) {
     CKR(mixed_resid_reset(c->mw, st));
-    // near the real axis the products also run on the exact-level tile
-    mixed_set_precise(c->mw, c->slices_near > 0 && std::fabs(c->ce.y) < c->near_im);
     mixed_set_fused(c->mw, c->fused_b != 0);
   }
   plan_pack(c);
@@ -1850,9 +1847,9 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
                    (double)c->ngeff * ni * lk2 * sizeof(zd);
     if (use_mixed(c, false)) {
       // BF16 slice staging: up to MIXED_SLOTS operands per side, S slices of
-      // the padded real embedding (A: 128-row tiles, B: 96-row tiles, K: 2n);
+      // the padded real embedding (A: 128-row tiles, B: 64-row tiles, K: 2n);
       // an energy that runs wholly in FP64 stages nothing
-      const double Mp = 128.0 * ((n + 127) / 128), Np = 96.0 * ((2 * n + 95) / 96),
+      const double Mp = 128.0 * ((n + 127) / 128), Np = 64.0 * ((2 * n + 63) / 64),
                    Kp = 32.0 * ((2 * n + 31) / 32);
       per_k += (double)ncmax * MIXED_SLOTS * c->slices_res * (Mp + Np) * Kp * 2.0;
     }

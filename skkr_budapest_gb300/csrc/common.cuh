@@ -52,11 +52,14 @@ struct MatRef {
 
 // (the map entry by static selects: a dynamic index into a kernel
 // parameter's array would copy the whole MatRef to the thread's stack)
-__device__ inline zd *mat_ptr(const MatRef &m, int k, int c) {
+__device__ inline int map_at(const MatRef &m, int c) {
   int mc = 0;
 #pragma unroll
   for (int i = 0; i < SKKR_MAPN; i++) mc = i == c ? m.map[i] : mc;
-  return m.base + (long long)k * m.sk + (long long)mc * m.sc;
+  return mc;
+}
+__device__ inline zd *mat_ptr(const MatRef &m, int k, int c) {
+  return m.base + (long long)k * m.sk + (long long)map_at(m, c) * m.sc;
 }
 
 // host-side constructors

@@ -109,9 +109,6 @@ constexpr int NEWTON_EXTRA = 4;
 // that several products read is split once into its slot instead
 int mixed_split(MixedWork *w, int side, int slot, int S, const MatRef &M, int n, int K, int nk, int nc,
                 const int *act, cudaStream_t st, bool reused = false);
-// products of 6+ slices on 64-column tiles with 7 TMEM accumulators (levels
-// 0..5 exact): rounding below FP64's, for ill-conditioned energies
-void mixed_set_precise(MixedWork *w, bool on);
 // the 2 x 2 block FP32 start of inverses above 64 rows (default on)
 void mixed_set_blocked(MixedWork *w, bool on);
 // B operands formed by the products themselves (default on)

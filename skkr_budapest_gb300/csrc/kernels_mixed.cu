@@ -14,9 +14,10 @@
 // its own TMEM accumulator: the tensor core aligns addends to the largest
 // exponent and truncates, so sums of one level stay exact (integer multiples
 // of the level's unit, at most (c+1) K 2^14 units, within FP32's 24 bits for
-// K <= 256) whereas mixing levels would drop the low bits of the smaller one.
-// Products with p+q > S+1 are dropped; S = 5 keeps 15 products in 5 levels
-// (5 x 96 TMEM columns) and gives about 2^-39 relative to sigma_i tau_j.
+// K <= 256 and c <= 3) whereas mixing levels would drop the low bits of the
+// smaller one.  Products with p+q > S+1 are dropped: S slices keep S(S+1)/2
+// products in S levels (S x 64 TMEM columns) and give about 2^-8S relative to
+// sigma_i tau_j.
 //
 // Complex to real: [Cr Ci] = [Ar Ai] [[Br Bi], [-Bi Br]], i.e. a real GEMM of
 // M = n, N = 2n, K' = 2K.  The real depth K' runs over groups of 16 complex
@@ -27,12 +28,11 @@
 // Staging layouts (bf16, K-major for both UMMA operands, tiled by k-block so
 // that one TMA box is one contiguous block):
 //   A'[item][s][kb][M'][32]   M' = 128 * mtiles, kb < kblocks = ceil(K/16)
-//   B'[item][s][kb][N'][32]   N' = TN * ntiles (zero padded; TN = 96, or 64
-//                                 for the exact-level tile)
+//   B'[item][s][kb][N'][32]   N' = 64 * ntiles (zero padded)
 // A tiles reach shared memory by TMA (3-D tensor maps, 64-byte swizzle).  B
-// tiles either the same way from B' or, fused, straight from the FP64 B: the
-// ten warps that run the epilogue form each stage's B slices in shared
-// memory while the tensor core works on the previous stage.
+// tiles either the same way from B' or, fused, straight from the FP64 B: TMA
+// brings its values into a ring of shared memory and converting warps form
+// the slices beside the tensor core.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -51,18 +51,45 @@
 
 namespace {
 
-constexpr int NT = 96;            // N tile (TMEM columns per accumulator)
+constexpr int NT = 64;            // N tile (TMEM columns per accumulator)
 constexpr int MT = 128;           // M tile (UMMA M)
 constexpr int KB = 32;            // K per k-block (one 64-byte swizzle row of bf16)
 constexpr int OZ_SMEM_MAX = 232448;  // shared memory one CTA may use (opt-in)
-// shared-memory pipeline stages of the sliced GEMM: three where three stages
-// of S A tiles and S B tiles fit (S <= 5 at the 96-column tile), else two
-__host__ __device__ constexpr int oz_stages(int S, int TN) {
-  return 3 * S * (128 * 32 * 2 + TN * 32 * 2) + 1024 <= OZ_SMEM_MAX ? 3 : 2;
+constexpr int OZ_A_SLICE = MT * KB * 2, OZ_B_SLICE = NT * KB * 2;  // bytes of one slice's A / B tile of a k-block
+// accumulator sets: up to four slices (4 x 64 columns) leave room for a second
+// set, so that one tile's MMAs run while the previous tile's sums are read
+__host__ __device__ constexpr int oz_bufs(int S) { return S <= 4 ? 2 : 1; }
+// Shared memory of S slices: a ring of A k-blocks (TMA), one of B k-blocks
+// (TMA, or formed here: fused) and, fused, one of FP64 k-blocks of B, the raw
+// values the conversion reads (32 columns of 16 values, as two TMA boxes of
+// eight values = 128 bytes per column, 128-byte swizzle).
+constexpr int OZ_RAW_BYTES = (NT / 2) * 16 * 16;
+constexpr int OZ_SMEM_RINGS = OZ_SMEM_MAX - 1024 - 4096;  // alignment, OzShared
+__host__ __device__ constexpr int oz_min(int a, int b) { return a < b ? a : b; }
+__host__ __device__ constexpr int oz_a_stages(int S, bool fused) {
+  return !fused ? oz_min(6, OZ_SMEM_RINGS / (S * (OZ_A_SLICE + OZ_B_SLICE))) : S <= 3 ? 4 : S <= 6 ? 3 : 2;
 }
-constexpr int NACC = 5;           // TMEM accumulators: one per level p+q = 0..4
+__host__ __device__ constexpr int oz_b_stages(int S, bool fused) {
+  return !fused ? oz_a_stages(S, false) : S <= 3 ? 4 : S == 4 ? 3 : 2;
+}
+__host__ __device__ constexpr int oz_ring_bytes(int S, bool fused) {
+  return S * (oz_a_stages(S, fused) * OZ_A_SLICE + oz_b_stages(S, fused) * OZ_B_SLICE);
+}
+__host__ __device__ constexpr int oz_raw_stages(int S) {
+  return oz_min(8, (OZ_SMEM_RINGS - oz_ring_bytes(S, true)) / OZ_RAW_BYTES);
+}
 constexpr long long WAIT_LIMIT = 1LL << 22;
-constexpr int OZ_THREADS = 384;   // 12 warps: producer and MMA lanes in warps 0-1, all 12 run the epilogue
+// The TMA lane of A (warp 0), the MMA lane (warp 1), the column scales (warp
+// 2), the TMA lane of B's raw values (warp 3), the epilogue (warps 4-11) and
+// the conversion of B: one group of four warps (16 warps in all, 128 registers
+// a thread), or two groups taking alternate k-blocks where the epilogue does
+// with 96 registers (up to four slices: few MMAs per k-block, so that the
+// conversion sets the pace).
+constexpr int OZ_EPI0 = 4, OZ_EPI_WARPS = 8, OZ_CONV0 = 12;
+__host__ __device__ constexpr int oz_conv_groups(int S) { return S <= 4 ? 2 : 1; }
+__host__ __device__ constexpr int oz_threads(int S) { return 32 * (OZ_CONV0 + 4 * oz_conv_groups(S)); }
+constexpr int OZ_SCALE_RING = 4;  // tiles the column scales may run ahead of the conversion
+constexpr int OZ_EXP_RING = 16;   // tiles whose column scales are kept
 
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -102,6 +129,23 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *tm, in
       "l"((uint64_t)tm), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
       : "memory");
 }
+// a load that the compiler keeps in program order (a batch of them is then in
+// flight together)
+__device__ __forceinline__ uint32_t load_u32(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *tm, int c0, int c1, int c2, int c3,
+                                            uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::
+          "r"(smem_u32(dst)),
+      "l"((uint64_t)tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+      : "memory");
+}
+// the 128-byte line of p towards L2
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // bytes (a multiple of 16, 16-byte aligned) of global memory towards L2
 __device__ __forceinline__ void bulk_prefetch_l2(const void *p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -136,16 +180,19 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// 16 consecutive accumulator columns of this warp's 32 TMEM lanes, without
+// 8 / 4 consecutive accumulator columns of this warp's 32 TMEM lanes, without
 // the wait (tmem_ld_wait after a batch of loads)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-        "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -337,8 +384,7 @@ __global__ void __launch_bounds__(256, 3) k_split_b(MatRef B, int n, int K, int 
 // ------------------------------------------------------------------ the GEMM
 struct OzArgs {
   int n, mtiles, ntiles, kblocks, nc, mode;
-  int eoff;             // 32 + 2 (DB - 1): result = acc 2^(sigma_i + tau_j - eoff), acc in 2^-16 units
-  int db;               // digit bits DB
+  int tiles;            // items x mtiles x ntiles
   const int *sigma;     // [item][M']  row scale exponents of A
   const int *tau;       // [item][n]   column scale exponents of B (staged B)
   MatRef B;             // the FP64 K x n operand B (fused B)
@@ -348,55 +394,53 @@ struct OzArgs {
   int *err;
 };
 
-// FP32 accumulator value -> int64 in units of 2^-16 (bit manipulation only).
-// Levels 0..3 hold exact multiples of 2^(16-DB l) >= 2^-8; the shared tail
-// level is truncated at 2^-16, about 2^-53 below the leading level.
-// exact level l <= 3 (its FP32 accumulator holds an integer N times
-// 2^(16 - DB l), |N| < 2^24) in the same 2^-16 units: N from one conversion,
-// then a shift (32 - DB l >= 0 for l <= 3); the result equals f2fix16(v)
-__device__ __forceinline__ long long level_fix16(float v, int l, int db) {
-  const int n = __float2int_rn(v * pow2f(db * l - 16));
-  return (long long)n << (32 - db * l);
+// The exact integer sum of one level, from its FP32 accumulator (integer
+// times 2^(16 - DB l))
+template <int DB>
+__device__ __forceinline__ int level_int(uint32_t v, int l) {
+  return __float2int_rn(__uint_as_float(v) * pow2f(DB * l - 16));
 }
-__device__ __forceinline__ long long f2fix16(float v) {
-  const int b = __float_as_int(v);
-  const int ex = (b >> 23) & 0xFF;
-  if (ex == 0) return 0;
-  const long long mant = (b & 0x7FFFFF) | 0x800000;
-  const int sh = ex - 150 + 16;
-  const long long m = sh >= 0 ? (mant << sh) : (sh > -31 ? (mant >> -sh) : 0);
-  return b < 0 ? -m : m;
+// The weighted sum of the S levels of one output in units of level
+// min(S - 1, 5) (weight 2^(-5 DB) of level 0 at most: 62 bits hold it, as
+// |N_0| <= 2^22); deeper levels are rounded into that unit.  32 x 32 + 64 bit
+// multiply-adds with constant powers of two.
+template <int S, int DB, int W>
+__device__ __forceinline__ long long levels_sum(const uint32_t (&v)[S][W], int t) {
+  constexpr int B1 = 1 << DB, B2 = 1 << (2 * DB);
+  const long long hi = (long long)level_int<DB>(v[0][t], 0) * B2 +
+                       ((long long)level_int<DB>(v[1][t], 1) * B1 + level_int<DB>(v[2][t], 2));
+  if constexpr (S == 3) return hi;
+  if constexpr (S == 4) return hi * B1 + level_int<DB>(v[3][t], 3);
+  if constexpr (S == 5)
+    return hi * B2 + ((long long)level_int<DB>(v[3][t], 3) * B1 + level_int<DB>(v[4][t], 4));
+  if constexpr (S >= 6) {
+    long long lo = (long long)level_int<DB>(v[3][t], 3) * B2 +
+                   ((long long)level_int<DB>(v[4][t], 4) * B1 + level_int<DB>(v[5][t], 5));
+    if constexpr (S == 7) lo += (level_int<DB>(v[6][t], 6) + B1 / 2) >> DB;
+    if constexpr (S == 8)
+      lo += ((long long)level_int<DB>(v[6][t], 6) * B1 + level_int<DB>(v[7][t], 7) + B2 / 2) >> (2 * DB);
+    return (hi << (3 * DB)) + lo;
+  }
 }
 // round-to-nearest-even double of a * 2^e from integer operations only (the
 // FP64 pipe of this GPU is ~1/40 of the integer rate): normalise with a
 // leading-zero count, keep 53 bits, round on the dropped 11, add e to the
-// exponent.  Equal to __ll2double_rn(a) * 2^e for normal results.
+// exponent (the leading one and a carry of the rounding add into the exponent
+// field).  Equal to __ll2double_rn(a) * 2^e for normal results; a result
+// below the normal range is 0, one above it infinite.
 __device__ __forceinline__ double fix_to_double(long long a, int e) {
-  if (a == 0) return 0.0;
-  const unsigned long long sign = a < 0 ? 0x8000000000000000ull : 0ull;
+  const unsigned long long sign = (unsigned long long)a & 0x8000000000000000ull;
   unsigned long long m = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
   const int lz = __clzll((long long)m);
-  m <<= lz;                                    // leading one at bit 63
+  m <<= (lz & 63);                             // leading one at bit 63
   unsigned long long mant = m >> 11;           // 53 significant bits
-  const unsigned long long rem = m & 0x7FFull;
-  int ex = 63 - lz + e;
-  mant += (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) ? 1ull : 0ull;
-  if (mant >> 53) {                            // rounding carried into bit 53
-    mant >>= 1;
-    ex++;
-  }
-  return __longlong_as_double((long long)(sign | ((unsigned long long)(ex + 1023) << 52) |
-                                          (mant & 0xFFFFFFFFFFFFFull)));
+  mant += (((unsigned)m & 0x7FFu) + ((unsigned)mant & 1u)) > 0x400u ? 1ull : 0ull;
+  const int bx = 63 - lz + e + 1022;           // biased exponent less the leading one
+  unsigned long long r = ((unsigned long long)(unsigned)bx << 52) + mant;
+  r = bx >= 2046 ? 0x7FF0000000000000ull : r;
+  r = (a == 0 || bx < 0) ? 0ull : r;
+  return __longlong_as_double((long long)(sign | r));
 }
-
-// accumulator of product (p, q), 0-based slices: its level p+q; levels >= 4
-// share the last accumulator (they sit 2^-32 and further below the leading
-// level, so the truncation of the shared sum is far below the slice error)
-template <int NA>
-__host__ __device__ constexpr int level_of(int p, int q) { return p + q < NA ? p + q : NA - 1; }
-// accumulators in use for S slices (levels 0 .. S-1)
-template <int NA>
-__host__ __device__ constexpr int nlevels(int S) { return S < NA ? S : NA; }
 
 // byte offset of bf16 (row r, column t < 32) in a K-major tile of 64-byte rows
 // with the 64-byte swizzle, as TMA lays it out and the UMMA descriptor reads
@@ -405,332 +449,488 @@ __device__ __forceinline__ uint32_t sw64_off(int r, int t) {
   return (uint32_t)(r * 64 + ((((t >> 3) ^ (r >> 1)) & 3) << 4) + ((t & 7) << 1));
 }
 
-// Fused B operand, run by the 320 threads of warps 2-11 of k_ozaki: first
-// the scale exponents of the CTA's TN/2 complex columns over the whole depth
-// K (into col_exp, which the epilogue reads as well), then per k-block the S
-// B tiles of a stage: thread t takes column t/4 and the four complex indices
-// 16 kb + 4 (t%4) .. +3, forms their digits once (as k_split_b does) and
-// stores them four times (rows 2j and 2j+1, the Re and Im halves of the
-// k-block, -Im with flipped sign bits).  The next k-block's values are loaded
-// before the wait for the stage.  Each thread orders its stores before the
-// tensor core's reads (proxy fence); lane 0 of each warp, after the warp's
-// barrier, arrives on the stage's full barrier.
-template <int S, int TN, int DB, int NSTAGE>
-__device__ __forceinline__ void fused_b_tiles(const OzArgs &g, int item, int nt, unsigned char *sb0,
-                                              uint32_t stage_bytes, uint64_t *bar_full, uint64_t *bar_empty,
-                                              int *col_exp, volatile int &failed) {
-  constexpr int NCT = OZ_THREADS - 64;
-  constexpr uint32_t B_BYTES = TN * KB * 2;
-  const int ct = threadIdx.x - 64, lane = threadIdx.x & 31;
-  const zd *bsrc = mat_ptr(g.B, item / g.nc, item % g.nc);
-  const int j0 = (nt * TN) >> 1;
-  // warp w, four columns 4w .. 4w+3 per round (40 per round), 16 loads of
-  // each lane in flight
-  for (int jl0 = 4 * (ct >> 5); jl0 < TN / 2; jl0 += 4 * (NCT / 32)) {
-    unsigned long long m[4] = {0, 0, 0, 0};
-    for (int kc = 0; kc < g.K; kc += 128) {
-      zd v[4][4];
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int k = kc + lane + 32 * i, j = j0 + jl0 + c;
-          v[c][i] = (k < g.K && j < g.n && jl0 + c < TN / 2) ? bsrc[k + (long long)j * g.B.ld]
-                                                             : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const unsigned long long bx = abs_bits(v[c][i].x), by = abs_bits(v[c][i].y);
-          m[c] = bx > m[c] ? bx : m[c];
-          m[c] = by > m[c] ? by : m[c];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, m[c], o);
-        m[c] = t > m[c] ? t : m[c];
-      }
-      const int jl = jl0 + c;
-      if (lane == 0 && jl < TN / 2) col_exp[jl] = j0 + jl < g.n ? scale_exp(m[c]) : 0;
-    }
+// One CTA's walk over its tiles (t = blockIdx.x, + gridDim.x, ...; the N tiles
+// of an item side by side, so that they read its A slices from L2 together),
+// tiles of masked items left out; the mask of the tile after next is loaded
+// ahead.  Every role walks the same list.
+struct TileWalk {
+  const OzArgs &g;
+  int t, i, next_on;  // tile, its number in this CTA's list, mask of the next candidate
+  __device__ __forceinline__ explicit TileWalk(const OzArgs &g_) : g(g_), t((int)blockIdx.x - (int)gridDim.x), i(-1) {
+    next_on = on(t + (int)gridDim.x);
+    step();
   }
-  asm volatile("bar.sync 1, %0;" ::"n"(NCT) : "memory");
-  const int jl = ct >> 2, kq = ct & 3;
-  const bool on = ct < 2 * TN;
-  const bool col_ok = on && j0 + jl < g.n;
-  const zd *bcol = bsrc + (long long)(col_ok ? j0 + jl : 0) * g.B.ld;
-  const int es = on ? col_exp[jl] : 0;
-  zd cur[4], nxt[4];
-  auto fetch = [&](int kb, zd(&v)[4]) {
-    const int k = 16 * kb + 4 * kq;
-#pragma unroll
-    for (int e = 0; e < 4; e++) v[e] = (col_ok && k + e < g.K) ? bcol[k + e] : make_double2(0.0, 0.0);
+  __device__ __forceinline__ int on(int u) const {
+    return (g.act && u < g.tiles) ? g.act[u / (g.mtiles * g.ntiles)] : 1;
+  }
+  __device__ __forceinline__ void step() {
+    int keep;
+    do {
+      t += (int)gridDim.x;
+      keep = next_on;
+      next_on = on(t + (int)gridDim.x);
+    } while (t < g.tiles && !keep);
+    i++;
+  }
+  __device__ __forceinline__ bool valid() const { return t < g.tiles; }
+  __device__ __forceinline__ int item() const { return t / (g.mtiles * g.ntiles); }
+  __device__ __forceinline__ int mt() const { return t % (g.mtiles * g.ntiles) / g.ntiles; }
+  __device__ __forceinline__ int nt() const { return t % g.ntiles; }
+};
+
+struct OzShared {
+  __align__(8) uint64_t a_full[6], a_empty[6], b_full[6], b_empty[6], raw_full[8], raw_empty[8];
+  uint64_t acc_full[2], acc_empty[2], sc_full[OZ_SCALE_RING], sc_empty[OZ_SCALE_RING], done;
+  uint32_t tmem_base;
+  volatile int failed;
+  volatile int a_issued, raw_issued;      // k-blocks asked for (counts over all tiles)
+  int col_exp[OZ_EXP_RING][NT / 2];       // column scale exponents of each tile's complex columns
+};
+
+// the warp waits for a phase of a barrier; false (for the whole warp) once
+// anything failed
+__device__ __forceinline__ bool oz_warp_wait(OzShared &sh, uint64_t *bar, uint32_t parity, bool skip = false) {
+  if (skip || __all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) ok = !sh.failed && mbar_wait(bar, parity);
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  if (!ok) sh.failed = 1;
+  return ok != 0;
+}
+
+// n rows x 32 columns of an operand's tile towards L2, one column per lane
+__device__ __forceinline__ void oz_prefetch(const zd *p, int ld, int rows, int cols) {
+  const int lane = threadIdx.x & 31;
+  if (lane < cols) bulk_prefetch_l2(p + (long long)lane * ld, (uint32_t)rows * (uint32_t)sizeof(zd));
+}
+
+// The scale role (warp 2, fused B only): the exponents of each tile's 32
+// columns of B over the whole depth K, into the ring the conversion and the
+// epilogue read, with the columns of B two tiles ahead started towards L2.
+// Only the exponent field of a value matters (scale_exp), so the maxima run on
+// the upper words, and only those are loaded (64 loads of a lane in flight:
+// the role's pace is its load latency).  A ring slot of exponents is free
+// again when the role returns to it: it runs at most four tiles ahead of the
+// conversion, the conversion at most four k-blocks, hence five tiles, ahead of
+// the MMAs, and those wait for the epilogue of the tile oz_bufs before.
+__device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
+  const int lane = threadIdx.x & 31;
+  auto prefetch_b = [&](const TileWalk &w) {
+    const int item = w.item(), j0 = w.nt() * (NT / 2);
+    if (w.valid())
+      oz_prefetch(mat_ptr(g.B, item / g.nc, item % g.nc) + (long long)j0 * g.B.ld, g.B.ld, g.K,
+                  g.n - j0 < NT / 2 ? g.n - j0 : NT / 2);
   };
-  fetch(0, cur);
-  const int nkb = g.kblocks;
-  for (int kb = 0; kb < nkb; kb++) {
-    // the warp leaves together (lane 0 reads the flag), so its barriers and
-    // shuffles below always see all 32 lanes
-    if (__shfl_sync(0xffffffffu, (int)failed, 0)) break;
-    const int st = kb % NSTAGE;
-    if (kb + 1 < nkb) fetch(kb + 1, nxt);
-    // lane 0 waits for the stage, the warp follows it (its stores come after
-    // the tensor core's reads of the stage)
-    int ok = 1;
-    if (kb >= NSTAGE && lane == 0) ok = mbar_wait(&bar_empty[st], ((kb / NSTAGE) - 1) & 1);
-    if (!__shfl_sync(0xffffffffu, ok, 0)) {
-      failed = 1;
+  TileWalk wp(g);
+  prefetch_b(wp);
+  wp.step();
+  prefetch_b(wp);
+  for (TileWalk w(g); w.valid(); w.step()) {
+    const int item = w.item(), j0 = w.nt() * (NT / 2), nj = g.n - j0 < NT / 2 ? g.n - j0 : NT / 2;
+    if (wp.valid()) wp.step();
+    prefetch_b(wp);
+    if (!oz_warp_wait(sh, &sh.sc_empty[w.i % OZ_SCALE_RING], ((w.i / OZ_SCALE_RING) - 1) & 1, w.i < OZ_SCALE_RING))
       break;
+    const zd *b = mat_ptr(g.B, item / g.nc, item % g.nc) + (long long)j0 * g.B.ld;
+    int mine = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < nj; c0 += 8) {
+      unsigned m[8];
+#pragma unroll
+      for (int c = 0; c < 8; c++) m[c] = 0;
+#pragma unroll 1
+      for (int kc = 0; kc < g.K; kc += 128) {
+        // indices past the end repeat the last one: every load is valid and
+        // all of them are in flight together
+        unsigned v[8][8];
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const uint32_t *q = reinterpret_cast<const uint32_t *>(b + min(kc + lane + 32 * e, g.K - 1) +
+                                                                   (long long)min(c0 + c, nj - 1) * g.B.ld);
+            v[c][2 * e] = load_u32(q + 1);
+            v[c][2 * e + 1] = load_u32(q + 3);
+          }
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+#pragma unroll
+          for (int e = 0; e < 8; e++) m[c] = max(m[c], v[c][e] & 0x7FFFFFFFu);
+      }
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const unsigned t = __reduce_max_sync(0xffffffffu, m[c]);
+        if (lane == c0 + c && lane < nj) mine = scale_exp((unsigned long long)t << 32);
+      }
     }
-    if (on) {
+    sh.col_exp[w.i % OZ_EXP_RING][lane] = mine;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.sc_full[w.i % OZ_SCALE_RING]);
+  }
+}
+
+// The conversion role (fused B): the S B tiles of every k-block, eight columns
+// per warp.  A thread takes one column and the four complex indices
+// 16 kb + 4 (lane % 4) .. +3, forms their digits once and stores them four
+// times (rows 2j and 2j+1, the Re and Im halves of the k-block, -Im with
+// flipped sign bits).  Each thread orders its stores before the tensor core's
+// reads (proxy fence); lane 0, after the warp's barrier, arrives on the
+// stage's full barrier.  (Values outside the matrix arrive as zeros.)
+template <int S, int DB, int NB, int NRAW>
+__device__ __forceinline__ void oz_convert(const OzArgs &g, OzShared &sh, unsigned char *sb0, const unsigned char *raw) {
+  const int cw = (threadIdx.x >> 5) - OZ_CONV0, lane = threadIdx.x & 31;
+  const int nkb = g.kblocks, jl = 8 * (cw & 3) + (lane >> 2), kq = 4 * (lane & 3);
+  const int r = 2 * jl;
+  const uint32_t o0 = sw64_off(r, kq), o1 = sw64_off(r, kq + 16), o2 = sw64_off(r + 1, kq),
+                 o3 = sw64_off(r + 1, kq + 16);
+  // this thread's 16-byte values in a raw block: box kq / 8, row jl, chunks kq % 8 .. +3 XORed with jl % 8
+  const unsigned char *src = raw + (kq >> 3) * (OZ_RAW_BYTES / 2) + jl * 128;
+  for (TileWalk w(g); w.valid(); w.step()) {
+    if (!oz_warp_wait(sh, &sh.sc_full[w.i % OZ_SCALE_RING], (w.i / OZ_SCALE_RING) & 1)) return;
+    const int es = sh.col_exp[w.i % OZ_EXP_RING][jl];
+    for (int kb = cw >> 2; kb < nkb; kb += oz_conv_groups(S)) {
+      const int kc = w.i * nkb + kb, st = kc % NB, rr = kc % NRAW;
+      if (!oz_warp_wait(sh, &sh.raw_full[rr], (kc / NRAW) & 1)) return;
       double re[4], im[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        re[e] = cur[e].x;
-        im[e] = cur[e].y;
+        const zd v = *reinterpret_cast<const zd *>(src + rr * OZ_RAW_BYTES + ((((kq & 7) + e) ^ (jl & 7)) << 4));
+        re[e] = v.x;
+        im[e] = v.y;
       }
       uint32_t wr[S][2], wi[S][2];
-      slice4<S, DB>(re, im, es, 16, wr, wi);
-      unsigned char *sb = sb0 + st * stage_bytes;
-      const int r = 2 * jl, t = 4 * kq;
-      const uint32_t o0 = sw64_off(r, t), o1 = sw64_off(r, t + 16), o2 = sw64_off(r + 1, t),
-                     o3 = sw64_off(r + 1, t + 16);
+      if constexpr (DB == 8) slice4b<S>(re, im, es, wr, wi);
+      else slice4<S, DB>(re, im, es, 16, wr, wi);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.raw_empty[rr]);
+      // the stores come after the tensor core's reads of the stage
+      if (!oz_warp_wait(sh, &sh.b_empty[st], ((kc / NB) - 1) & 1, kc < NB)) return;
+      unsigned char *sb = sb0 + st * (S * OZ_B_SLICE);
 #pragma unroll
       for (int p = 0; p < S; p++) {
-        unsigned char *tp = sb + p * B_BYTES;
+        unsigned char *tp = sb + p * OZ_B_SLICE;
         *reinterpret_cast<uint2 *>(tp + o0) = make_uint2(wr[p][0], wr[p][1]);
         *reinterpret_cast<uint2 *>(tp + o1) = make_uint2(wi[p][0] ^ 0x80008000u, wi[p][1] ^ 0x80008000u);
         *reinterpret_cast<uint2 *>(tp + o2) = make_uint2(wi[p][0], wi[p][1]);
         *reinterpret_cast<uint2 *>(tp + o3) = make_uint2(wr[p][0], wr[p][1]);
       }
+      // every lane's stores visible to the tensor core, then one arrival per warp
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.b_full[st]);
     }
-    // every lane's stores visible to the tensor core, then one arrival per warp
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bar_full[st]);
-#pragma unroll
-    for (int e = 0; e < 4; e++) cur[e] = nxt[e];
+    if (lane == 0) mbar_arrive(&sh.sc_empty[w.i % OZ_SCALE_RING]);
   }
 }
 
-// TN: N tile (TMEM columns per accumulator); NA: TMEM accumulators, one per
-// level p+q = 0..NA-2 and a shared tail for the deeper levels (NA * TN <= 512).
-// (96, 5) is the default tile; (64, 7) keeps levels 0..5 exact and pushes the
-// truncation of the shared tail below 2^-60 of the leading level.  Four
-// levels would not do: with the shared tail from level 3 on, the tensor
-// core's truncating FP32 addition leaves ~2^-47 of the leading level per
-// accumulation step in it (4e-12 over a 128-deep product instead of 7e-14).
-// FB = 0: B tiles by TMA from the staged B'; FB = DB (7 or 8): B fused, its
-// tiles formed from the FP64 g.B by warps 2-11 (tmB unused).
-template <int S, int TN, int NA, int FB>
-__global__ void __launch_bounds__(OZ_THREADS, 1) k_ozaki(const __grid_constant__ CUtensorMap tmA,
-                                                  const __grid_constant__ CUtensorMap tmB, OzArgs g) {
-  static_assert(NA * TN <= 512 && TN % 32 == 0, "accumulators must fit the 512 TMEM columns");
-  constexpr int NCT = OZ_THREADS - 64;  // threads of warps 2-11
-  static_assert(FB == 0 || 2 * TN <= NCT, "fused B: one (column, four k) group per thread of warps 2-11");
-  const int item = blockIdx.y;
-  if (g.act && !g.act[item]) return;
-  const int mt = blockIdx.x / g.ntiles, nt = blockIdx.x % g.ntiles;
+// The epilogue role (warps 4-11): warp w reads TMEM lanes 32 (w % 4) .. +31
+// (rows of the M tile) and one half of the tile's 64 columns, as one 64-bit
+// integer per output.  With one accumulator set the level sums of the whole
+// tile are combined first and the accumulators handed back to the MMAs; the
+// rounding to FP64 and the update of C, D, E run beside the next tile's MMAs.
+template <int S, int DB, int FB>
+__device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint32_t tbase) {
+  constexpr int NBUF = oz_bufs(S), CH = S <= 6 ? 8 : 4;  // columns per TMEM load (registers)
+  constexpr bool EARLY = NBUF == 1;  // hand the accumulators back before the rounding
+  constexpr int NA = EARLY ? 32 : CH, NO = EARLY ? 8 : 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = warp & 3, half = (warp - OZ_EPI0) >> 2;
+  const int mode = g.mode;
+  const bool rd = mode == 1 || mode == 5 || mode == 2 || mode == 3, rd_c = mode == 1 || mode == 5;
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  for (TileWalk w(g); w.valid(); w.step()) {
+    const int item = w.item(), kk = item / g.nc, cc = item % g.nc, buf = w.i % NBUF;
+    const int row = w.mt() * MT + quarter * 32 + lane, j0 = w.nt() * (NT / 2) + half * 16;
+    // level 0 carries 2^(sigma_i + tau_j - 2 (DB - 1)); levels_sum is in units of level min(S - 1, 5)
+    const int sig = row < g.n ? g.sigma[(long long)item * (g.mtiles * MT) + row] : 0;
+    const int erow = sig - 2 * (DB - 1) - DB * (S - 1 < 5 ? S - 1 : 5);
+    const int nq = row < g.n ? g.n - j0 : 0;  // columns of this thread's row inside the matrix
+    zd *pc = mat_ptr(g.C, kk, cc) + row + (long long)j0 * g.C.ld;
+    zd *pd = mat_ptr(g.D, kk, cc) + row + (long long)j0 * g.D.ld;
+    zd *pe = mat_ptr(g.E, kk, cc) + row + (long long)j0 * g.E.ld;
+    // modes that read the old C (1, 5) or D (2, 3) load it ahead
+    const zd *src = rd_c ? pc : pd;
+    const long long sld = rd_c ? g.C.ld : g.D.ld;
+    // the column scales: of the scale role (fused B), or of the split
+    const int *ce = FB ? sh.col_exp[w.i % OZ_EXP_RING] + half * 16 : g.tau + (long long)item * g.n + j0;
+    zd old[NO];
+    auto load_old = [&](const zd *src, long long sld, int q0) {  // columns q0 .. q0 + NO - 1
+#pragma unroll
+      for (int q = 0; q < NO; q++)
+        if (q0 + q < nq) old[q] = src[(q0 + q) * sld];
+    };
+    // one output (column q of this thread's row) into C (mode 2: into D), `o` its old C or D
+    auto emit = [&](zd val, int q, zd o) {
+      zd *out = (mode == 2 ? pd : pc) + q * (long long)(mode == 2 ? g.D.ld : g.C.ld);
+      if (mode == 0) *out = val;
+      else if (mode == 4) *out = make_double2(row == j0 + q ? 1.0 - val.x : -val.x, -val.y);
+      else if (mode == 5) *out = zadd(o, val);
+      else *out = zsub(o, val);
+    };
+    // the level sums in FP64; a row of A or a column of B that holds an infinity or a NaN has no digits
+    auto value = [&](long long ar, long long ai, int q) {
+      const int tj = ce[q];
+      zd val = make_double2(fix_to_double(ar, erow + tj), fix_to_double(ai, erow + tj));
+      if (sig == SCALE_NONFINITE || tj == SCALE_NONFINITE) val = make_double2(nan, nan);
+      return val;
+    };
+    if (!EARLY && rd) load_old(src, sld, 0);
+    if (rd) {
+      // the next tile's old values towards L2: 16 columns x 512 bytes of this
+      // warp, one 128-byte line per lane and step
+      TileWalk wn = w;
+      wn.step();
+      if (wn.valid()) {
+        const int in = wn.item(), rn = wn.mt() * MT + quarter * 32 + 8 * (lane & 3), jn = wn.nt() * (NT / 2) + half * 16;
+        const MatRef &M = rd_c ? g.C : g.D;
+        const zd *p = mat_ptr(M, in / g.nc, in % g.nc) + rn;
+        const zd *pe2 = mat_ptr(g.E, in / g.nc, in % g.nc) + rn;
+#pragma unroll
+        for (int q = 0; q < 16; q += 8) {
+          const int j = jn + q + (lane >> 2);
+          if (rn < g.n && j < g.n) {
+            prefetch_l2(p + (long long)j * M.ld);
+            if (mode == 2) prefetch_l2(pe2 + (long long)j * g.E.ld);
+          }
+        }
+      }
+    }
+    if (!oz_warp_wait(sh, &sh.acc_full[buf], (w.i / NBUF) & 1)) break;
+    tc_fence_after();
+    const uint32_t ta = tbase + ((uint32_t)(quarter * 32) << 16) + buf * 256 + half * 32;
+    long long acc[NA];
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += CH) {
+      uint32_t v[S][CH];
+#pragma unroll
+      for (int l = 0; l < S; l++) {
+        if constexpr (CH == 8) tmem_ld8(ta + l * NT + c0, v[l]);
+        else tmem_ld4(ta + l * NT + c0, v[l]);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int t = 0; t < CH; t++) acc[(EARLY ? c0 : 0) + t] = levels_sum<S, DB, CH>(v, t);
+      if constexpr (!EARLY) {
+        const int q0 = c0 / 2;
+#pragma unroll
+        for (int q = 0; q < CH / 2; q++)
+          if (q0 + q < nq) {
+            const zd val = value(acc[2 * q], acc[2 * q + 1], q0 + q);
+            emit(val, q0 + q, old[q]);
+            if (mode == 2) pe[(q0 + q) * (long long)g.E.ld] = zsub(pe[(q0 + q) * (long long)g.E.ld], val);
+          }
+        if (rd && q0 + NO < 16) load_old(src, sld, q0 + NO);
+        __syncwarp();
+      }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
+    if constexpr (EARLY) {
+#pragma unroll
+      for (int q0 = 0; q0 < 16; q0 += NO) {
+        if (rd) load_old(src, sld, q0);
+#pragma unroll
+        for (int q = 0; q < NO; q++)
+          if (q0 + q < nq) {
+            const zd val = value(acc[(2 * (q0 + q)) % NA], acc[(2 * (q0 + q) + 1) % NA], q0 + q);
+            emit(val, q0 + q, old[q]);
+            acc[(2 * (q0 + q)) % NA] = __double_as_longlong(val.x);  // for E
+            acc[(2 * (q0 + q) + 1) % NA] = __double_as_longlong(val.y);
+          }
+      }
+      if (mode == 2) {
+#pragma unroll
+        for (int q0 = 0; q0 < 16; q0 += NO) {
+          load_old(pe, g.E.ld, q0);
+#pragma unroll
+          for (int q = 0; q < NO; q++)
+            if (q0 + q < nq)
+              pe[(q0 + q) * (long long)g.E.ld] =
+                  zsub(old[q], make_double2(__longlong_as_double(acc[(2 * (q0 + q)) % NA]),
+                                            __longlong_as_double(acc[(2 * (q0 + q) + 1) % NA])));
+        }
+      }
+    }
+  }
+}
+
+// Sliced product, persistent: one CTA per SM walks its output tiles (128 rows
+// x 32 complex columns) with the roles below running side by side, so that
+// the loads, the conversion of B and the rounding of one tile hide behind
+// another tile's MMAs.  (Before, one CTA of 128 x 48 per tile did these in
+// turn: of the 16.7 us a six-slice tile of it took, 4.4 were launch, TMEM
+// allocation and pipeline fill, 5 the epilogue, 5.2 the MMAs.)
+// What bounds it, 590 products of n = 128 from cold operands, before -> now:
+// staged B, six slices 293 -> 187 us (MMAs 12.5 of a tile's 21 thousand
+// cycles, the hand-over of the accumulators 4, operand loads 4; DRAM floor
+// 125 us); staged three slices 184 -> 112 us (epilogue: 64-bit integer
+// arithmetic at half the FP32 rate); fused B, seven slices 391 -> 258 us,
+// three slices 280 -> 164 us (conversion, likewise integer arithmetic);
+// R = I - AX and X += XR of the Newton step 422 + 316 -> 258 + 187 us.
+// More epilogue or conversion warps do not pay where they cost registers: 20
+// warps with 96 registers spill the six-slice epilogue's 64-bit sums (187 ->
+// 244 us); neither does redistributing registers with setmaxnreg (291 us).
+// Every level p + q has its own accumulator (64 TMEM columns each), so that
+// every level sum stays an exact integer while its bound allows (levels 0..3
+// always), and the slices of B lie side by side in a stage: A_p against up
+// to four of them is ONE instruction of N = 64..256 whose columns land in the
+// consecutive accumulators p + q.  A slice of A is then read once per 256
+// columns instead of once per pair.
+// FB = 0: B tiles by TMA from the staged B'; FB = 1: B fused, its tiles
+// formed by the conversion role from the FP64 B, which tmB then maps (g.B is
+// the same operand).
+template <int S, int DB, int FB>
+__global__ void __launch_bounds__(oz_threads(S), 1) k_ozaki(const __grid_constant__ CUtensorMap tmA,
+                                                         const __grid_constant__ CUtensorMap tmB,
+                                                         const __grid_constant__ OzArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // NSTAGE stages, each: S A tiles (MT x KB) then S B tiles (TN x KB), 1024-byte aligned
-  constexpr int NSTAGE = oz_stages(S, TN);
-  unsigned char *tiles = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr uint32_t A_BYTES = MT * KB * 2, B_BYTES = TN * KB * 2;
-  constexpr uint32_t STAGE_BYTES = S * (A_BYTES + B_BYTES);
-  __shared__ __align__(8) uint64_t bar_full[NSTAGE], bar_empty[NSTAGE], bar_acc;
-  __shared__ uint32_t tmem_base;
-  __shared__ volatile int failed, issued_kb, consumed_kb;
-  __shared__ int col_exp[TN / 2];  // column scale exponents of this tile's complex columns
+  constexpr int NA = oz_a_stages(S, FB > 0), NB = oz_b_stages(S, FB > 0), NBUF = oz_bufs(S);
+  constexpr int NRAW = FB > 0 ? oz_raw_stages(S) : 1;
+  static_assert(NA >= 2 && NB >= 2 && (FB == 0 || NRAW >= 2), "the rings must fit the shared memory");
+  unsigned char *sA = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char *sB = sA + NA * S * OZ_A_SLICE, *raw = sB + NB * S * OZ_B_SLICE;  // (all 1024-byte aligned)
+  __shared__ OzShared sh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (warp == 0) {
-    tmem_alloc(&tmem_base, 512);
+    tmem_alloc(&sh.tmem_base, 512);
     tmem_relinquish();
   }
-  if (FB > 0 && threadIdx.x >= 64 && lane == 0) {
-    // fused B: start the CTA's K x TN/2 block of B towards L2 (one bulk
-    // prefetch per column, lane 0 of warps 2-11)
-    const zd *bsrc = mat_ptr(g.B, item / g.nc, item % g.nc);
-    for (int jl = warp - 2; jl < TN / 2; jl += NCT / 32) {
-      const int j = (nt * TN) / 2 + jl;
-      if (j < g.n) bulk_prefetch_l2(bsrc + (long long)j * g.B.ld, (uint32_t)g.K * (uint32_t)sizeof(zd));
-    }
-  }
-  if (FB == 0 && threadIdx.x >= 64) {  // warps 2-11: column scales of the tile (read by the epilogue)
-    for (int t = threadIdx.x - 64; t < TN / 2; t += blockDim.x - 64) {
-      const int j = (nt * TN) / 2 + t;
-      col_exp[t] = j < g.n ? g.tau[(long long)item * g.n + j] : 0;
-    }
-  }
   if (threadIdx.x == 32) {
-    failed = 0;
-    issued_kb = -1;
-    consumed_kb = -1;
-    for (int i = 0; i < NSTAGE; i++) {
-      mbar_init(&bar_full[i], FB ? 1 + NCT / 32 : 1);  // fused B: each converting warp arrives too
-      mbar_init(&bar_empty[i], 1);
+    sh.failed = 0;
+    sh.a_issued = 0;
+    sh.raw_issued = 0;
+    for (int i = 0; i < 6; i++) {
+      mbar_init(&sh.a_full[i], 1);
+      mbar_init(&sh.a_empty[i], 1);
+      mbar_init(&sh.b_full[i], FB ? 4 : 1);  // fused B: the four warps of a group
+      mbar_init(&sh.b_empty[i], 1);
     }
-    mbar_init(&bar_acc, 1);
+    for (int i = 0; i < 8; i++) {
+      mbar_init(&sh.raw_full[i], 1);
+      mbar_init(&sh.raw_empty[i], 4);
+    }
+    for (int i = 0; i < OZ_SCALE_RING; i++) {
+      mbar_init(&sh.sc_full[i], 1);
+      mbar_init(&sh.sc_empty[i], 4 * oz_conv_groups(S));
+    }
+    for (int i = 0; i < NBUF; i++) {
+      mbar_init(&sh.acc_full[i], 1);
+      mbar_init(&sh.acc_empty[i], OZ_EPI_WARPS);
+    }
+    mbar_init(&sh.done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = tmem_base;
-  constexpr uint32_t IDESC = idesc_bf16(MT, TN);
+  const uint32_t tbase = sh.tmem_base;
   const int nkb = g.kblocks;
 
-  if (warp == 0 && lane == 0) {
-    // TMA producer
-    for (int kb = 0; kb < nkb && !failed; kb++) {
-      const int st = kb % NSTAGE;
-      if (kb >= NSTAGE && !mbar_wait(&bar_empty[st], ((kb / NSTAGE) - 1) & 1)) {
-        failed = 1;
-        break;
-      }
-      unsigned char *sA = tiles + st * STAGE_BYTES, *sB = sA + S * A_BYTES;
-      mbar_expect_tx(&bar_full[st], FB ? S * A_BYTES : STAGE_BYTES);
+  if (warp == 0) {
+    // TMA producer (with staged B both operands, in rings of equal length)
+    if (lane == 0) {
+      int kc = 0;
+      for (TileWalk w(g); w.valid() && !sh.failed; w.step()) {
+        const int item = w.item(), mt = w.mt(), nt = w.nt();
+        for (int kb = 0; kb < nkb; kb++, kc++) {
+          const int st = kc % NA;
+          if (sh.failed || (kc >= NA && !mbar_wait(&sh.a_empty[st], ((kc / NA) - 1) & 1))) {
+            sh.failed = 1;
+            break;
+          }
+          mbar_expect_tx(&sh.a_full[st], S * OZ_A_SLICE);
+          if (FB == 0) mbar_expect_tx(&sh.b_full[st], S * OZ_B_SLICE);
 #pragma unroll
-      for (int sl = 0; sl < S; sl++) {
-        const int z = (item * S + sl) * nkb + kb;
-        tma_load_3d(sA + sl * A_BYTES, &tmA, 0, mt * MT, z, &bar_full[st]);
-        if (FB == 0) tma_load_3d(sB + sl * B_BYTES, &tmB, 0, nt * TN, z, &bar_full[st]);
+          for (int sl = 0; sl < S; sl++) {
+            const int z = (item * S + sl) * nkb + kb;
+            tma_load_3d(sA + (st * S + sl) * OZ_A_SLICE, &tmA, 0, mt * MT, z, &sh.a_full[st]);
+            if (FB == 0) tma_load_3d(sB + (st * S + sl) * OZ_B_SLICE, &tmB, 0, nt * NT, z, &sh.b_full[st]);
+          }
+          sh.a_issued = kc + 1;
+        }
       }
-      issued_kb = kb;
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // MMA issuer
-    bool first[NA];
-#pragma unroll
-    for (int l = 0; l < NA; l++) first[l] = true;
-    for (int kb = 0; kb < nkb; kb++) {
-      const int st = kb % NSTAGE;
-      if (failed || !mbar_wait(&bar_full[st], (kb / NSTAGE) & 1)) {
-        failed = 1;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t a0 = smem_u32(tiles + st * STAGE_BYTES), b0 = a0 + S * A_BYTES;
-#pragma unroll
-      for (int p = 0; p < S; p++)
-#pragma unroll
-        for (int q = 0; q < S; q++) {
-          if (p + q > S - 1) continue;  // keep p+q <= S+1 in 1-based slices
-          const int lv = level_of<NA>(p, q);
-#pragma unroll
-          for (int k = 0; k < KB / 16; k++) {
-            umma_bf16(tbase + lv * TN, sdesc_sw64(a0 + p * A_BYTES + 32 * k),
-                      sdesc_sw64(b0 + q * B_BYTES + 32 * k), IDESC, first[lv] ? 0u : 1u);
-            first[lv] = false;
-          }
+    if (lane == 0) {
+      int kc = 0;
+      for (TileWalk w(g); w.valid() && !sh.failed; w.step()) {
+        const int buf = w.i % NBUF;
+        if (w.i >= NBUF && !mbar_wait(&sh.acc_empty[buf], ((w.i / NBUF) - 1) & 1)) {
+          sh.failed = 1;
+          break;
         }
-      umma_commit(&bar_empty[st]);  // stage free once these MMAs have read it
-      consumed_kb = kb;
+        const uint32_t td = tbase + buf * 256;
+        for (int kb = 0; kb < nkb; kb++, kc++) {
+          const int sa = kc % NA, sb = kc % NB;
+          if (sh.failed || !mbar_wait(&sh.a_full[sa], (kc / NA) & 1) || !mbar_wait(&sh.b_full[sb], (kc / NB) & 1)) {
+            sh.failed = 1;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(sA) + sa * (S * OZ_A_SLICE), b0 = smem_u32(sB) + sb * (S * OZ_B_SLICE);
+#pragma unroll
+          for (int k = 0; k < KB / 16; k++)
+#pragma unroll
+            for (int p = 0; p < S; p++)
+#pragma unroll
+              for (int q = 0; q < S - p; q += 4) {  // p + q <= S - 1; up to four slices of B at once
+                const int nb = S - p - q < 4 ? S - p - q : 4;
+                umma_bf16(td + (p + q) * NT, sdesc_sw64(a0 + p * OZ_A_SLICE + 32 * k),
+                          sdesc_sw64(b0 + q * OZ_B_SLICE + 32 * k), idesc_bf16(MT, NT * nb),
+                          (kb == 0 && k == 0 && p == 0) ? 0u : 1u);
+              }
+          umma_commit(&sh.a_empty[sa]);  // the stages are free once these MMAs have read them
+          umma_commit(&sh.b_empty[sb]);
+        }
+        umma_commit(&sh.acc_full[buf]);  // accumulators complete
+      }
+      umma_commit(&sh.done);
     }
-    umma_commit(&bar_acc);  // accumulators complete
-  } else if (warp >= 2) {
-    if constexpr (FB > 0) fused_b_tiles<S, TN, FB, NSTAGE>(g, item, nt, tiles + S * A_BYTES, STAGE_BYTES,
-                                                           bar_full, bar_empty, col_exp, failed);
+  } else if (warp == 2) {
+    if constexpr (FB > 0) oz_scales(g, sh);
+  } else if (warp == 3) {
+    // fused B: the FP64 k-blocks of B into their ring
+    if (FB > 0 && lane == 0) {
+      int rc = 0;
+      for (TileWalk w(g); w.valid() && !sh.failed; w.step()) {
+        const int kk = w.item() / g.nc, cc = w.item() % g.nc, j0 = w.nt() * (NT / 2);
+        const int mc = map_at(g.B, cc);
+        for (int kb = 0; kb < nkb; kb++, rc++) {
+          const int r = rc % NRAW;
+          if (sh.failed || (rc >= NRAW && !mbar_wait(&sh.raw_empty[r], ((rc / NRAW) - 1) & 1))) {
+            sh.failed = 1;
+            break;
+          }
+          mbar_expect_tx(&sh.raw_full[r], OZ_RAW_BYTES);
+          unsigned char *dst = raw + r * OZ_RAW_BYTES;
+          tma_load_4d(dst, &tmB, 32 * kb, j0, mc, kk, &sh.raw_full[r]);
+          tma_load_4d(dst + OZ_RAW_BYTES / 2, &tmB, 32 * kb + 16, j0, mc, kk, &sh.raw_full[r]);
+          sh.raw_issued = rc + 1;
+        }
+      }
+    }
+  } else if (warp < OZ_CONV0) {
+    oz_epilogue<S, DB, FB>(g, sh, tbase);
+  } else if constexpr (FB > 0) {
+    oz_convert<S, DB, NB, NRAW>(g, sh, sB, raw);
   }
   __syncthreads();
-  // all MMAs (and with them every TMA load they consumed) are done once
-  // bar_acc completes; a bounded wait, then a second one if the first expired
-  if (!mbar_wait(&bar_acc, 0)) {
-    failed = 1;
-    mbar_wait(&bar_acc, 0);
-  }
-  tc_fence_after();
+  // every MMA issued is complete (bounded wait) before the accumulators go
+  if (!mbar_wait(&sh.done, 0)) sh.failed = 1;
   __syncthreads();
-  if (failed) {
-    if (threadIdx.x == 0) {
-      atomicOr(g.err, 1);
-      // TMA loads issued but never consumed: let them land (bounded) before exit
-      for (int kb = consumed_kb + 1; kb <= issued_kb; kb++)
-        mbar_wait(&bar_full[kb % NSTAGE], (kb / NSTAGE) & 1);
+  if (sh.failed && threadIdx.x == 0) {
+    atomicOr(g.err, 1);
+    // copies asked for but perhaps not consumed: let them land (bounded) before exit
+    for (int kc = sh.a_issued > NA ? sh.a_issued - NA : 0; kc < sh.a_issued; kc++) {
+      mbar_wait(&sh.a_full[kc % NA], (kc / NA) & 1);
+      if (FB == 0) mbar_wait(&sh.b_full[kc % NB], (kc / NB) & 1);
     }
-  } else {
-    // epilogue, 12 warps: warp w reads TMEM lanes 32 (w % 4) .. +31 (rows of
-    // this M tile) and the 16-column chunks part, part + 3, ... (part = w / 4)
-    const int quarter = warp & 3, part = warp >> 2;
-    const int row = mt * MT + quarter * 32 + lane;
-    const uint32_t lane_addr = tbase + ((uint32_t)(quarter * 32) << 16);
-    const int kk = item / g.nc, cc = item % g.nc;
-    // accumulators carry 2^-30 sigma_i tau_j; the int64 sum is in units of 2^-16
-    const int erow = row < g.n ? g.sigma[(long long)item * (g.mtiles * MT) + row] - g.eoff : 0;
-    double *pc = (double *)mat_ptr(g.C, kk, cc);
-    double *pd = (double *)mat_ptr(g.D, kk, cc);
-    double *pe = (double *)mat_ptr(g.E, kk, cc);
-    constexpr int NL = nlevels<NA>(S);
-    // modes that read the old C (1, 5) or D (2, 3) load the chunk's eight
-    // elements of it first, so that the loads are in flight together
-    const bool rd_c = g.mode == 1 || g.mode == 5, rd_d = g.mode == 2 || g.mode == 3;
-    const double2 *src = (const double2 *)(rd_c ? pc : pd);
-    const long long sld = rd_c ? g.C.ld : g.D.ld;
-#pragma unroll 1
-    for (int c0 = part * 16; c0 < TN; c0 += 3 * 16) {
-      uint32_t v[NA][16];
-#pragma unroll
-      for (int l = 0; l < NL; l++) tmem_ld16(lane_addr + l * TN + c0, v[l]);
-      // (the seven-accumulator tile has no registers to spare for it)
-      constexpr bool PF = NA <= 5;
-      double2 old[PF ? 8 : 1];
-      if (PF && row < g.n && (rd_c || rd_d)) {
-#pragma unroll
-        for (int t = 0; t < 16; t += 2) {
-          const int j = (nt * TN + c0 + t) >> 1;
-          if (j < g.n) old[PF ? t >> 1 : 0] = src[row + (long long)j * sld];
-        }
-      }
-      tmem_ld_wait();
-      if (row >= g.n) continue;
-#pragma unroll
-      for (int t = 0; t < 16; t += 2) {  // accumulator columns 2j, 2j+1 = Re, Im of column j
-        const int j = (nt * TN + c0 + t) >> 1;
-        if (j < g.n) {
-          long long ar = 0, ai = 0;
-#pragma unroll
-          for (int l = 0; l < NL; l++) {
-            // exact levels by conversion and shift; the shared tail bitwise
-            const float vr = __uint_as_float(v[l][t]), vi = __uint_as_float(v[l][t + 1]);
-            ar += (l < NA - 1 && l <= 3) ? level_fix16(vr, l, g.db) : f2fix16(vr);
-            ai += (l < NA - 1 && l <= 3) ? level_fix16(vi, l, g.db) : f2fix16(vi);
-          }
-          const int e = erow + col_exp[(c0 + t) >> 1];
-          const double2 val = make_double2(fix_to_double(ar, e), fix_to_double(ai, e));
-          double2 *oc = (double2 *)pc + row + (long long)j * g.C.ld;
-          double2 *od = (double2 *)pd + row + (long long)j * g.D.ld;
-          const int q = t >> 1;
-          double2 o = make_double2(0.0, 0.0);  // the old C or D of this element
-          if constexpr (PF) {
-            o = old[q];
-          } else {
-            if (g.mode == 1 || g.mode == 5) o = *oc;
-            if (g.mode == 2 || g.mode == 3) o = *od;
-          }
-          if (g.mode == 0) {
-            *oc = val;
-          } else if (g.mode == 1) {
-            *oc = make_double2(o.x - val.x, o.y - val.y);
-          } else if (g.mode == 2) {
-            double2 *oe = (double2 *)pe + row + (long long)j * g.E.ld;
-            const double2 x = *oe;
-            *od = make_double2(o.x - val.x, o.y - val.y);
-            *oe = make_double2(x.x - val.x, x.y - val.y);
-          } else if (g.mode == 3) {
-            *oc = make_double2(o.x - val.x, o.y - val.y);
-          } else if (g.mode == 4) {
-            *oc = make_double2((row == j ? 1.0 : 0.0) - val.x, -val.y);
-          } else {
-            *oc = make_double2(o.x + val.x, o.y + val.y);
-          }
-        }
-      }
-    }
+    for (int rc = sh.raw_issued > NRAW ? sh.raw_issued - NRAW : 0; rc < sh.raw_issued; rc++)
+      mbar_wait(&sh.raw_full[rc % NRAW], (rc / NRAW) & 1);
   }
   tc_fence_before();
   __syncthreads();
@@ -1058,11 +1258,41 @@ int make_map(CUtensorMap *m, void *base, int rows, long long depth, int boxrows)
   return r == CUDA_SUCCESS ? 0 : -1;
 }
 
-// at least 120 KB so that only one CTA (and one 512-column TMEM allocation)
-// is resident per SM
-size_t oz_smem_bytes(int S, int TN) {
-  size_t b = (size_t)oz_stages(S, TN) * S * (MT * KB * 2 + TN * KB * 2) + 1024;
-  return b < 120 * 1024 ? 120 * 1024 : b;
+// the FP64 operand B (K rows, n columns, nk x nc items): dims {2 K doubles,
+// columns, class blocks, k points}; one box = eight complex values of 32
+// columns.  False where a stride cannot be mapped (the caller stages B then).
+bool make_raw_map(CUtensorMap *m, const MatRef &B, int n, int K, int nk, int nc) {
+  int cmax = 0;
+  for (int c = 0; c < nc; c++) {
+    if (B.map[c] < 0) return false;
+    cmax = std::max(cmax, B.map[c]);
+  }
+  const long long sc = cmax > 0 ? B.sc : (long long)n * B.ld, sk = nk > 1 ? B.sk : sc * (cmax + 1);
+  const long long top = 1LL << 35;
+  if (B.ld < K || sc <= 0 || sk <= 0 || sc >= top || sk >= top) return false;
+  cuuint64_t dims[4] = {(cuuint64_t)2 * K, (cuuint64_t)n, (cuuint64_t)cmax + 1, (cuuint64_t)nk};
+  cuuint64_t strides[3] = {(cuuint64_t)B.ld * sizeof(zd), (cuuint64_t)sc * sizeof(zd), (cuuint64_t)sk * sizeof(zd)};
+  cuuint32_t box[4] = {16, NT / 2, 1, 1}, es[4] = {1, 1, 1, 1};
+  return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, B.base, dims, strides, box, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// above half of an SM's shared memory for every S, so that no second CTA
+// (whose 512-column TMEM allocation would wait) becomes resident
+size_t oz_smem_bytes(int S, bool fused) {
+  return (size_t)oz_ring_bytes(S, fused) + (fused ? (size_t)oz_raw_stages(S) * OZ_RAW_BYTES : 0) + 1024;
+}
+
+int sm_count() {
+  static const int n = []() {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1)
+      return 152;
+    return v;
+  }();
+  return n;
 }
 
 }  // namespace
@@ -1077,7 +1307,6 @@ struct Stage {
   int *scale = nullptr;    // row (A) / column (B) scale exponents
   size_t scap = 0;
   int n = -1, K = -1;      // padding layout of p
-  int tn = 0;              // N tile the B layout is padded to
   int S = 0, DB = 0;       // the operand held: slices, digit base, dims, items
   int cn = -1, cK = -1;
   long long items = 0;
@@ -1102,19 +1331,12 @@ struct MixedWork {
   unsigned long long *nref = nullptr;  // [0] inverses that took further Newton steps, [1] kernels run by the
                                        // IF bodies of captured further steps (device counts)
   cudaStream_t side = nullptr;         // captures the bodies of conditional graph nodes
-  int smem_set[64] = {0};
-  bool precise = false;    // (64, 7) tile: exact levels 0..5 (mixed_set_precise)
   bool fuse_b = true;      // B operands formed inside the product (mixed_set_fused)
   bool blocked = true;     // 2 x 2 block start of inverses above 64 rows (mixed_set_blocked)
 };
 
-void mixed_set_precise(MixedWork *w, bool on) { w->precise = on; }
 void mixed_set_blocked(MixedWork *w, bool on) { w->blocked = on; }
 void mixed_set_fused(MixedWork *w, bool on) { w->fuse_b = on; }
-
-// the (64, 7) tile serves products of 6 slices and more (the low-slice
-// Newton corrections keep the default tile); split and multiply agree on it
-static bool use_precise(const MixedWork *w, int S) { return w->precise && S >= 6; }
 
 // the callers' streams are non-blocking: free the old buffer only once the
 // device is idle (cudaFree does not wait for those streams)
@@ -1214,36 +1436,28 @@ int mixed_error_flag(MixedWork *w) {
   return h;
 }
 
-// dims of the staged real problem for complex n x K times K x n, N tile tn
-static void oz_dims(int n, int K, int tn, int *Mp, int *Np, int *Kp, int *mtiles, int *ntiles, int *kblocks) {
+// dims of the staged real problem for complex n x K times K x n
+static void oz_dims(int n, int K, int *Mp, int *Np, int *Kp, int *mtiles, int *ntiles, int *kblocks) {
   *mtiles = (n + MT - 1) / MT;
   *Mp = *mtiles * MT;
-  *ntiles = (2 * n + tn - 1) / tn;
-  *Np = *ntiles * tn;
+  *ntiles = (2 * n + NT - 1) / NT;
+  *Np = *ntiles * NT;
   *kblocks = (2 * K + KB - 1) / KB;
   *Kp = *kblocks * KB;
 }
 
-// digit base for depth K: 8 bits while 2K <= 256 (8 slices then act as 7:
-// the fixed-point value is limited to 62 bits), 7 bits above so that the FP32
-// level sums stay exact integers
-static void oz_digits(int S, int K, int *Se, int *DB) {
-  *DB = K <= 128 ? 8 : 7;
-  *Se = (*DB == 8 && S > 7) ? 7 : S;
-}
+// digit base for depth K: 8 bits while 2K <= 256, 7 bits above so that the
+// FP32 level sums stay exact integers
+static int oz_digits(int K) { return K <= 128 ? 8 : 7; }
 
-// B operands of the default tile are fused into the product unless turned off
-static bool fuses_b(const MixedWork *w, int S) { return w->fuse_b && !use_precise(w, S); }
-
-// side 1 with fuses_b: the slot only records B (the product reads it when it
+// side 1 with fuse_b: the slot only records B (the product reads it when it
 // runs: B must not change in between, which every caller keeps); `real`
 // (an operand several products read) splits it all the same
 template <int S, int DB>
 static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int K, int nk, int nc,
                    const int *act, cudaStream_t st, bool real = false) {
   int Mp, Np, Kp, mtiles, ntiles, kblocks;
-  const int tn = use_precise(w, S) ? 64 : NT;
-  oz_dims(n, K, tn, &Mp, &Np, &Kp, &mtiles, &ntiles, &kblocks);
+  oz_dims(n, K, &Mp, &Np, &Kp, &mtiles, &ntiles, &kblocks);
   const long long items = (long long)nk * nc;
   Stage &sg = side == 0 ? w->A[slot] : w->B[slot];
   sg.S = S;
@@ -1251,7 +1465,7 @@ static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int
   sg.cn = n;
   sg.cK = K;
   sg.items = items;
-  sg.fused = side == 1 && !real && fuses_b(w, S);
+  sg.fused = side == 1 && !real && w->fuse_b;
   if (sg.fused) {
     sg.src = M;
     return 0;
@@ -1264,14 +1478,13 @@ static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int
   if ((rc = grow(&sg.p, &sg.cap, (size_t)items * S * rows * Kp * 2, true))) return rc;
   if ((rc = grow((void **)&sg.scale, &sg.scap, (size_t)items * (side == 0 ? Mp : n) * sizeof(int), false)))
     return rc;
-  if (sg.n != n || sg.K != K || (side == 1 && sg.tn != tn)) {
+  if (sg.n != n || sg.K != K) {
     // padding (rows beyond the operand, K' places of complex indices >= K)
     // must be zero; a new layout clears what an earlier one wrote there
     if (cudaMemsetAsync(sg.p, 0, sg.cap, st) != cudaSuccess) return SKKR_ERR_CUDA;
     sg.n = n;
     sg.K = K;
   }
-  sg.tn = side == 1 ? tn : 0;
   const long long active_s = act ? skkr_active_items(items) : items;
   // split traffic: FP64 operand read + S bf16 slices of the real embedding written
   const double split_bytes = (double)active_s * n * K * (16.0 + S * 2.0 * 2.0);
@@ -1289,51 +1502,39 @@ static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int
   return 0;
 }
 
-template <int S, int TN, int NA, int FB>
-static int oz_launch(MixedWork *w, int key, dim3 grid, const CUtensorMap &ma, const CUtensorMap &mb,
-                     const OzArgs &g, cudaStream_t st) {
-  const size_t smem = oz_smem_bytes(S, TN);
-  if (!w->smem_set[key]) {
-    if (cudaFuncSetAttribute(k_ozaki<S, TN, NA, FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return SKKR_ERR_CUDA;
-    w->smem_set[key] = 1;
-  }
-  k_ozaki<S, TN, NA, FB><<<grid, OZ_THREADS, smem, st>>>(ma, mb, g);
+template <int S, int DB, int FB>
+static int oz_launch(const CUtensorMap &ma, const CUtensorMap &mb, const OzArgs &g, cudaStream_t st) {
+  const size_t smem = oz_smem_bytes(S, FB > 0);
+  static const cudaError_t set =  // once per process (thread-safe static initialisation)
+      cudaFuncSetAttribute(k_ozaki<S, DB, FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (set != cudaSuccess) return SKKR_ERR_CUDA;
+  k_ozaki<S, DB, FB><<<std::min(g.tiles, sm_count()), oz_threads(S), smem, st>>>(ma, mb, g);
   return 0;
 }
 
-template <int S, int TN, int NA>
+template <int S, int DB>
 static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const MatRef &D, const MatRef &E,
                   int n, int K, int nk, int nc, const int *act, cudaStream_t st) {
   if (get_encoder()) return SKKR_ERR_CUDA;
   int Mp, Np, Kp, mtiles, ntiles, kblocks;
-  oz_dims(n, K, TN, &Mp, &Np, &Kp, &mtiles, &ntiles, &kblocks);
+  oz_dims(n, K, &Mp, &Np, &Kp, &mtiles, &ntiles, &kblocks);
   const long long items = (long long)nk * nc;
   const Stage &A = w->A[sa];
   Stage &B = w->B[sb];
-  if (A.fused || A.S != S || B.S != S || A.DB != B.DB || A.cn != n || B.cn != n || A.cK != K || B.cK != K ||
-      A.items != items || B.items != items || (!B.fused && B.tn != TN))
+  if (A.fused || A.S != S || B.S != S || A.DB != DB || B.DB != DB || A.cn != n || B.cn != n || A.cK != K ||
+      B.cK != K || A.items != items || B.items != items)
     return SKKR_ERR_ARG;  // the slots do not hold splits of this product's operands
+  CUtensorMap ma, mb;
   // a fused B that the product writes over (C, D or E) is split first, so
-  // that no CTA reads an element another one has already replaced
+  // that no CTA reads an element another one has already replaced; so is one
+  // whose strides no tensor map takes
   if (B.fused && (mref_overlap(B.src, C, nk, nc, n) || mref_overlap(B.src, D, nk, nc, n) ||
-                  mref_overlap(B.src, E, nk, nc, n))) {
-    int rc;
-    if constexpr (S <= 7)
-      rc = A.DB == 8 ? split_s<S, 8>(w, 1, sb, B.src, n, K, nk, nc, act, st, true)
-                     : split_s<S, 7>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
-    else
-      rc = split_s<S, 7>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
+                  mref_overlap(B.src, E, nk, nc, n) || !make_raw_map(&mb, B.src, n, K, nk, nc))) {
+    const int rc = split_s<S, DB>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
     if (rc) return rc;
   }
-  CUtensorMap ma, mb;
   if (make_map(&ma, A.p, Mp, items * S * kblocks, MT)) return SKKR_ERR_CUDA;
-  if (B.fused) {
-    mb = ma;  // unused by the fused kernel
-  } else if (make_map(&mb, B.p, Np, items * S * kblocks, TN)) {
-    return SKKR_ERR_CUDA;
-  }
+  if (!B.fused && make_map(&mb, B.p, Np, items * S * kblocks, NT)) return SKKR_ERR_CUDA;
   OzArgs g;
   g.n = n;
   g.mtiles = mtiles;
@@ -1341,8 +1542,6 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   g.kblocks = kblocks;
   g.nc = nc;
   g.mode = mode;
-  g.eoff = 32 + 2 * (A.DB - 1);
-  g.db = A.DB;
   g.sigma = A.scale;
   g.tau = B.scale;
   g.B = B.src;
@@ -1357,77 +1556,41 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   // FP64-equivalent: one complex n x K by K x n product per item
   kstat_begin2(KS_OZAKI, (double)(S * (S + 1) / 2) * 8.0 * n * (double)n * K * (double)active,
                8.0 * n * (double)n * K * (double)active, st);
-  dim3 grid(mtiles * ntiles, items);
-  // shared-memory attribute keys: S + 16 x (0 staged, 1 exact-level tile, 2 / 3 fused B at 8 / 7 digit bits)
-  int rc;
-  if (!B.fused) {
-    rc = oz_launch<S, TN, NA, 0>(w, S + (TN == NT ? 0 : 16), grid, ma, mb, g, st);
-  } else if constexpr (TN == NT && NA == NACC) {
-    if (A.DB == 8) {
-      if constexpr (S <= 7) rc = oz_launch<S, TN, NA, 8>(w, S + 32, grid, ma, mb, g, st);
-      else rc = SKKR_ERR_ARG;
-    } else {
-      rc = oz_launch<S, TN, NA, 7>(w, S + 48, grid, ma, mb, g, st);
-    }
-  } else {
-    rc = SKKR_ERR_ARG;  // fused B only on the default tile
-  }
+  g.tiles = (int)(items * mtiles * ntiles);
+  const int rc = B.fused ? oz_launch<S, DB, 1>(ma, mb, g, st) : oz_launch<S, DB, 0>(ma, mb, g, st);
   kstat_end(st);
   if (rc) return rc;
   SKKR_LAUNCHED();
   return 0;
 }
 
+// f<S, DB>(...) for S = 3..8 and the digit base of the depth
+#define OZ_DISPATCH(S, K, f, ...)                                    \
+  do {                                                               \
+    const bool d8 = oz_digits(K) == 8;                               \
+    switch (S) {                                                     \
+      case 3: return d8 ? f<3, 8>(__VA_ARGS__) : f<3, 7>(__VA_ARGS__); \
+      case 4: return d8 ? f<4, 8>(__VA_ARGS__) : f<4, 7>(__VA_ARGS__); \
+      case 5: return d8 ? f<5, 8>(__VA_ARGS__) : f<5, 7>(__VA_ARGS__); \
+      case 6: return d8 ? f<6, 8>(__VA_ARGS__) : f<6, 7>(__VA_ARGS__); \
+      case 7: return d8 ? f<7, 8>(__VA_ARGS__) : f<7, 7>(__VA_ARGS__); \
+      case 8: return d8 ? f<8, 8>(__VA_ARGS__) : f<8, 7>(__VA_ARGS__); \
+      default: return SKKR_ERR_ARG;                                  \
+    }                                                                \
+  } while (0)
+
 int mixed_split(MixedWork *w, int side, int slot, int S, const MatRef &M, int n, int K, int nk, int nc,
                 const int *act, cudaStream_t st, bool reused) {
   if (n < 1 || n > 256 || K < 1 || K > 256 || nk * (long long)nc > 65535 || slot < 0 ||
       slot >= MIXED_SLOTS || (side != 0 && side != 1))
     return SKKR_ERR_ARG;
-  int Se, DB;
-  oz_digits(S, K, &Se, &DB);
-  if (DB == 8) {
-    switch (Se) {
-      case 3: return split_s<3, 8>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-      case 4: return split_s<4, 8>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-      case 5: return split_s<5, 8>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-      case 6: return split_s<6, 8>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-      case 7: return split_s<7, 8>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-      default: return SKKR_ERR_ARG;
-    }
-  }
-  switch (Se) {
-    case 3: return split_s<3, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    case 4: return split_s<4, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    case 5: return split_s<5, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    case 6: return split_s<6, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    case 7: return split_s<7, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    case 8: return split_s<8, 7>(w, side, slot, M, n, K, nk, nc, act, st, reused);
-    default: return SKKR_ERR_ARG;
-  }
+  OZ_DISPATCH(S, K, split_s, w, side, slot, M, n, K, nk, nc, act, st, reused);
 }
 
 int mixed_gemm_staged(MixedWork *w, int mode, int S, int sa, int sb, const MatRef &C, const MatRef &D,
                       const MatRef &E, int n, int K, int nk, int nc, const int *act, cudaStream_t st) {
   if (sa < 0 || sa >= MIXED_SLOTS || sb < 0 || sb >= MIXED_SLOTS) return SKKR_ERR_ARG;
-  int Se, DB;
-  oz_digits(S, K, &Se, &DB);
-  if (use_precise(w, Se)) {
-    switch (Se) {  // 64-column tiles, levels 0..5 in their own accumulators
-      case 6: return gemm_s<6, 64, 7>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-      case 7: return gemm_s<7, 64, 7>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-      case 8: return gemm_s<8, 64, 7>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-      default: return SKKR_ERR_ARG;
-    }
-  }
-  switch (Se) {
-    case 3: return gemm_s<3, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    case 4: return gemm_s<4, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    case 5: return gemm_s<5, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    case 6: return gemm_s<6, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    case 7: return gemm_s<7, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    case 8: return gemm_s<8, NT, NACC>(w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
-    default: return SKKR_ERR_ARG;
-  }
+  OZ_DISPATCH(S, K, gemm_s, w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
 }
 
 int mixed_zgemm_k(MixedWork *w, int mode, int S, const MatRef &A, const MatRef &B, const MatRef &C,
@@ -1690,21 +1853,13 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
   if ((rc = grow((void **)&w->flag, &w->flag_cap, (size_t)items * sizeof(int), false))) return rc;
   if ((rc = grow((void **)&w->mark, &w->mark_cap, (size_t)items * sizeof(int), false))) return rc;
   // the further Newton steps split X (and, unless B is fused, R) into slot 5
-  // at sres slices (the standard correction uses 3): reserve that size, for
-  // either B tile, while not capturing, so that a captured step never has to
-  // grow the slot
-  int Se, DB;
-  oz_digits(sres, n, &Se, &DB);
+  // at sres slices (the standard correction uses 3): reserve that size while
+  // not capturing, so that a captured step never has to grow the slot
   if (!stream_capturing(st)) {
     int Mp, Np, Kp, mt, ntl, kbl;
-    size_t bb = 0, ba = 0;
-    for (int tn : {NT, 64}) {
-      oz_dims(n, n, tn, &Mp, &Np, &Kp, &mt, &ntl, &kbl);
-      ba = (size_t)items * Se * Mp * Kp * 2;
-      bb = std::max(bb, (size_t)items * Se * Np * Kp * 2);
-    }
-    if ((rc = grow(&w->A[5].p, &w->A[5].cap, ba, true))) return rc;
-    if (!fuses_b(w, Se) && (rc = grow(&w->B[5].p, &w->B[5].cap, bb, true))) return rc;
+    oz_dims(n, n, &Mp, &Np, &Kp, &mt, &ntl, &kbl);
+    if ((rc = grow(&w->A[5].p, &w->A[5].cap, (size_t)items * sres * Mp * Kp * 2, true))) return rc;
+    if (!w->fuse_b && (rc = grow(&w->B[5].p, &w->B[5].cap, (size_t)items * sres * Np * Kp * 2, true))) return rc;
   }
   // A itself serves the Gauss-Jordan start, the residuals and the FP64 redo
   // unless X overwrites it (in place): then a copy does
@@ -1745,7 +1900,7 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
     if (cap && (rc = cond_handle(st, &h))) return rc;
     // the IF body below launches 2 sliced products, 1 norm and the splits:
     // 3, or 1 with the B operands fused
-    const int nbody = fuses_b(w, Se) ? 4 : 6;
+    const int nbody = w->fuse_b ? 4 : 6;
     k_newton_select<<<1, 1024, 0, st>>>(w->rnorm, act, (int)items, 1e-6, 0.5, w->mark, w->cnt, w->nref, e == 0,
                                         h, cap ? 1 : 0, nbody);
     SKKR_LAUNCHED();

@@ -55,13 +55,15 @@ SLC_HD uint32_t slc_hi_pair(uint32_t a, uint32_t b) {
 
 // |x| bits of a double (non-negative doubles order like their bit patterns)
 SLC_HD unsigned long long abs_bits(double x) { return slc_dbits(x) & 0x7FFFFFFFFFFFFFFFull; }
-// log2 of the power-of-two scale for a max-|x| bit pattern (0 for zero)
+// log2 of the power-of-two scale for a max-|x| bit pattern (0 for zero;
+// SCALE_NONFINITE when an infinity or a NaN is the maximum: both order above
+// every finite value)
+constexpr int SCALE_NONFINITE = 0x7FF - 1022;
 SLC_HD int scale_exp(unsigned long long amax_bits) {
   const int ex = (int)(amax_bits >> 52);
   return ex == 0 ? 0 : ex - 1022;
 }
-// |round(x 2^E)| (halves away from zero) as a 64-bit integer (callers keep it
-// below 2^62) and the sign of x; zero and subnormal inputs give 0
+// |round(x 2^E)| (halves away from zero) as a 64-bit integer (at most 2^63) and the sign of x; zero and subnormal inputs give 0
 SLC_HD unsigned long long fix_round_mag(double x, int E, bool *neg) {
   const unsigned long long b = slc_dbits(x);
   *neg = (b >> 63) != 0;
@@ -101,7 +103,7 @@ SLC_HD constexpr unsigned long long digit_bias() {
 // stays an exact integer below 2^24.
 template <int S, int DB>
 SLC_HD void slice_digits(double x, int es, int *dig) {
-  static_assert(DB * S <= 62, "digits must fit the 62-bit fixed-point value");
+  static_assert(DB * S <= 64, "digits must fit the 64-bit fixed-point value");
   bool neg;
   const unsigned long long v = fix_round_mag(x, (DB - 1) + DB * (S - 1) - es, &neg) + digit_bias<S, DB>();
   constexpr int LOW = (1 << (DB - 1)) - 1;
@@ -175,3 +177,75 @@ SLC_HD void slice4(const double (&re)[4], const double (&im)[4], int es, int wsh
     }
   }
 }
+
+#ifdef __CUDACC__
+// fix_round_mag(x, 7 + 8 (S - 1) - es) + digit_bias<S, 8> on the device
+// without branches: the mantissa with its leading one at bit 63 (at bit 31
+// for S <= 4, whose 32 bits the upper 32 hold: nested floors are exact), one
+// right shift by one place less than wanted, and the last place rounds.  es
+// is at least the scale of x, so the shift is never to the left.
+template <int S>
+__device__ __forceinline__ unsigned long long biased_mag(double x, int es, bool *neg) {
+  constexpr unsigned long long BIAS = digit_bias<S, 8>();
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  *neg = (int)hi < 0;
+  const int ex = (int)((hi >> 20) & 0x7FFu);
+  const int r1 = es + 1022 - ex + (S <= 4 ? 32 - 8 * S : 64 - 8 * S);  // shift less one
+  uint32_t t0;
+  if constexpr (S <= 4) {
+    uint32_t m = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+    m = ex == 0 ? 0u : m;
+    asm("shr.u32 %0, %1, %2;" : "=r"(t0) : "r"(m), "r"(r1));
+    return (((unsigned long long)t0 + 1) >> 1) + BIAS;
+  } else {
+    uint32_t mh = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+    mh = ex == 0 ? 0u : mh;
+    const unsigned long long m = ((unsigned long long)mh << 32) | (ex == 0 ? 0u : lo << 11);
+    unsigned long long t;
+    asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m), "r"(r1));
+    return ((t >> 1) + (t & 1)) + BIAS;
+  }
+}
+
+// The same words for DB = 8 and wshift = 16, on the device, in about half the
+// instructions: the digits are bytes of |Y| + digit_bias, so one byte permute
+// pairs the digits f of two values, and 128 + (f & 127) is the bf16 with f's
+// low seven bits as its mantissa.  Adding -127 or -255 (as bit 7 of f is set
+// or not: a second permute replicates it over the half word, which then
+// selects) gives the digit f - 127; the top digit, which carries no bias,
+// takes 0 or -128.  The weight 2^(16 - 8 p) comes with the same packed FMA;
+// every value has at most eight significant bits, so nothing rounds.
+template <int S>
+__device__ __forceinline__ void slice4b(const double (&re)[4], const double (&im)[4], int es, uint32_t (&wr)[S][2],
+                                        uint32_t (&wi)[S][2]) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+#pragma unroll
+    for (int part = 0; part < 2; part++) {
+      bool s0, s1;
+      const unsigned long long y0 = biased_mag<S>(part ? im[2 * h] : re[2 * h], es, &s0);
+      const unsigned long long y1 = biased_mag<S>(part ? im[2 * h + 1] : re[2 * h + 1], es, &s1);
+      const uint32_t flip = (s0 ? 0x8000u : 0u) | (s1 ? 0x80000000u : 0u);
+#pragma unroll
+      for (int p = 0; p < S; p++) {
+        const int q = S - 1 - p, b = q & 3;  // byte q of the value
+        const uint32_t u0 = q < 4 ? (uint32_t)y0 : (uint32_t)(y0 >> 32);
+        const uint32_t u1 = q < 4 ? (uint32_t)y1 : (uint32_t)(y1 >> 32);
+        const uint32_t f = __byte_perm(u0, u1, (uint32_t)(b | (b << 4) | ((4 + b) << 8) | ((4 + b) << 12)));
+        uint32_t msb;  // byte b's bit 7 over each half word
+        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(msb) : "r"(u0), "r"(u1),
+            "r"((uint32_t)((8 + b) | ((8 + b) << 4) | ((12 + b) << 8) | ((12 + b) << 12))));
+        const uint32_t x = (f & 0x007F007Fu) | 0x43004300u;
+        const int e = (16 - 8 * p) * 128;  // the weight's shift of a bf16 exponent field
+        const uint32_t set = p == 0 ? 0u : (uint32_t)(0xC2FE + e) * 0x10001u;
+        const uint32_t clr = (uint32_t)((p == 0 ? 0xC300 : 0xC37F) + e) * 0x10001u;
+        const uint32_t c = (msb & set) | (~msb & clr);
+        const uint32_t w = (uint32_t)(0x3F80 + e) * 0x10001u;
+        uint32_t d;
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(w), "r"(c));
+        (part ? wi : wr)[p][h] = d ^ flip;
+      }
+    }
+  }
+}
+#endif
