@@ -798,9 +798,16 @@ static int check_slot_quirk(const skkr_ctx *c) {
 // ---------------------------------------------------------------------------
 // engine: the dense operations of decimation and tau2d in FP64 or split
 // precision (tcgen05 sliced products, FP32 inverse + Newton refinement)
-// electron-first principal-layer layout: BdG on the split-precision path
+// FP64 arithmetic (an FP64 context, or the FP64 parts of a split-precision
+// one) above WIDE_ROWS rows runs its products and inverses on the tensor cores
+// with eight slices per operand (wide_zgemm, wide_zinv); smaller blocks fill
+// too little of a 128-row tile and stay on the FP64 pipe.
+constexpr int WIDE_ROWS = 32;
+static bool wide_engine(const skkr_ctx *c) { return c->n > WIDE_ROWS && c->mw != nullptr; }
+
+// electron-first principal-layer layout: BdG on the tensor-core engines
 static int ehsplit(const skkr_ctx *c) {
-  return c->sz.mode == SKKR_BDG && c->sz.precision == SKKR_MIXED;
+  return c->sz.mode == SKKR_BDG && (c->sz.precision == SKKR_MIXED || c->n > WIDE_ROWS);
 }
 
 // slices of the products of the staged energy (more near the real axis)
@@ -833,6 +840,7 @@ static int eng_gemm(skkr_ctx *c, bool mixed, int mode, const MatRef &A, const Ma
     return mixed_zgemm_k(c->mw, m2, slices_for(c), A2, B2, C, D, E, n, h, nk, nc, act, c->st);
   }
   if (mixed) return mixed_zgemm(c->mw, mode, slices_for(c), A, B, C, D, E, n, nk, nc, act, c->st);
+  if (wide_engine(c)) return wide_zgemm(c->mw, mode, A, B, C, D, E, n, n > 128 || ehsplit(c), nk, nc, act, c->st);
   launch_zgemm(mode, A, B, C, D, E, n, n, n, nk, nc, act, c->st);
   return SKKR_OK;
 }
@@ -843,11 +851,20 @@ static int eng_inv(skkr_ctx *c, bool mixed, const MatRef &A, const MatRef &X, bo
   if (mixed && n <= 128) {
     mixed_set_blocked(c->mw, c->blocked_start != 0);
     return mixed_zinv(c->mw, A, X, n, nk, nc, act, c->newton,
-                      std::min(8, std::max(c->slices_res, slices_for(c) + 1)), inplace, c->st);
+                      std::min(8, std::max(c->slices_res, slices_for(c) + 1)), 3, 1e-6, inplace, c->st);
+  }
+  if (!mixed && wide_engine(c)) {
+    mixed_set_blocked(c->mw, true);
+    return wide_zinv(c->mw, A, X, n, n > 128 || ehsplit(c), nk, nc, act, inplace, c->st);
   }
   if (!inplace) launch_zaxpby(X, A, nullptr, 0, nullptr, 0, n, nk, nc, act, c->st);
   launch_zgj(X, n, nk, nc, act, c->st);
   return SKKR_OK;
+}
+
+// slices the staging slots hold at most, for the chunk size
+static int stage_slices(const skkr_ctx *c) {
+  return c->sz.precision == SKKR_MIXED ? c->slices_res : WIDE_SLICES;
 }
 
 static bool use_mixed(const skkr_ctx *c, bool decimation) {
@@ -991,6 +1008,8 @@ static int run_decimation(skkr_ctx *c, int k0, int nkc, const std::vector<int> &
   }
   const int itermax = std::max(c->sz.itermaxl, c->sz.itermaxr);
   const bool mx = use_mixed(c, true);
+  // products by whole operands of one depth: split each operand once
+  const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
   // one iteration (surfgf.f:47-96); the parity picks the alfa / beta buffers
   // read and written; iter_dev: the iteration number lives on the device (the
   // captured loop), else `iter` from the host
@@ -998,11 +1017,11 @@ static int run_decimation(skkr_ctx *c, int k0, int nkc, const std::vector<int> &
     MatRef &ac = odd ? a0 : a1, &an = odd ? a1 : a0;
     MatRef &bc = odd ? b0 : b1, &bn = odd ? b1 : b0;
     CKR(eng_inv(c, mx, eps, y1, false, n, nkc, nc, act));              // y1 = eps^-1
-    if (mx && !ehsplit(c)) {
-      // split-precision engine: each operand split once (B slots 1-3: y1,
+    if (staged) {
+      // tensor-core engines: each operand split once (B slots 1-3: y1,
       // alfa, beta; A slots 1-4: alfa, beta, P, Q) for the six products
       MixedWork *w = c->mw;
-      const int S = slices_for(c);
+      const int S = mx ? slices_for(c) : WIDE_SLICES;
       CKR(mixed_split(w, 1, 1, S, y1, n, n, nkc, nc, act, st, true));
       CKR(mixed_split(w, 0, 1, S, ac, n, n, nkc, nc, act, st));
       CKR(mixed_split(w, 0, 2, S, bc, n, n, nkc, nc, act, st));
@@ -1123,12 +1142,12 @@ static int run_tau2d(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls)
   MatRef Ys = mref_map(sbase, (long long)c->nsl * MB, MB, n, ysl, nc);
   MatRef Xs = mref_map(sbase, (long long)c->nsl * MB, MB, n, xsl, nc);
   const bool mx = use_mixed(c, false);
-  // split-precision engine: M10 and M01 enter every step on the same side,
+  // tensor-core engines: M10 and M01 enter every step on the same side,
   // so they are split once (A slot 1 = M10, B slot 1 = M01, A slot 3 = M01,
   // B slot 3 = M10); the per-step operands use slot 2
-  const bool staged = mx && !ehsplit(c);
+  const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
   MixedWork *w = c->mw;
-  const int S = slices_for(c);
+  const int S = mx ? slices_for(c) : WIDE_SLICES;
   auto prod = [&](int sa, const MatRef *A, int sb, const MatRef *B, const MatRef &C) -> int {
     if (A) CKR(mixed_split(w, 0, sa, S, *A, n, n, nkc, nc, nullptr, st));
     if (B) CKR(mixed_split(w, 1, sb, S, *B, n, n, nkc, nc, nullptr, st));
@@ -1581,7 +1600,7 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
   c->tot_dec = 0;
   c->err_code = 0;
   c->first_bad_k = -1;
-  if (c->sz.precision == SKKR_MIXED && !c->mw) {
+  if ((c->sz.precision == SKKR_MIXED || c->n > WIDE_ROWS) && !c->mw) {
     c->mw = mixed_create();
     if (!c->mw) return SKKR_ERR_NOMEM;
   }
@@ -1614,9 +1633,9 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
     const int ncmax = 2 * ng;
     double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + (5.0 * c->nprc + 1) * ng) +
                    (double)nc * ni * ni * lk2 * sizeof(zd);
-    if (c->sz.precision == SKKR_MIXED) {
+    if (c->mw) {
       const double Mp = 128.0 * ((n + 127) / 128), Np = 64.0 * ((2 * n + 63) / 64), Kp = 32.0 * ((2 * n + 31) / 32);
-      per_k += (double)ncmax * MIXED_SLOTS * c->slices_res * (Mp + Np) * Kp * 2.0;
+      per_k += (double)ncmax * MIXED_SLOTS * stage_slices(c) * (Mp + Np) * Kp * 2.0;
     }
     kc = c->sz.nk_chunk > 0 ? c->sz.nk_chunk : (int)std::max(1.0, std::floor(32.0e9 / per_k));
     kc = std::max(1, std::min(std::min(kc, 65535 / (2 * ng)), nk));
@@ -1827,7 +1846,7 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   c->graph_kernels = 0;
   c->graph_launches = 0;
   CKR(c->knorm.ensure((size_t)nk * sizeof(double)));
-  if (c->sz.precision == SKKR_MIXED && !c->mw) {
+  if ((c->sz.precision == SKKR_MIXED || c->n > WIDE_ROWS) && !c->mw) {
     c->mw = mixed_create();
     if (!c->mw) return SKKR_ERR_NOMEM;
   }
@@ -1845,13 +1864,12 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
     const int ncmax = 2 * c->ngeff;
     double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + (5.0 * c->nprc + 1) * c->ngeff) +
                    (double)c->ngeff * ni * lk2 * sizeof(zd);
-    if (use_mixed(c, false)) {
+    if (c->mw) {
       // BF16 slice staging: up to MIXED_SLOTS operands per side, S slices of
-      // the padded real embedding (A: 128-row tiles, B: 64-row tiles, K: 2n);
-      // an energy that runs wholly in FP64 stages nothing
+      // the padded real embedding (A: 128-row tiles, B: 64-row tiles, K: 2n)
       const double Mp = 128.0 * ((n + 127) / 128), Np = 64.0 * ((2 * n + 63) / 64),
                    Kp = 32.0 * ((2 * n + 31) / 32);
-      per_k += (double)ncmax * MIXED_SLOTS * c->slices_res * (Mp + Np) * Kp * 2.0;
+      per_k += (double)ncmax * MIXED_SLOTS * stage_slices(c) * (Mp + Np) * Kp * 2.0;
     }
     double budget = 64.0e9;  // of the 280 GB: the estimate counts every class slot as used
     int kc = c->sz.nk_chunk > 0 ? c->sz.nk_chunk : (int)std::max(1.0, std::floor(budget / per_k));
@@ -1952,7 +1970,8 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   trace_point("after CPA loop");
   c->inv_fallbacks = 0;
   c->inv_refined = 0;
-  if (c->mw) CKR(mixed_resid_read(c->mw, &c->max_resid, &c->inv_fallbacks, &c->inv_refined, st));
+  if (c->sz.precision == SKKR_MIXED)
+    CKR(mixed_resid_read(c->mw, &c->max_resid, &c->inv_fallbacks, &c->inv_refined, st));
   if (c->mw && c->err_code == 0) {
     int f = mixed_error_flag(c->mw);
     if (f != 0) {
@@ -2701,7 +2720,7 @@ extern "C" int skkr_gpu_zinv_batch(int precision, int n, int batch, double *a, i
     if (!w) return SKKR_ERR_NOMEM;
     double r = 0.0;
     int rc = mixed_resid_reset(w, 0);
-    if (!rc) rc = mixed_zinv(w, Am, Am, n, batch, 1, nullptr, newton, 7, true, 0);
+    if (!rc) rc = mixed_zinv(w, Am, Am, n, batch, 1, nullptr, newton, 7, 3, 1e-6, true, 0);
     if (!rc) rc = mixed_resid_read(w, &r, nullptr, nullptr, 0);
     if (rc == SKKR_OK && cudaDeviceSynchronize() != cudaSuccess) rc = SKKR_ERR_CUDA;
     if (rc == SKKR_OK && mixed_error_flag(w) != 0) rc = SKKR_ERR_CUDA;

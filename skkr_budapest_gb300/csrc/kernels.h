@@ -123,7 +123,15 @@ int mixed_zgemm_k(MixedWork *w, int mode, int S, const MatRef &A, const MatRef &
 int mixed_zgemm(MixedWork *w, int mode, int S, const MatRef &A, const MatRef &B, const MatRef &C,
                 const MatRef &D, const MatRef &E, int n, int nk, int nc, const int *act, cudaStream_t st);
 int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, int nc, const int *act,
-               int newton, int sres, bool inplace, cudaStream_t st);
+               int newton, int sres, int scorr, double limit, bool inplace, cudaStream_t st);
+// FP64 products (modes 0, 1, 2, 3, 4, 5) and inverses of FP64 contexts on the
+// tensor cores, n <= 256: eight slices per operand
+constexpr int WIDE_SLICES = 8;
+constexpr double WIDE_LIMIT = 1e-9;
+int wide_zgemm(MixedWork *w, int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D,
+               const MatRef &E, int n, bool halves, int nk, int nc, const int *act, cudaStream_t st);
+int wide_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, bool halves, int nk, int nc, const int *act,
+              bool inplace, cudaStream_t st);
 // running maximum of the accepted Newton residual norms and the count of
 // inverses redone in FP64 (device scalars), and the count of inverses that
 // took further Newton steps (host): reset asynchronously, read with a

@@ -1316,8 +1316,8 @@ struct Stage {
 
 struct MixedWork {
   Stage A[MIXED_SLOTS], B[MIXED_SLOTS];
-  zd *acopy = nullptr, *rbuf = nullptr;
-  size_t ac_cap = 0, rb_cap = 0;
+  zd *acopy = nullptr, *rbuf = nullptr, *big = nullptr;
+  size_t ac_cap = 0, rb_cap = 0, big_cap = 0;
   double *rnorm = nullptr;
   size_t rn_cap = 0;
   int *err = nullptr;
@@ -1423,7 +1423,7 @@ void mixed_destroy(MixedWork *w) {
     for (void *p : q)
       if (p) cudaFree(p);
   }
-  void *ps[] = {w->acopy, w->rbuf, w->rnorm, w->err, w->dmax, w->nfb, w->flag, w->mark, w->cnt, w->nref};
+  void *ps[] = {w->acopy, w->rbuf, w->big, w->rnorm, w->err, w->dmax, w->nfb, w->flag, w->mark, w->cnt, w->nref};
   for (void *p : ps)
     if (p) cudaFree(p);
   if (w->side) cudaStreamDestroy(w->side);
@@ -1840,10 +1840,11 @@ static void block_start(const MatRef &A, const MatRef &X, int n, int nc, const i
 }
 
 // X = A^-1: FP32 Gauss-Jordan, then `newton` steps X += X (I - A X) with the
-// residual product at S = sres slices and the correction at S = 3.  X may be
-// A itself (`inplace`); otherwise the two must not overlap.
+// residual product at S = sres slices and the correction at S = scorr.  An
+// item is accepted when the residual before the last correction is at most
+// `limit`.  X may be A itself (`inplace`); otherwise the two must not overlap.
 int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, int nc, const int *act,
-               int newton, int sres, bool inplace, cudaStream_t st) {
+               int newton, int sres, int scorr, double limit, bool inplace, cudaStream_t st) {
   if (n < 1 || n > 128 || newton < 1) return SKKR_ERR_ARG;
   const long long items = (long long)nk * nc, MB = (long long)n * n;
   int rc;
@@ -1853,7 +1854,7 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
   if ((rc = grow((void **)&w->flag, &w->flag_cap, (size_t)items * sizeof(int), false))) return rc;
   if ((rc = grow((void **)&w->mark, &w->mark_cap, (size_t)items * sizeof(int), false))) return rc;
   // the further Newton steps split X (and, unless B is fused, R) into slot 5
-  // at sres slices (the standard correction uses 3): reserve that size while
+  // at sres slices (the standard correction uses fewer): reserve that size while
   // not capturing, so that a captured step never has to grow the slot
   if (!stream_capturing(st)) {
     int Mp, Np, Kp, mt, ntl, kbl;
@@ -1883,9 +1884,9 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
     if ((rc = mixed_gemm_staged(w, 4, sres, 0, 0, R, R, R, n, n, nk, nc, act, st))) return rc;
     if (it == newton - 1) launch_fnorm(R, n, nk, nc, act, w->rnorm, st);
     // X = X + X R (slot 5: slot 0 keeps A)
-    if ((rc = mixed_split(w, 0, 5, 3, X, n, n, nk, nc, act, st))) return rc;
-    if ((rc = mixed_split(w, 1, 5, 3, R, n, n, nk, nc, act, st))) return rc;
-    if ((rc = mixed_gemm_staged(w, 5, 3, 5, 5, X, X, X, n, n, nk, nc, act, st))) return rc;
+    if ((rc = mixed_split(w, 0, 5, scorr, X, n, n, nk, nc, act, st))) return rc;
+    if ((rc = mixed_split(w, 1, 5, scorr, R, n, n, nk, nc, act, st))) return rc;
+    if ((rc = mixed_gemm_staged(w, 5, scorr, 5, 5, X, X, X, n, n, nk, nc, act, st))) return rc;
   }
   // Items above the limit but inside Newton's basin (|R| < 1/2) take up to
   // NEWTON_EXTRA further steps with the correction at sres slices as well:
@@ -1901,7 +1902,7 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
     // the IF body below launches 2 sliced products, 1 norm and the splits:
     // 3, or 1 with the B operands fused
     const int nbody = w->fuse_b ? 4 : 6;
-    k_newton_select<<<1, 1024, 0, st>>>(w->rnorm, act, (int)items, 1e-6, 0.5, w->mark, w->cnt, w->nref, e == 0,
+    k_newton_select<<<1, 1024, 0, st>>>(w->rnorm, act, (int)items, limit, 0.5, w->mark, w->cnt, w->nref, e == 0,
                                         h, cap ? 1 : 0, nbody);
     SKKR_LAUNCHED();
     const long long l_body = g_skkr_launches;
@@ -1942,7 +1943,92 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
   // Newton's basin: such items are inverted again in FP64 (copy A, column-
   // pivoting Gauss-Jordan), masked so that the others are untouched.  The
   // residual before the last correction bounds the final error by its square.
-  k_newton_check<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(w->rnorm, act, (int)items, 1e-6, w->flag,
+  k_newton_check<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(w->rnorm, act, (int)items, limit, w->flag,
+                                                                   w->dmax, w->nfb);
+  SKKR_LAUNCHED();
+  launch_zaxpby(X, Ac, nullptr, 0, nullptr, 0, n, nk, nc, w->flag, st);
+  launch_zgj(X, n, nk, nc, w->flag, st);
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 products and inverses on the tensor cores.  Eight slices of eight bits
+// hold a 64-bit fixed-point value per element (exact for every element down
+// to 2^-11 of its row's or column's largest, the others to 2^-64 of it), so a
+// product errs by less than the FP64 pipe's own rounding of its 2K terms.  The
+// depth is cut into `halves` above 128, where the level sums would leave
+// FP32's integers, and for BdG blocks (electron-first layout): each half then
+// has its own row and column scales, so that the O(Delta) electron-hole blocks
+// keep their own relative precision beside the diagonal ones.  590 products of n = 128: 8.01 ms on the FP64 pipe (99.5 % of its
+// rate), 0.29 ms here; relative Frobenius error 5e-16 either way.
+int wide_zgemm(MixedWork *w, int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D,
+               const MatRef &E, int n, bool halves, int nk, int nc, const int *act, cudaStream_t st) {
+  if (n <= 128 && !halves) return mixed_zgemm(w, mode, WIDE_SLICES, A, B, C, D, E, n, nk, nc, act, st);
+  // A B = A[:, :h] B[:h, :] + A[:, h:] B[h:, :]; every mode but 0, 3 and 4 is additive per half
+  const int h = n / 2, m2 = mode == 0 ? 5 : (mode == 3 || mode == 4) ? 1 : mode;
+  const MatRef A2 = mref_offset(A, (long long)h * A.ld), B2 = mref_offset(B, h);
+  const int rc = mixed_zgemm_k(w, mode, WIDE_SLICES, A, B, C, D, E, n, h, nk, nc, act, st);
+  if (rc) return rc;
+  return mixed_zgemm_k(w, m2, WIDE_SLICES, A2, B2, C, D, E, n, n - h, nk, nc, act, st);
+}
+
+// X = A^-1 to FP64 accuracy.  Up to 128 rows: mixed_zinv with eight-slice
+// residuals, four-slice corrections and the acceptance limit at 1e-9, whose
+// square is below FP64's rounding.  Above, and in `halves` (n even): the 2 x 2
+// block form of block_start with such inverses and products, then one Newton step on the
+// whole matrix, which also checks it.  What is not accepted is inverted by the
+// FP64 Gauss-Jordan, as are odd sizes above 128.  30 inverses of n = 256:
+// 18.9 ms by k_zgj (one block, hence one SM, per matrix).
+int wide_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, bool halves, int nk, int nc, const int *act,
+              bool inplace, cudaStream_t st) {
+  if (n <= 128 && !halves) return mixed_zinv(w, A, X, n, nk, nc, act, 2, WIDE_SLICES, 4, WIDE_LIMIT, inplace, st);
+  if (n > 256) return SKKR_ERR_ARG;
+  if (n & 1) {
+    if (!inplace) launch_zaxpby(X, A, nullptr, 0, nullptr, 0, n, nk, nc, act, st);
+    launch_zgj(X, n, nk, nc, act, st);
+    return 0;
+  }
+  const int h = n / 2;
+  const long long items = (long long)nk * nc, HB = (long long)h * h, NN = (long long)n * n;
+  // per item: X11, U, T, S, Y (h x h each), R and, in place, A (n x n each); then one zero block
+  const long long per = 5 * HB + (inplace ? 2 : 1) * NN;
+  int rc;
+  const size_t need = ((size_t)items * per + HB) * sizeof(zd);
+  if (need > w->big_cap && stream_capturing(st)) return SKKR_ERR_CUDA;
+  if ((rc = grow((void **)&w->big, &w->big_cap, need, false))) return rc;
+  if ((rc = grow((void **)&w->rnorm, &w->rn_cap, (size_t)items * sizeof(double), false))) return rc;
+  if ((rc = grow((void **)&w->flag, &w->flag_cap, (size_t)items * sizeof(int), false))) return rc;
+  auto blk = [&](long long off, int ld) { return mref(w->big + HB + off, nc * per, per, ld); };
+  const MatRef Z = mref(w->big, 0, 0, h), X11 = blk(0, h), U = blk(HB, h), T = blk(2 * HB, h), S = blk(3 * HB, h),
+               Y = blk(4 * HB, h), R = blk(5 * HB, n), Ac = inplace ? blk(5 * HB + NN, n) : A;
+  if (cudaMemsetAsync(w->big, 0, HB * sizeof(zd), st) != cudaSuccess) return SKKR_ERR_CUDA;
+  if (inplace) launch_zaxpby(Ac, A, nullptr, 0, nullptr, 0, n, nk, nc, act, st);
+  auto sub = [&](const MatRef &M, int r, int c) { return mref_offset(M, r + (long long)c * M.ld); };
+  const MatRef A12 = sub(Ac, 0, h), A21 = sub(Ac, h, 0), A22 = sub(Ac, h, h);
+  const MatRef Xa = X, X12 = sub(X, 0, h), X21 = sub(X, h, 0), X22 = sub(X, h, h);
+  auto prod = [&](int mode, const MatRef &a, const MatRef &b, const MatRef &c, const MatRef &d) {
+    return wide_zgemm(w, mode, a, b, c, d, c, h, false, nk, nc, act, st);
+  };
+  if ((rc = wide_zinv(w, Ac, X11, h, false, nk, nc, act, false, st))) return rc;
+  if ((rc = prod(0, X11, A12, U, U))) return rc;    // U = X11 A12
+  if ((rc = prod(0, A21, X11, T, T))) return rc;    // T = A21 X11
+  if ((rc = prod(3, A21, U, S, A22))) return rc;    // S = A22 - A21 U
+  if ((rc = wide_zinv(w, S, Y, h, false, nk, nc, act, false, st))) return rc;
+  launch_zaxpby(X22, Y, nullptr, 0, nullptr, 0, h, nk, nc, act, st);
+  if ((rc = prod(3, U, Y, X12, Z))) return rc;      // X12 = -U Y
+  if ((rc = prod(3, Y, T, X21, Z))) return rc;      // X21 = -Y T
+  if ((rc = prod(3, X12, T, Xa, X11))) return rc;   // X11 - X12 T
+  // one Newton step: R = I - A X, X += X R
+  if ((rc = wide_zgemm(w, 4, Ac, X, R, R, R, n, true, nk, nc, act, st))) return rc;
+  launch_fnorm(R, n, nk, nc, act, w->rnorm, st);
+  const MatRef Xr = sub(X, 0, h), R2 = mref_offset(R, h);
+  if ((rc = mixed_split(w, 0, 1, 4, X, n, h, nk, nc, act, st))) return rc;
+  if ((rc = mixed_split(w, 0, 2, 4, Xr, n, h, nk, nc, act, st))) return rc;
+  if ((rc = mixed_split(w, 1, 1, 4, R, n, h, nk, nc, act, st))) return rc;
+  if ((rc = mixed_split(w, 1, 2, 4, R2, n, h, nk, nc, act, st))) return rc;
+  if ((rc = mixed_gemm_staged(w, 5, 4, 1, 1, X, X, X, n, h, nk, nc, act, st))) return rc;
+  if ((rc = mixed_gemm_staged(w, 5, 4, 2, 2, X, X, X, n, h, nk, nc, act, st))) return rc;
+  k_newton_check<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(w->rnorm, act, (int)items, WIDE_LIMIT, w->flag,
                                                                    w->dmax, w->nfb);
   SKKR_LAUNCHED();
   launch_zaxpby(X, Ac, nullptr, 0, nullptr, 0, n, nk, nc, w->flag, st);
