@@ -278,18 +278,87 @@ __global__ void __launch_bounds__(256) k_zgemm(MatRef A, MatRef B, MatRef C, Mat
     }
 }
 
+// The same product for blocks of at most 64 rows, one thread per output and the
+// outputs of an item dealt flat (rows fastest) over blocks of T threads: no
+// thread of a full block idles on padding, and a few items still spread over
+// the SMs.  The FP64 pipe bounds both forms (about two multiply-adds a clock
+// per SM): an 18-row block fills 324 of 352 lanes here against 324 of 1024
+// outputs of a 32 x 32 tile, and one 32-row product takes 16 SMs instead of
+// one (36.6 us).  Every output is summed in the same order (same bits).
+constexpr int ZF_ROWS = 64, ZF_K = 32;
+template <int MODE>
+__global__ void __launch_bounds__(256) k_zgemm_flat(MatRef A, MatRef B, MatRef C, MatRef D, MatRef E, int M, int N,
+                                                    int K, int nc, const int *__restrict__ act) {
+  const int item = blockIdx.y, kk = item / nc, cc = item % nc;
+  if (act && !act[item]) return;
+  extern __shared__ zd zf_smem[];
+  const int T = blockDim.x, e0 = blockIdx.x * T, e1 = min(M * N, e0 + T) - 1;
+  const int c0 = e0 / M, ncol = e1 / M - c0 + 1;  // the columns this block's outputs touch
+  zd *As = zf_smem, *Bs = zf_smem + M * ZF_K;     // [k][row], [column][k]
+  const zd *a = mat_ptr(A, kk, cc), *b = mat_ptr(B, kk, cc);
+  const int e = e0 + (int)threadIdx.x, r = e % M, c = e / M;
+  const bool on = e < M * N;
+  zd acc = make_double2(0.0, 0.0);
+  for (int k0 = 0; k0 < K; k0 += ZF_K) {
+    const int kn = min(ZF_K, K - k0);
+    for (int i = threadIdx.x; i < M * kn; i += T) As[i] = a[i % M + (long long)(k0 + i / M) * A.ld];
+    for (int i = threadIdx.x; i < ncol * kn; i += T)
+      Bs[i / kn * ZF_K + i % kn] = b[k0 + i % kn + (long long)(c0 + i / kn) * B.ld];
+    __syncthreads();
+    if (on) {
+      const zd *ap = As + r, *bp = Bs + (c - c0) * ZF_K;
+#pragma unroll 4
+      for (int q = 0; q < kn; q++) zfma(acc, ap[q * M], bp[q]);
+    }
+    __syncthreads();
+  }
+  if (!on) return;
+  if (MODE == 0) {
+    mat_ptr(C, kk, cc)[r + (long long)c * C.ld] = acc;
+  } else if (MODE == 1) {
+    zd *p = mat_ptr(C, kk, cc) + r + (long long)c * C.ld;
+    *p = zsub(*p, acc);
+  } else if (MODE == 2) {
+    zd *p = mat_ptr(D, kk, cc) + r + (long long)c * D.ld;
+    *p = zsub(*p, acc);
+    zd *q2 = mat_ptr(E, kk, cc) + r + (long long)c * E.ld;
+    *q2 = zsub(*q2, acc);
+  } else {
+    const zd d = mat_ptr(D, kk, cc)[r + (long long)c * D.ld];
+    mat_ptr(C, kk, cc)[r + (long long)c * C.ld] = zsub(d, acc);
+  }
+}
+
+template <int MODE>
+static void zgemm_go(const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D, const MatRef &E, int m, int n,
+                     int kdim, int nk, int nc, const int *act, cudaStream_t st) {
+  const long long outs = (long long)m * n, items = (long long)nk * nc;
+  if (m <= ZF_ROWS) {
+    // blocks of 64 outputs while they do not give every SM one, else of 128
+    const int T = items * ((outs + 63) / 64) < 2 * 152 ? 64 : 128;
+    const int ncol = std::min(n, (T + m - 2) / m + 1);
+    const size_t smem = (size_t)(m + ncol) * ZF_K * sizeof(zd);
+    if (smem <= 48 * 1024) {
+      k_zgemm_flat<MODE><<<dim3((unsigned)((outs + T - 1) / T), (unsigned)items), T, smem, st>>>(A, B, C, D, E, m, n,
+                                                                                                 kdim, nc, act);
+      return;
+    }
+  }
+  dim3 grid(((m + 31) / 32) * ((n + 31) / 32), (unsigned)items);
+  k_zgemm<MODE><<<grid, 256, 0, st>>>(A, B, C, D, E, m, n, kdim, nc, act);
+}
+
 void launch_zgemm(int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D,
                   const MatRef &E, int m, int n, int kdim, int nk, int nc, const int *act,
                   cudaStream_t st) {
   if (nk <= 0 || nc <= 0 || m <= 0 || n <= 0) return;
-  dim3 grid(((m + 31) / 32) * ((n + 31) / 32), nk * nc);
   const long long items = act ? skkr_active_items((long long)nk * nc) : (long long)nk * nc;
   kstat_begin(KS_GEMM, 8.0 * m * n * kdim * (double)items, st);
   switch (mode) {
-    case 0: k_zgemm<0><<<grid, 256, 0, st>>>(A, B, C, D, E, m, n, kdim, nc, act); break;
-    case 1: k_zgemm<1><<<grid, 256, 0, st>>>(A, B, C, D, E, m, n, kdim, nc, act); break;
-    case 2: k_zgemm<2><<<grid, 256, 0, st>>>(A, B, C, D, E, m, n, kdim, nc, act); break;
-    default: k_zgemm<3><<<grid, 256, 0, st>>>(A, B, C, D, E, m, n, kdim, nc, act); break;
+    case 0: zgemm_go<0>(A, B, C, D, E, m, n, kdim, nk, nc, act, st); break;
+    case 1: zgemm_go<1>(A, B, C, D, E, m, n, kdim, nk, nc, act, st); break;
+    case 2: zgemm_go<2>(A, B, C, D, E, m, n, kdim, nk, nc, act, st); break;
+    default: zgemm_go<3>(A, B, C, D, E, m, n, kdim, nk, nc, act, st); break;
   }
   kstat_end(st);
   SKKR_LAUNCHED();
@@ -379,12 +448,176 @@ __global__ void __launch_bounds__(512) k_zgj(MatRef A, int n, int nc, const int 
   }
 }
 
+// |z|^2, or |z| where the squares of a row leave the doubles' range
+__device__ __forceinline__ double zmag(zd v, bool far) { return far ? hypot(v.x, v.y) : v.x * v.x + v.y * v.y; }
+
+// The same inverse for n <= 64 with the matrix in registers: TY x LW threads,
+// thread (ty, tx) owning rows ty + TY a (a < RA) and columns tx + LW b (b < RB).
+// As in the FP32 form (k_cgj32) the pivot columns stay in place (step i uses
+// pivot (i, kp), sigma(i) = kp; the permutations are undone at the store).
+// The LW threads that own row i + 1 pick its pivot after its update, by the
+// largest modulus with the first index on ties (compared as squares, with the
+// moduli themselves where squares would overflow or vanish), and stage the
+// row divided by the pivot, so that a step is one multiply-add per element and
+// one block barrier.  The FP64 pipe bounds it (n^2 complex multiply-adds a
+// step, about half a clock each per SM), so the layouts follow n in steps of
+// eight columns and warps without a row of the matrix only keep the barriers.
+// 506 matrices of 18 rows: 212 us, 24 of 32 rows: 200 us by k_zgj, whose steps
+// take four barriers and pass over global memory.
+template <int LW, int TY, int RA, int RB>
+__device__ __forceinline__ void zgj_stage(const zd (&m)[RA][RB], int row, unsigned used, int tx, unsigned gmask,
+                                          zd *prow, int *kp_out) {
+  const int ia0 = row / TY;
+  zd v[RB];
+#pragma unroll
+  for (int ib = 0; ib < RB; ib++) {
+    v[ib] = m[0][ib];
+#pragma unroll
+    for (int ia = 1; ia < RA; ia++)
+      if (ia == ia0) v[ib] = m[ia][ib];
+  }
+  double best = -1.0;
+  int bj = 0x7FFFFFFF;
+  bool far = false;
+  for (int pass = 0; pass < 2; pass++) {
+    best = -1.0;
+    bj = 0x7FFFFFFF;
+    int fu = 0x7FFFFFFF;
+#pragma unroll
+    for (int ib = 0; ib < RB; ib++) {
+      const int j = tx + LW * ib;
+      const bool free = !((used >> ib) & 1u);
+      const double q = zmag(v[ib], far);
+      if (free && (q > best || (q == best && j < bj))) {
+        best = q;
+        bj = j;
+      }
+      if (free && j < fu) fu = j;
+    }
+#pragma unroll
+    for (int o = LW / 2; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(gmask, best, o, LW);
+      const int oj = __shfl_xor_sync(gmask, bj, o, LW), of = __shfl_xor_sync(gmask, fu, o, LW);
+      if (ob > best || (ob == best && oj < bj)) {
+        best = ob;
+        bj = oj;
+      }
+      fu = of < fu ? of : fu;
+    }
+    if (bj == 0x7FFFFFFF) bj = fu;  // every candidate NaN
+    if (far || (best > 1e-280 && best < 1e280)) break;
+    far = true;
+  }
+  const int kb = bj / LW;
+  zd pv = v[0];
+#pragma unroll
+  for (int ib = 1; ib < RB; ib++)
+    if (ib == kb) pv = v[ib];
+  pv.x = __shfl_sync(gmask, pv.x, bj % LW, LW);
+  pv.y = __shfl_sync(gmask, pv.y, bj % LW, LW);
+  zd q;
+  if (far) {
+    q = zrecip(pv);
+  } else {
+    const double d = 1.0 / best;
+    q = make_double2(pv.x * d, -pv.y * d);
+  }
+#pragma unroll
+  for (int ib = 0; ib < RB; ib++) {
+    const int j = tx + LW * ib;
+    prow[j] = j == bj ? q : zmul(v[ib], q);
+  }
+  if (tx == 0) *kp_out = bj;
+}
+
+template <int LW, int TY, int RA, int RB>
+__global__ void __launch_bounds__(TY *LW) k_zgj_reg(MatRef A, int n, int nc, const int *__restrict__ act) {
+  static_assert((TY * LW) % 32 == 0, "whole warps");
+  constexpr int NR = TY * RA, NCOL = LW * RB, WR = 32 / LW;  // rows of one a per warp
+  const int item = blockIdx.x, kk = item / nc, cc = item % nc;
+  if (act && !act[item]) return;
+  __shared__ zd prow[2][NCOL];
+  __shared__ int sig[NR], sinv[NCOL], kpn[2];
+  const int tid = threadIdx.x, ty = tid / LW, tx = tid % LW;
+  const bool live = ty / WR * WR < n;  // the warp has a row of the matrix (its smallest is that of a = 0)
+  zd *a = mat_ptr(A, kk, cc);
+  zd m[RA][RB];
+  unsigned used = 0;
+#pragma unroll
+  for (int ib = 0; ib < RB; ib++) {
+    const int j = tx + LW * ib;
+    if (j >= n) used |= 1u << ib;  // columns past the matrix never pivot
+#pragma unroll
+    for (int ia = 0; ia < RA; ia++) {
+      const int r = ty + TY * ia;
+      m[ia][ib] = (r < n && j < n) ? a[r + (long long)j * A.ld] : make_double2(0.0, 0.0);
+    }
+  }
+  const unsigned gmask = (LW == 32 ? 0xFFFFFFFFu : ((1u << (LW & 31)) - 1)) << (tid % 32 / LW * LW);  // this ty's threads
+  if (ty == 0) zgj_stage<LW, TY, RA, RB>(m, 0, used, tx, gmask, prow[0], &kpn[0]);
+  __syncthreads();
+  for (int i = 0; i < n; i++) {
+    const int kp = kpn[i & 1], kb = kp / LW, kt = kp % LW;
+    if (tid == 0) {
+      sig[i] = kp;
+      sinv[kp] = i;
+    }
+    if (tx == kt) used |= 1u << kb;
+    if (live) {
+      const zd *pr = prow[i & 1];
+      zd c[RA];
+#pragma unroll
+      for (int ia = 0; ia < RA; ia++) {
+        zd w = m[ia][0];
+#pragma unroll
+        for (int ib = 1; ib < RB; ib++)
+          if (ib == kb) w = m[ia][ib];
+        c[ia].x = __shfl_sync(0xFFFFFFFFu, w.x, kt, LW);  // a(r, kp) from its owner beside this thread
+        c[ia].y = __shfl_sync(0xFFFFFFFFu, w.y, kt, LW);
+      }
+#pragma unroll
+      for (int ib = 0; ib < RB; ib++) {
+        const int j = tx + LW * ib;
+        const zd p = pr[j];
+#pragma unroll
+        for (int ia = 0; ia < RA; ia++) {
+          zd v = j == kp ? make_double2(0.0, 0.0) : m[ia][ib];
+          zfms(v, c[ia], p);
+          m[ia][ib] = ty + TY * ia == i ? p : v;
+        }
+      }
+      if (i + 1 < n && ty == (i + 1) % TY)
+        zgj_stage<LW, TY, RA, RB>(m, i + 1, used, tx, gmask, prow[(i + 1) & 1], &kpn[(i + 1) & 1]);
+    }
+    __syncthreads();
+  }
+  // storage (r, j) holds A^-1(sigma(r), sigma^-1(j))
+#pragma unroll
+  for (int ia = 0; ia < RA; ia++)
+#pragma unroll
+    for (int ib = 0; ib < RB; ib++) {
+      const int r = ty + TY * ia, j = tx + LW * ib;
+      if (r < n && j < n) a[sig[r] + (long long)sinv[j] * A.ld] = m[ia][ib];
+    }
+}
+
+template <int LW, int TY, int RA, int RB>
+static void zgj_go(const MatRef &A, int n, int items, int nc, const int *act, cudaStream_t st) {
+  k_zgj_reg<LW, TY, RA, RB><<<items, TY * LW, 0, st>>>(A, n, nc, act);
+}
+
 void launch_zgj(const MatRef &A, int n, int nk, int nc, const int *act, cudaStream_t st) {
   if (nk <= 0 || nc <= 0 || n <= 0) return;
-  int th = n * n >= 4096 ? 512 : 256;
   const long long items = act ? skkr_active_items((long long)nk * nc) : (long long)nk * nc;
   kstat_begin(KS_GJ, 8.0 * n * n * (double)n * (double)items, st);
-  k_zgj<<<nk * nc, th, 0, st>>>(A, n, nc, act);
+  const int N = nk * nc;
+  if (n <= 8) zgj_go<8, 8, 1, 1>(A, n, N, nc, act, st);
+  else if (n <= 16) zgj_go<8, 16, 1, 2>(A, n, N, nc, act, st);
+  else if (n <= 24) zgj_go<8, 24, 1, 3>(A, n, N, nc, act, st);
+  else if (n <= 32) zgj_go<16, 32, 1, 2>(A, n, N, nc, act, st);
+  else if (n <= 48) zgj_go<16, 24, 2, 3>(A, n, N, nc, act, st);
+  else if (n <= 64) zgj_go<16, 32, 2, 4>(A, n, N, nc, act, st);
+  else k_zgj<<<N, 512, 0, st>>>(A, n, nc, act);
   kstat_end(st);
   SKKR_LAUNCHED();
 }
@@ -457,24 +690,30 @@ void launch_add_tblocks(const MatRef &out, const MatRef &in, const MatRef &t, in
   SKKR_LAUNCHED();
 }
 
-__global__ void k_fnorm(MatRef A, int n, int nc, const int *__restrict__ act, double *out) {
+// One block per matrix, a warp per column, eight loads of a lane in flight
+// (one 256-thread block with a division per element: 42 us for any number of
+// 128-row matrices up to one per SM).  The FP64 pipe's two multiply-adds per
+// element set the floor: 8 us per 128-row matrix and SM.
+__global__ void __launch_bounds__(1024) k_fnorm(MatRef A, int n, int nc, const int *__restrict__ act, double *out) {
   const int item = blockIdx.x;
   const int kk = item / nc, cc = item % nc;
   if (act && !act[item]) return;
   const zd *a = mat_ptr(A, kk, cc);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double s = 0.0;
-  const int tot = n * n;
-  for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-    zd v = a[(e % n) + (long long)(e / n) * A.ld];
-    s += v.x * v.x + v.y * v.y;
-  }
+  for (int r = lane; r < n; r += 32)
+#pragma unroll 8
+    for (int c = w; c < n; c += nw) {
+      const zd v = a[r + (long long)c * A.ld];
+      s = fma(v.x, v.x, fma(v.y, v.y, s));
+    }
   __shared__ double red[32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  if (lane == 0) red[w] = s;
   __syncthreads();
   if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+    s = (int)threadIdx.x < nw ? red[threadIdx.x] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (threadIdx.x == 0) out[item] = sqrt(s);
@@ -484,7 +723,9 @@ __global__ void k_fnorm(MatRef A, int n, int nc, const int *__restrict__ act, do
 void launch_fnorm(const MatRef &a, int n, int nk, int nc, const int *act, double *out,
                   cudaStream_t st) {
   if (nk <= 0 || nc <= 0) return;
-  k_fnorm<<<nk * nc, 256, 0, st>>>(a, n, nc, act, out);
+  // a warp per column of small matrices, at most 32 warps
+  const int th = 32 * std::min(32, std::max(8, n));
+  k_fnorm<<<nk * nc, th, 0, st>>>(a, n, nc, act, out);
   SKKR_LAUNCHED();
 }
 
