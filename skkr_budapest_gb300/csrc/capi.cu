@@ -1104,114 +1104,138 @@ static int run_decimation(skkr_ctx *c, int k0, int nkc, const std::vector<int> &
 }
 
 // ---------------------------------------------------------------------------
-// tau2d (main/tau2d.f) for k in [k0, k0+nkc), items (k, class)
-static int run_tau2d(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls) {
+// Work buffers of the tau2d sweeps per item (k, class): T00[p], YY[p], Yraw[p],
+// XX[p], Xraw[p] (p < nprc), then the pair's matrices W and inverses V.
+static int tau2d_bufs(int nprc) { return 5 * nprc + 4; }
+
+// The sweeps of tau2d (main/tau2d.f:53-109, tau2d_god.f:53-114) for k in
+// [k0, k0+nkc), items (k, class), and the inverses of the diagonal
+// (tau2d.f:114-149): tau(p,p) is left in XX(p), the factors
+// Yr(p) = (T00 - YY)^-1 M01 of p-1 and Xr(p) = (T00 - XX)^-1 M10 of p+1 in
+// theirs.  The forward sweep at p and the backward one at nprc-1-p do not
+// depend on each other, nor do the diagonal inverses: each pair of steps, and
+// the diagonal of as many PLs as 16 classes take, is one batch of twice (or
+// several times) the items.  With three PLs that is three inverses in a row
+// instead of seven, which is what an energy of few k points waits for (21 k
+// points: an inverse of 21 items takes 0.43 ms, one of 63 0.5).
+static int tau2d_sweeps(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls) {
   const int n = c->n, lk = c->lk, lk2 = lk * lk, pl = c->pl, nprc = c->nprc, ni = c->nintfc;
   const int nc = (int)icls.size();
   const long long MB = (long long)n * n;
-  const int nbuf = 5 * nprc + 1;
+  const int nbuf = tau2d_bufs(nprc);
   CKR(c->tauw.ensure((size_t)nkc * nc * nbuf * MB * sizeof(zd)));
-  CKR(c->tauk.ensure((size_t)nkc * nc * ni * lk2 * sizeof(zd)));
   cudaStream_t st = c->st;
   zd *Wb = c->tauw.as<zd>();
-  auto buf = [&](int b) { return mref(Wb + (long long)b * MB, (long long)nc * nbuf * MB, nbuf * MB, n); };
-  // buffers: T00[p]=p, YY[p]=nprc+p, Yraw[p]=2nprc+p, XX[p]=3nprc+p, Xraw[p]=4nprc+p, W=5nprc
-  auto T00 = [&](int p) { return buf(p); };
-  auto YY = [&](int p) { return buf(nprc + p); };
-  auto Yr = [&](int p) { return buf(2 * nprc + p); };
-  auto XX = [&](int p) { return buf(3 * nprc + p); };
-  auto Xr = [&](int p) { return buf(4 * nprc + p); };
-  MatRef Wm = buf(5 * nprc);
+  // classes [0, nc): buffer bf of each item; classes [nc, 2 nc): buffer bb (two < 0: the first half only)
+  auto pair = [&](int bf, int bb) {
+    int map[SKKR_MAPN];
+    for (int s = 0; s < nc; s++) {
+      map[s] = s * nbuf + bf;
+      if (bb >= 0) map[nc + s] = s * nbuf + bb;
+    }
+    return mref_map(Wb, (long long)nc * nbuf * MB, MB, n, map, bb >= 0 ? 2 * nc : nc);
+  };
+  auto T00 = [&](int p) { return p; };
+  auto YY = [&](int p) { return nprc + p; };
+  auto Yr = [&](int p) { return 2 * nprc + p; };
+  auto XX = [&](int p) { return 3 * nprc + p; };
+  auto Xr = [&](int p) { return 4 * nprc + p; };
+  const int W = 5 * nprc, V = 5 * nprc + 2;
   zd *poolk = c->pool.as<zd>();
   const long long psk = (long long)c->nmat * MB;
-  int m00[SKKR_MAPN], m10[SKKR_MAPN], m01[SKKR_MAPN], ysl[SKKR_MAPN], xsl[SKKR_MAPN], tmap[SKKR_MAPN];
+  auto pool = [&](int f, int b) {
+    int map[SKKR_MAPN];
+    for (int s = 0; s < nc; s++) {
+      map[s] = f;
+      map[nc + s] = b;
+    }
+    return mref_map(poolk, psk, MB, n, map, 2 * nc);
+  };
   const int nlay = 2 * pl + ni;
+  int m00[SKKR_MAPN], ysl[SKKR_MAPN], xsl[SKKR_MAPN];
   for (int s = 0; s < nc; s++) {
-    int g = icls[s];
+    const int g = icls[s];
     m00[s] = c->idx00;
-    m10[s] = c->idx10;
-    m01[s] = c->idx01;
     ysl[s] = c->igordl[c->ieqgl[g] - 1] - 1;
     xsl[s] = c->nls + c->igordr[c->ieqgr[g] - 1] - 1;
-    tmap[s] = g * nlay + 2 * pl;  // interface layers of trot[g]
   }
-  MatRef M00 = mref_map(poolk, psk, MB, n, m00, nc);
-  MatRef M10 = mref_map(poolk, psk, MB, n, m10, nc);
-  MatRef M01 = mref_map(poolk, psk, MB, n, m01, nc);
+  const MatRef M00 = mref_map(poolk, psk, MB, n, m00, nc);
   zd *sbase = c->sspo.as<zd>() + (long long)k0 * c->nsl * MB;
-  MatRef Ys = mref_map(sbase, (long long)c->nsl * MB, MB, n, ysl, nc);
-  MatRef Xs = mref_map(sbase, (long long)c->nsl * MB, MB, n, xsl, nc);
-  const bool mx = use_mixed(c, false);
-  // tensor-core engines: M10 and M01 enter every step on the same side,
-  // so they are split once (A slot 1 = M10, B slot 1 = M01, A slot 3 = M01,
-  // B slot 3 = M10); the per-step operands use slot 2
-  const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
-  MixedWork *w = c->mw;
-  const int S = mx ? slices_for(c) : WIDE_SLICES;
-  auto prod = [&](int sa, const MatRef *A, int sb, const MatRef *B, const MatRef &C) -> int {
-    if (A) CKR(mixed_split(w, 0, sa, S, *A, n, n, nkc, nc, nullptr, st));
-    if (B) CKR(mixed_split(w, 1, sb, S, *B, n, n, nkc, nc, nullptr, st));
-    return mixed_gemm_staged(w, 0, S, sa, sb, C, C, C, n, n, nkc, nc, nullptr, st);
-  };
-  if (staged) {
-    CKR(mixed_split(w, 0, 1, S, M10, n, n, nkc, nc, nullptr, st));
-    CKR(mixed_split(w, 1, 1, S, M01, n, n, nkc, nc, nullptr, st, true));
-  }
-  // forward (tau2d.f:53-85)
+  const MatRef Ys = mref_map(sbase, (long long)c->nsl * MB, MB, n, ysl, nc);
+  const MatRef Xs = mref_map(sbase, (long long)c->nsl * MB, MB, n, xsl, nc);
   for (int p = 0; p < nprc; p++) {
     int tm2[SKKR_MAPN];
-    for (int s = 0; s < nc; s++) tm2[s] = tmap[s] + p * pl;
-    MatRef Tt = mref_map(c->trot.as<zd>(), 0, lk2, lk, tm2, nc);
-    launch_add_tblocks(T00(p), M00, Tt, lk, pl, n, nkc, nc, nullptr, ehsplit(c), st);
-    if (p == 0) {
-      launch_zaxpby(YY(0), Ys, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
-    } else if (staged) {
-      MatRef yr = Yr(p);
-      CKR(prod(1, nullptr, 2, &yr, YY(p)));                       // YY = M10 Yr
+    for (int s = 0; s < nc; s++) tm2[s] = icls[s] * nlay + 2 * pl + p * pl;  // interface layers of trot[g]
+    const MatRef Tt = mref_map(c->trot.as<zd>(), 0, lk2, lk, tm2, nc);
+    launch_add_tblocks(pair(T00(p), -1), M00, Tt, lk, pl, n, nkc, nc, nullptr, ehsplit(c), st);
+  }
+  launch_zaxpby(pair(YY(0), -1), Ys, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
+  launch_zaxpby(pair(XX(nprc - 1), -1), Xs, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
+  const bool mx = use_mixed(c, false);
+  // tensor-core engines: the pairs (M10, M01) on the left and (M01, M10) on
+  // the right enter every step, so they are split once (A slot 1, B slot 1);
+  // the per-step operands use slot 2
+  const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
+  MixedWork *w = c->mw;
+  const int S = mx ? slices_for(c) : WIDE_SLICES, nc2 = 2 * nc;
+  const MatRef Ml = pool(c->idx10, c->idx01), Mr = pool(c->idx01, c->idx10);
+  if (staged && nprc > 1) {
+    CKR(mixed_split(w, 0, 1, S, Ml, n, n, nkc, nc2, nullptr, st));
+    CKR(mixed_split(w, 1, 1, S, Mr, n, n, nkc, nc2, nullptr, st, true));
+  }
+  for (int s = 0; s < nprc; s++) {
+    const int p = s, q = nprc - 1 - s;  // forward at p, backward at q
+    if (s > 0) {
+      const MatRef r = pair(Yr(p), Xr(q)), o = pair(YY(p), XX(q));  // YY = M10 Yr, XX = M01 Xr
+      if (staged) {
+        CKR(mixed_split(w, 1, 2, S, r, n, n, nkc, nc2, nullptr, st));
+        CKR(mixed_gemm_staged(w, 0, S, 1, 2, o, o, o, n, n, nkc, nc2, nullptr, st));
+      } else {
+        CKR(eng_gemm(c, mx, 0, Ml, r, o, o, o, n, nkc, nc2, nullptr));
+      }
+    }
+    if (s == nprc - 1) break;
+    const MatRef wm = pair(W, W + 1), vm = pair(V, V + 1), o = pair(Yr(p + 1), Xr(q - 1)), sub = pair(YY(p), XX(q));
+    launch_zaxpby(wm, pair(T00(p), T00(q)), &sub, -1.0, nullptr, 0, n, nkc, nc2, nullptr, st);
+    CKR(eng_inv(c, mx, wm, vm, false, n, nkc, nc2, nullptr));
+    if (staged) {  // Yr(p+1) = V M01, Xr(q-1) = V M10
+      CKR(mixed_split(w, 0, 2, S, vm, n, n, nkc, nc2, nullptr, st));
+      CKR(mixed_gemm_staged(w, 0, S, 2, 1, o, o, o, n, n, nkc, nc2, nullptr, st));
     } else {
-      CKR(eng_gemm(c, mx, 0, M10, Yr(p), YY(p), YY(p), YY(p), n, nkc, nc, nullptr));
-    }
-    if (p < nprc - 1) {
-      MatRef yy = YY(p);
-      launch_zaxpby(Wm, T00(p), &yy, -1.0, nullptr, 0, n, nkc, nc, nullptr, st);
-      CKR(eng_inv(c, mx, Wm, Wm, true, n, nkc, nc, nullptr));
-      if (staged)
-        CKR(prod(2, &Wm, 1, nullptr, Yr(p + 1)));                  // Yr(p+1) = W M01
-      else
-        CKR(eng_gemm(c, mx, 0, Wm, M01, Yr(p + 1), Yr(p + 1), Yr(p + 1), n, nkc, nc, nullptr));
+      CKR(eng_gemm(c, mx, 0, vm, Mr, o, o, o, n, nkc, nc2, nullptr));
     }
   }
-  if (staged) {
-    CKR(mixed_split(w, 0, 3, S, M01, n, n, nkc, nc, nullptr, st));
-    CKR(mixed_split(w, 1, 3, S, M10, n, n, nkc, nc, nullptr, st, true));
+  // tau(p,p) = (T00 - XX - YY)^-1, several PLs per batch: at most as many
+  // classes as the chunk size and the split staging count on
+  const int group = std::max(1, std::min(nprc, 2 * c->ngeff / nc));
+  for (int p0 = 0; p0 < nprc; p0 += group) {
+    const int np = std::min(group, nprc - p0), ng = np * nc;
+    auto many = [&](int b0) {  // class q nc + s: buffer b0 + q of class s
+      int map[SKKR_MAPN];
+      for (int q = 0; q < np; q++)
+        for (int s = 0; s < nc; s++) map[q * nc + s] = s * nbuf + b0 + q;
+      return mref_map(Wb, (long long)nc * nbuf * MB, MB, n, map, ng);
+    };
+    const MatRef t = many(T00(p0)), xx = many(XX(p0)), yy = many(YY(p0));
+    launch_zaxpby(t, t, &xx, -1.0, &yy, -1.0, n, nkc, ng, nullptr, st);
+    CKR(eng_inv(c, mx, t, xx, false, n, nkc, ng, nullptr));
   }
-  // backward (tau2d.f:89-109)
-  for (int p = nprc - 1; p >= 0; p--) {
-    if (p == nprc - 1) {
-      launch_zaxpby(XX(p), Xs, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
-    } else if (staged) {
-      MatRef xr = Xr(p);
-      CKR(prod(3, nullptr, 2, &xr, XX(p)));                       // XX = M01 Xr
-    } else {
-      CKR(eng_gemm(c, mx, 0, M01, Xr(p), XX(p), XX(p), XX(p), n, nkc, nc, nullptr));
-    }
-    if (p > 0) {
-      MatRef xx = XX(p);
-      launch_zaxpby(Wm, T00(p), &xx, -1.0, nullptr, 0, n, nkc, nc, nullptr, st);
-      CKR(eng_inv(c, mx, Wm, Wm, true, n, nkc, nc, nullptr));
-      if (staged)
-        CKR(prod(2, &Wm, 3, nullptr, Xr(p - 1)));                  // Xr(p-1) = W M10
-      else
-        CKR(eng_gemm(c, mx, 0, Wm, M10, Xr(p - 1), Xr(p - 1), Xr(p - 1), n, nkc, nc, nullptr));
-    }
-  }
-  // diagonal blocks (tau2d.f:114-149), weight wk/ngeff
+  return SKKR_OK;
+}
+
+// ---------------------------------------------------------------------------
+// tau2d (main/tau2d.f) for k in [k0, k0+nkc), items (k, class): the sweeps,
+// then the layer-diagonal blocks with weight wk/ngeff
+static int run_tau2d(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls) {
+  const int n = c->n, lk = c->lk, lk2 = lk * lk, pl = c->pl, nprc = c->nprc, ni = c->nintfc;
+  const int nc = (int)icls.size(), nbuf = tau2d_bufs(nprc);
+  const long long MB = (long long)n * n;
+  CKR(c->tauk.ensure((size_t)nkc * nc * ni * lk2 * sizeof(zd)));
+  CKR(tau2d_sweeps(c, k0, nkc, icls));
   for (int p = 0; p < nprc; p++) {
-    MatRef xx = XX(p), yy = YY(p);
-    launch_zaxpby(Wm, T00(p), &xx, -1.0, &yy, -1.0, n, nkc, nc, nullptr, st);
-    CKR(eng_inv(c, mx, Wm, Wm, true, n, nkc, nc, nullptr));
-    launch_extract_tau(Wm, lk, pl, p * pl, c->wk.as<double>() + k0, 1.0 / c->ngeff, c->tauk.as<zd>(),
-                       (long long)nc * ni * lk2, (long long)ni * lk2, nkc, nc, ehsplit(c), st);
+    const MatRef t = mref(c->tauw.as<zd>() + (long long)(3 * nprc + p) * MB, (long long)nc * nbuf * MB, nbuf * MB, n);
+    launch_extract_tau(t, lk, pl, p * pl, c->wk.as<double>() + k0, 1.0 / c->ngeff, c->tauk.as<zd>(),
+                       (long long)nc * ni * lk2, (long long)ni * lk2, nkc, nc, ehsplit(c), c->st);
   }
   return SKKR_OK;
 }
@@ -1223,92 +1247,35 @@ static int run_tau2d(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls)
 // tau(q,p) = dd(q) tau(q+1,p) above (dd(q) = -Yr(q+1)); the signs are applied
 // at the extraction into tauf[item][li][lj][lk^2] (weight wk/ngeff).
 static int run_tau2d_full(skkr_ctx *c, int k0, int nkc, const std::vector<int> &icls, zd *tauf) {
-  const int n = c->n, lk = c->lk, lk2 = lk * lk, pl = c->pl, nprc = c->nprc, ni = c->nintfc;
-  const int nc = (int)icls.size();
+  const int n = c->n, lk2 = c->lk * c->lk, lk = c->lk, pl = c->pl, nprc = c->nprc, ni = c->nintfc;
+  const int nc = (int)icls.size(), nbuf = tau2d_bufs(nprc);
   const long long MB = (long long)n * n;
-  const int nbuf = 5 * nprc + 1;
-  CKR(c->tauw.ensure((size_t)nkc * nc * nbuf * MB * sizeof(zd)));
   cudaStream_t st = c->st;
+  CKR(tau2d_sweeps(c, k0, nkc, icls));
   zd *Wb = c->tauw.as<zd>();
   auto buf = [&](int b) { return mref(Wb + (long long)b * MB, (long long)nc * nbuf * MB, nbuf * MB, n); };
-  auto T00 = [&](int p) { return buf(p); };
-  auto YY = [&](int p) { return buf(nprc + p); };
   auto Yr = [&](int p) { return buf(2 * nprc + p); };
-  auto XX = [&](int p) { return buf(3 * nprc + p); };
   auto Xr = [&](int p) { return buf(4 * nprc + p); };
-  MatRef Wm = buf(5 * nprc);
-  zd *poolk = c->pool.as<zd>();
-  const long long psk = (long long)c->nmat * MB;
-  int m00[SKKR_MAPN], m10[SKKR_MAPN], m01[SKKR_MAPN], ysl[SKKR_MAPN], xsl[SKKR_MAPN], tmap[SKKR_MAPN];
-  const int nlay = 2 * pl + ni;
-  for (int s = 0; s < nc; s++) {
-    int g = icls[s];
-    m00[s] = c->idx00;
-    m10[s] = c->idx10;
-    m01[s] = c->idx01;
-    ysl[s] = c->igordl[c->ieqgl[g] - 1] - 1;
-    xsl[s] = c->nls + c->igordr[c->ieqgr[g] - 1] - 1;
-    tmap[s] = g * nlay + 2 * pl;
-  }
-  MatRef M00 = mref_map(poolk, psk, MB, n, m00, nc);
-  MatRef M10 = mref_map(poolk, psk, MB, n, m10, nc);
-  MatRef M01 = mref_map(poolk, psk, MB, n, m01, nc);
-  zd *sbase = c->sspo.as<zd>() + (long long)k0 * c->nsl * MB;
-  MatRef Ys = mref_map(sbase, (long long)c->nsl * MB, MB, n, ysl, nc);
-  MatRef Xs = mref_map(sbase, (long long)c->nsl * MB, MB, n, xsl, nc);
+  auto tpp = [&](int p) { return buf(3 * nprc + p); };  // tau(p,p)
   const bool mx = use_mixed(c, false);
-  for (int p = 0; p < nprc; p++) {  // forward (tau2d_god.f:53-91)
-    int tm2[SKKR_MAPN];
-    for (int s = 0; s < nc; s++) tm2[s] = tmap[s] + p * pl;
-    MatRef Tt = mref_map(c->trot.as<zd>(), 0, lk2, lk, tm2, nc);
-    launch_add_tblocks(T00(p), M00, Tt, lk, pl, n, nkc, nc, nullptr, ehsplit(c), st);
-    if (p == 0)
-      launch_zaxpby(YY(0), Ys, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
-    else
-      CKR(eng_gemm(c, mx, 0, M10, Yr(p), YY(p), YY(p), YY(p), n, nkc, nc, nullptr));
-    if (p < nprc - 1) {
-      MatRef yy = YY(p);
-      launch_zaxpby(Wm, T00(p), &yy, -1.0, nullptr, 0, n, nkc, nc, nullptr, st);
-      CKR(eng_inv(c, mx, Wm, Wm, true, n, nkc, nc, nullptr));
-      CKR(eng_gemm(c, mx, 0, Wm, M01, Yr(p + 1), Yr(p + 1), Yr(p + 1), n, nkc, nc, nullptr));
-    }
-  }
-  for (int p = nprc - 1; p >= 0; p--) {  // backward (:93-114)
-    if (p == nprc - 1)
-      launch_zaxpby(XX(p), Xs, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
-    else
-      CKR(eng_gemm(c, mx, 0, M01, Xr(p), XX(p), XX(p), XX(p), n, nkc, nc, nullptr));
-    if (p > 0) {
-      MatRef xx = XX(p);
-      launch_zaxpby(Wm, T00(p), &xx, -1.0, nullptr, 0, n, nkc, nc, nullptr, st);
-      CKR(eng_inv(c, mx, Wm, Wm, true, n, nkc, nc, nullptr));
-      CKR(eng_gemm(c, mx, 0, Wm, M10, Xr(p - 1), Xr(p - 1), Xr(p - 1), n, nkc, nc, nullptr));
-    }
-  }
-  // PL-diagonal tau(p,p) in place of T00(p) (:115-119)
-  for (int p = 0; p < nprc; p++) {
-    MatRef t = T00(p), xx = XX(p), yy = YY(p);
-    launch_zaxpby(t, t, &xx, -1.0, &yy, -1.0, n, nkc, nc, nullptr, st);
-    CKR(eng_inv(c, mx, t, t, true, n, nkc, nc, nullptr));
-  }
-  // every PL block, carried from the diagonal (:151-205); YY(0) and XX(0)
+  // every PL block, carried from the diagonal (:151-205); YY(0) and T00(0)
   // serve as the two work matrices
   const double ws = 1.0 / c->ngeff;
   const long long osk = (long long)nc * ni * ni * lk2, osc = (long long)ni * ni * lk2;
   const double *wk = c->wk.as<double>() + k0;
   for (int p = 0; p < nprc; p++) {
-    launch_extract_pairs(T00(p), lk, pl, p * pl, p * pl, ni, wk, ws, tauf, osk, osc, nkc, nc, ehsplit(c), st);
-    MatRef cur = T00(p);
+    launch_extract_pairs(tpp(p), lk, pl, p * pl, p * pl, ni, wk, ws, tauf, osk, osc, nkc, nc, ehsplit(c), st);
+    MatRef cur = tpp(p);
     for (int q = p + 1; q < nprc; q++) {  // below: tau(q,p) = -Xr(q-1) tau(q-1,p)
-      MatRef nxt = ((q - p) & 1) ? YY(0) : XX(0);
+      MatRef nxt = ((q - p) & 1) ? buf(nprc) : buf(0);
       CKR(eng_gemm(c, mx, 0, Xr(q - 1), cur, nxt, nxt, nxt, n, nkc, nc, nullptr));
       launch_extract_pairs(nxt, lk, pl, q * pl, p * pl, ni, wk, ((q - p) & 1) ? -ws : ws, tauf, osk, osc, nkc, nc,
                            ehsplit(c), st);
       cur = nxt;
     }
-    cur = T00(p);
+    cur = tpp(p);
     for (int q = p - 1; q >= 0; q--) {  // above: tau(q,p) = -Yr(q+1) tau(q+1,p)
-      MatRef nxt = ((p - q) & 1) ? YY(0) : XX(0);
+      MatRef nxt = ((p - q) & 1) ? buf(nprc) : buf(0);
       CKR(eng_gemm(c, mx, 0, Yr(q + 1), cur, nxt, nxt, nxt, n, nkc, nc, nullptr));
       launch_extract_pairs(nxt, lk, pl, q * pl, p * pl, ni, wk, ((p - q) & 1) ? -ws : ws, tauf, osk, osc, nkc, nc,
                            ehsplit(c), st);
@@ -1631,7 +1598,7 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
   int kc;
   {
     const int ncmax = 2 * ng;
-    double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + (5.0 * c->nprc + 1) * ng) +
+    double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + tau2d_bufs(c->nprc) * (double)ng) +
                    (double)nc * ni * ni * lk2 * sizeof(zd);
     if (c->mw) {
       const double Mp = 128.0 * ((n + 127) / 128), Np = 64.0 * ((2 * n + 63) / 64), Kp = 32.0 * ((2 * n + 31) / 32);
@@ -1862,7 +1829,7 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   // chunk size: keep the per-chunk work within a fixed budget
   {
     const int ncmax = 2 * c->ngeff;
-    double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + (5.0 * c->nprc + 1) * c->ngeff) +
+    double per_k = (double)MB * sizeof(zd) * (c->nmat + 9.0 * ncmax + tau2d_bufs(c->nprc) * (double)c->ngeff) +
                    (double)c->ngeff * ni * lk2 * sizeof(zd);
     if (c->mw) {
       // BF16 slice staging: up to MIXED_SLOTS operands per side, S slices of

@@ -98,9 +98,10 @@ inline void mref_span(const MatRef &m, int nk, int nc, int cols, long long *lo, 
   *hi = mx + std::max(0LL, ks) + (long long)cols * m.ld;
 }
 // whether two operands' items may share an element: no when their ranges
-// are apart, or when both sit on the same lattice of item offsets (multiples
-// of g = gcd(sk, sc)) with footprints of cols x ld elements that stay apart
-// modulo g (buffers interleaved item by item in one allocation)
+// are apart; when both sit on the same lattice of item offsets (equal sk, sc
+// and ld, and each item's classes within one sk), exactly when an item of one
+// and an item of the other, of the same or a neighbouring k, are closer than a
+// footprint of cols x ld elements
 inline bool mref_overlap(const MatRef &a, const MatRef &b, int nk, int nc, int cols) {
   long long la, ha, lb, hb;
   mref_span(a, nk, nc, cols, &la, &ha);
@@ -109,17 +110,27 @@ inline bool mref_overlap(const MatRef &a, const MatRef &b, int nk, int nc, int c
   const uintptr_t b0 = (uintptr_t)(b.base + lb), b1 = (uintptr_t)(b.base + hb);
   if (!(a0 < b1 && b0 < a1)) return false;
   if (a.sk != b.sk || a.sc != b.sc || a.ld != b.ld) return true;
-  long long g = std::llabs(a.sk), h = std::llabs(a.sc);
-  while (h) {
-    const long long t = g % h;
-    g = h;
-    h = t;
-  }
   const long long fp = (long long)cols * a.ld;
-  if (g < 2 * fp) return true;
   const long long d = ((long long)(intptr_t)((uintptr_t)b.base - (uintptr_t)a.base)) / (long long)sizeof(zd);
-  const long long dm = ((d % g) + g) % g;
-  return !(fp <= dm && dm + fp <= g);
+  // distances of item pairs are d + (k2 - k1) sk + (map_b - map_a) sc
+  long long lo = 0, hi = 0;
+  bool any = false;
+  for (int i = 0; i < nc && i < SKKR_MAPN; i++)
+    for (int j = 0; j < nc && j < SKKR_MAPN; j++) {
+      const long long o = d + (long long)(b.map[j] - a.map[i]) * a.sc;
+      lo = any ? std::min(lo, o) : o;
+      hi = any ? std::max(hi, o) : o;
+      any = true;
+    }
+  const long long sk = std::llabs(a.sk);
+  if (nk > 1 && (sk == 0 || lo <= fp - 2 * sk || hi >= 2 * sk - fp)) return true;  // farther k may meet
+  for (int i = 0; i < nc && i < SKKR_MAPN; i++)
+    for (int j = 0; j < nc && j < SKKR_MAPN; j++)
+      for (int dk = nk > 1 ? -1 : 0; dk <= (nk > 1 ? 1 : 0); dk++) {
+        const long long o = d + dk * sk + (long long)(b.map[j] - a.map[i]) * a.sc;
+        if (o < fp && o > -fp) return true;
+      }
+  return false;
 }
 
 // One process-wide lock between CUDA graph capture and the calls that may
