@@ -144,11 +144,11 @@ int skkr_gpu_set_mixed_policy(skkr_ctx *ctx, double dec_fp64_im, double near_im,
  * whose FP32 start is already that close. */
 int skkr_gpu_set_newton(skkr_ctx *ctx, int steps);
 
-/* The FP32 start of split-precision inverses above 64 rows: blocked != 0
- * (the default) forms it by 2 x 2 blocks (two 64-row Gauss-Jordan inverses
- * with pivoting inside each block, six FP32 block products); 0 runs the
- * Gauss-Jordan of main/gjinv.f's column pivoting on the whole matrix.  The
- * Newton steps, their acceptance test and the FP64 redo are the same. */
+/* Accepted for programs that chose between two FP32 starts of split-precision
+ * inverses above 64 rows (2 x 2 blocks, or the Gauss-Jordan on the whole
+ * matrix); both values run the whole-matrix Gauss-Jordan with the column
+ * pivoting of main/gjinv.f, which is now the faster one at every size and
+ * the more accurate start. */
 int skkr_gpu_set_inverse_start(skkr_ctx *ctx, int blocked);
 
 /* The B operand of every split-precision product: on
@@ -159,11 +159,11 @@ int skkr_gpu_set_inverse_start(skkr_ctx *ctx, int blocked);
 int skkr_gpu_set_fused_split(skkr_ctx *ctx, int on);
 
 /* Autotuner of the split-precision inverse's FP32 Gauss-Jordan: each size
- * class (n <= 32, 64, 128) has 2-3 thread layouts that give the same inverse
+ * class (n <= 32, 64, 96, 128) has two thread layouts that give the same inverse
  * bit for bit; the first batch of each (class, batch size) times them (best
  * of three runs each; a later layout must be 5 % faster to be chosen) and
  * later calls use the choice (process wide).  report (may be NULL)
- * receives the choices so far, e.g. "n<=128 >=4 waves: 64x2x8; ".
+ * receives the choices so far, e.g. "n<=128 >=4 waves: 12+4 warps; ".
  * force > 0 makes every class use its layout force - 1 (tests); force = 0
  * with report NULL forgets the choices and tunes afresh. */
 int skkr_gpu_autotune(int force, char *report, int len);

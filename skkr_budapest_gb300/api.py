@@ -61,8 +61,8 @@ class Context:
         N._check(N.lib().skkr_gpu_set_newton(self.h, int(steps)), "skkr_gpu_set_newton")
 
     def set_inverse_start(self, blocked=True):
-        """FP32 start of split-precision inverses above 64 rows: 2 x 2 blocks
-        (default) or the whole-matrix Gauss-Jordan (skkr_gpu_set_inverse_start)."""
+        """Accepted; both values run the whole-matrix Gauss-Jordan start
+        (skkr_gpu_set_inverse_start)."""
         N._check(N.lib().skkr_gpu_set_inverse_start(self.h, 1 if blocked else 0), "skkr_gpu_set_inverse_start")
 
     def set_fused_split(self, on=True):

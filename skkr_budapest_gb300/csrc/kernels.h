@@ -109,8 +109,6 @@ constexpr int NEWTON_EXTRA = 4;
 // that several products read is split once into its slot instead
 int mixed_split(MixedWork *w, int side, int slot, int S, const MatRef &M, int n, int K, int nk, int nc,
                 const int *act, cudaStream_t st, bool reused = false);
-// the 2 x 2 block FP32 start of inverses above 64 rows (default on)
-void mixed_set_blocked(MixedWork *w, bool on);
 // B operands formed by the products themselves (default on)
 void mixed_set_fused(MixedWork *w, bool on);
 int mixed_gemm_staged(MixedWork *w, int mode, int S, int sa, int sb, const MatRef &C, const MatRef &D,

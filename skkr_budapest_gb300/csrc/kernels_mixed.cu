@@ -940,25 +940,39 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_ozaki(const __grid_constan
 // ------------------------------------------------------------------ FP32 GJ
 // Gauss-Jordan with column pivoting (main/gjinv.f: in row i the pivot is the
 // largest |a(i, j)| over the columns not yet used, first index on ties) in
-// complex FP32, the matrix held in registers: TY*16 threads as a TY x 16
-// grid, thread (ty, tx) owning rows ty + TY a (a < RA) and columns
-// tx + 16 b (b < RB); the 16 threads of one ty are one half warp.
+// complex FP32, in panels of eight rows.  The pivot columns are not swapped
+// into place: step i eliminates with the pivot (i, kp) where it lies and
+// records sigma(i) = kp, which is Gauss-Jordan on A P (P the column
+// permutation); the array then holds (A P)^-1 with its columns stored at the
+// positions of A P's, so A^-1(sigma(r), c) is found at (r, sigma(c)) and the
+// store permutes both indices.  The result (written as FP64) only seeds the
+// Newton refinement.
 //
-// The pivot columns are not swapped into place: step i eliminates with the
-// pivot (i, kp) where it lies and records sigma(i) = kp, which is Gauss-Jordan
-// on A P (P the column permutation); the array then holds (A P)^-1 with its
-// columns stored at the positions of A P's, so A^-1(sigma(r), c) is found at
-// (r, sigma(c)) and the store permutes both indices.  With
-//   c_r = a(r,kp)/piv (r != i), c_i = -1/piv,   p_j = a(i,j) (j != kp), p_kp = 1
-// and row i and column kp masked to zero first, every element takes the same
-// update a(r,j) <- s(r,j) a(r,j) - c_r p_j (s = 0 on row i and column kp,
-// else 1): the rank-1 update, the scaled pivot row a(i,j)/piv, the pivot
-// column -a(r,kp)/piv and the pivot 1/piv, as packed FP32x2 multiply-adds.
-// a(r,kp) comes from the owner in the same half warp (a shuffle); the pivot
-// row and the next pivot index are staged in shared memory (double-buffered)
-// by the 16 threads that own row i+1 after their update: one block barrier
-// per step.  The result
-// (written as FP64) only seeds the Newton refinement.
+// The last N / 32 warps factor the panel: a lane holds one column of the eight
+// rows in registers, and eight Gauss-Jordan steps run on those rows alone.
+// With the panel P (eight rows of the inverse tableau) and its pivot columns
+// K, every other row takes one update of depth eight,
+//   a(r, :) <- (a(r, :) with the columns K zeroed) - sum_q a(r, K_q) P(q, :),
+// and the panel's own rows become P.  The other
+// W warps do that on the matrix in shared memory (column-major): a warp takes
+// four columns at a time, a lane the rows lane + 32 a, with the lane's
+// multipliers in registers and P broadcast.  Each warp forms its columns of
+// the next panel's rows first and hands them over, so that the next panel is
+// factored while the update runs.
+//
+// Why panels: a rank-1 update per pivot needs a block barrier, the pivot
+// search and the multipliers' selects every step, 1750 clocks of which 128
+// were multiply-adds (n = 64); in panels a step takes one barrier of N / 32
+// warps and a chain of about 300 clocks, beside the update.  Why shared
+// memory: the columns K and the rows of a panel lie at run-time indices, which
+// registers answer with selects over the whole tile (45 us for 42 items of
+// n = 64).  Before and after: 57 and 30 us (42 items of n = 64), 99 and 57
+// (420), 277 and 149 (1640 of n = 54).  At n = 128 the whole matrix takes
+// 104 us (42 items, one wave) and 305 us (420), where the 2 x 2 block form on
+// 64-row inverses took 214 and 468 (and would take 160 and 384 on this one).
+// The FP32 multiply-adds alone are 32 us a wave at n = 128; loading and
+// storing with conversions (two a clock per SM) 16, the panel chain and the
+// barriers the rest.
 
 __device__ __forceinline__ unsigned long long pk2(float x, float y) {
   unsigned long long r;
@@ -976,256 +990,261 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
+constexpr int GJ_NB = 8;                                         // rows of a panel
+constexpr int GJ_BAR_PANEL = 1, GJ_BAR_RAW = 2, GJ_BAR_MUL = 3, GJ_BAR_STEP = 4;  // named barriers
+
+template <int ID>
+__device__ __forceinline__ void bar_sync_n(int threads) {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void bar_arrive_n(int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 
-// Pivot of row `row` among the unused columns (the row's owners: one half
-// warp): the largest |a(row, j)|^2, first index on ties; the row is staged
-// into `rowbuf` on the way.  Every candidate NaN: the first unused column.
-template <int TY, int RA, int RB>
-__device__ __forceinline__ void gj_search(const unsigned long long (&m)[RA][RB], int row, unsigned used, int tx,
-                                          unsigned hmask, float2 *rowbuf, int *kp_out) {
-  const int iar = row / TY;
-  float best = -1.f;
-  int bj = 0x7FFFFFFF, fu = 0x7FFFFFFF;
-#pragma unroll
-  for (int ib = 0; ib < RB; ib++) {
-    unsigned long long w = m[0][ib];
-#pragma unroll
-    for (int ia = 1; ia < RA; ia++) w = (ia == iar) ? m[ia][ib] : w;  // static indices keep m in registers
-    const float2 v = upk2(w);
-    const int j = tx + 16 * ib;
-    rowbuf[j] = v;
-    const bool free = !((used >> ib) & 1u);
-    const float mm = v.x * v.x + v.y * v.y;
-    const bool ok = free && (mm > best || (mm == best && j < bj));
-    best = ok ? mm : best;
-    bj = ok ? j : bj;
-    fu = (free && j < fu) ? j : fu;
-  }
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(hmask, best, o, 16);
-    const int oj = __shfl_xor_sync(hmask, bj, o, 16);
-    const int of = __shfl_xor_sync(hmask, fu, o, 16);
-    const bool take = ob > best || (ob == best && oj < bj);
-    best = take ? ob : best;
-    bj = take ? oj : bj;
-    fu = of < fu ? of : fu;
-  }
-  if (bj == 0x7FFFFFFF) bj = fu;
-  if (tx == 0) *kp_out = bj;
-}
-
-// MINB: blocks per SM the register allocation must allow (the 64-row
-// layouts run several matrices per SM, each block's barrier latency hidden by
-// the others)
-template <int TY, int RA, int RB, int MINB = 1>
-__global__ void __launch_bounds__(TY * 16, MINB) k_cgj32(MatRef A, MatRef X, int n, int nc,
-                                                      const int *__restrict__ act) {
-  constexpr int NR = TY * RA, NCOL = 16 * RB;
-  const int item = blockIdx.x, kk = item / nc, cc = item % nc;
-  if (act && !act[item]) return;
-  __shared__ float2 rowi[2][NCOL];
-  __shared__ int sig[NR], sinv[NCOL];
-  __shared__ int kpn[2];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const zd *a = mat_ptr(A, kk, cc);
-  unsigned long long m[RA][RB];  // (re, im) pairs
-#pragma unroll
-  for (int ia = 0; ia < RA; ia++)
-#pragma unroll
-    for (int ib = 0; ib < RB; ib++) {
-      const int r = ty + TY * ia, j = tx + 16 * ib;
-      float2 v = make_float2(0.f, 0.f);
-      if (r < n && j < n) {
-        const zd w = a[r + (long long)j * A.ld];
-        v = make_float2((float)w.x, (float)w.y);
-      }
-      m[ia][ib] = pk2(v.x, v.y);
-    }
-  // columns j >= n never pivot
-  unsigned used = 0;
-#pragma unroll
-  for (int ib = 0; ib < RB; ib++)
-    if (tx + 16 * ib >= n) used |= 1u << ib;
-  const unsigned hmask = (ty & 1) ? 0xFFFF0000u : 0x0000FFFFu;  // the 16 threads of this ty
-
-  if (ty == 0) gj_search<TY, RA, RB>(m, 0, used, tx, hmask, rowi[0], &kpn[0]);
-  __syncthreads();
-  for (int i = 0; i < n; i++) {
-    const int kp = kpn[i & 1], kb = kp >> 4, kt = kp & 15;
-    if (tid == 0) {
-      sig[i] = kp;
-      sinv[kp] = i;
-    }
-    if (tx == kt) used |= 1u << kb;
-    const float2 *ri = rowi[i & 1];
-    const float2 piv = ri[kp];
-    const float rden = __frcp_rn(piv.x * piv.x + piv.y * piv.y);
-    const float2 q = make_float2(piv.x * rden, -piv.y * rden);
-    // multipliers c_r as the pairs (-Re c, -Re c) and (Im c, Im c); row mask
-    unsigned long long ncx[RA], cy[RA];
-    float f[RA];
-#pragma unroll
-    for (int ia = 0; ia < RA; ia++) {
-      unsigned long long w = m[ia][0];
-#pragma unroll
-      for (int ib = 1; ib < RB; ib++) w = (ib == kb) ? m[ia][ib] : w;
-      w = __shfl_sync(0xFFFFFFFFu, w, kt, 16);  // a(r, kp) from its owner in this half warp
-      const float2 v = upk2(w);
-      const bool isrow = ty + TY * ia == i;
-      const float2 cr = isrow ? make_float2(-q.x, -q.y)
-                              : make_float2(v.x * q.x - v.y * q.y, v.x * q.y + v.y * q.x);
-      ncx[ia] = pk2(-cr.x, -cr.x);
-      cy[ia] = pk2(cr.y, cr.y);
-      f[ia] = isrow ? 0.f : 1.f;
-    }
-    // row i+1's owners reduce the next pivot after their update
-    const bool srch = i + 1 < n && ty == ((i + 1) % TY);
-#pragma unroll
-    for (int ib = 0; ib < RB; ib++) {
-      const int j = tx + 16 * ib;
-      const bool iscol = j == kp;
-      const float2 p = iscol ? make_float2(1.f, 0.f) : ri[j];
-      const float g = iscol ? 0.f : 1.f;
-      const unsigned long long pp = pk2(p.x, p.y), ps = pk2(p.y, -p.x);
-#pragma unroll
-      for (int ia = 0; ia < RA; ia++) {
-        const float sm = f[ia] * g;
-        const unsigned long long t = fma2(cy[ia], ps, mul2(ncx[ia], pp));
-        m[ia][ib] = fma2(m[ia][ib], pk2(sm, sm), t);
-      }
-    }
-    if (srch) gj_search<TY, RA, RB>(m, i + 1, used, tx, hmask, rowi[(i + 1) & 1], &kpn[(i + 1) & 1]);
-    __syncthreads();
-  }
-  // storage (r, j) holds A^-1(sigma(r), sigma^-1(j))
-  zd *x = mat_ptr(X, kk, cc);
-#pragma unroll
-  for (int ia = 0; ia < RA; ia++)
-#pragma unroll
-    for (int ib = 0; ib < RB; ib++) {
-      const int r = ty + TY * ia, j = tx + 16 * ib;
-      if (r < n && j < n) {
-        const float2 v = upk2(m[ia][ib]);
-        x[sig[r] + (long long)sinv[j] * X.ld] = make_double2((double)v.x, (double)v.y);
-      }
-    }
-}
-
-// ------------------------------------------------------------------ FP32 block products
-// C = A B (m x n, depth k; m, n, k <= 64) of one item per block in complex
-// FP32 from FP64 operands, for the 2 x 2 block start of the split-precision
-// inverse: mode 0 C = AB, 1 C = D - AB (D read in FP64), 2 C = -AB.  Up to
-// two independent products per launch (blockIdx.y picks one).  The 16 x 16
-// threads each hold 4 x 4 outputs (rows ty + 16 i, columns tx + 16 j) as two
-// packed FP32 pairs each (two fma.rn.f32x2 per complex multiply-add); the
-// operands pass through shared memory in K chunks of 32, converted to FP32
-// on the way; the sums run in a fixed order.
-struct G32Job {
-  MatRef A, B, C, D;
-  int m, n, k, mode;
-};
-struct G32Jobs {
-  G32Job j[2];
+// N: rows and columns, padded to 32.  The leading dimension N + 8 puts the
+// eight rows of a panel in four neighbouring columns on different banks.
+template <int N>
+struct GjShared {
+  unsigned long long m[N][N + 8];  // [column][row], (re, im) pairs
+  alignas(16) unsigned long long p[2][N][GJ_NB + 2];  // the panel, handed over and back: [column][row] (80 bytes a column: no
+                                          // bank conflicts between eight columns)
+  ulonglong2 pcol[2][N / 32][GJ_NB / 2 + 1];  // proposed pivot columns of a step, 1/pivot
+  unsigned pkey[2][N / 32];        // and their keys
+  alignas(16) int slot[2][N];      // q of a panel's pivot column, else -1
+  int kcol[2][GJ_NB];              // pivot columns of a panel
+  int sig[N], sinv[N];
 };
 
-__global__ void __launch_bounds__(256, 2) k_cgemm32(G32Jobs jobs, int nc, const int *__restrict__ act) {
+// 1/x to an ulp without the branches of the rounded reciprocal (0 and the
+// infinite: NaN, as good a mark of a lost start)
+__device__ __forceinline__ float gj_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
+// Eight Gauss-Jordan steps on the panel of rows i0 .. i0 + 7, column j in this
+// thread.  Each warp proposes the best pivot of its 32 columns together with
+// its column and reciprocal, so that a step takes one barrier of the panel
+// warps.  used: this column has been a pivot (or is >= n).  Rows >= n are unit
+// rows and pivot on themselves.
+template <int N>
+__device__ __forceinline__ void gj_panel(GjShared<N> &sh, int buf, int i0, int n, int j, bool &used) {
+  constexpr int PW = N / 32;
+  const int pw = j >> 5, lane = j & 31;
+  unsigned long long v[GJ_NB];
+#pragma unroll
+  for (int q = 0; q < GJ_NB; q++) v[q] = sh.p[buf][j][q];
+  int mine = -1;
+#pragma unroll
+  for (int q = 0; q < GJ_NB; q++) {
+    const int i = i0 + q;
+    // largest |a(i, j)|^2 over the unused columns: its bits order as integers;
+    // the last seven carry the column (first index on ties, that is within
+    // 2^-16), so that one reduction gives both.  NaN comes last.
+    const float2 w = upk2(v[q]);
+    const float mm = w.x * w.x + w.y * w.y;
+    const unsigned inv = 127u - (unsigned)j;
+    unsigned key = mm >= 0.f ? ((__float_as_uint(mm) | 0x80000000u) & ~127u) | inv : 128u | inv;
+    key = used ? 0u : key;
+    key = i < n ? key : j == i ? 0xFFFFFF80u | inv : 0u;
+    const float rden = gj_rcp(mm);
+    unsigned kmax = __reduce_max_sync(0xFFFFFFFFu, key);
+    ulonglong2(&pc)[PW][GJ_NB / 2 + 1] = sh.pcol[q & 1];
+    if (key == kmax && key != 0u) {
+#pragma unroll
+      for (int r = 0; r < GJ_NB; r += 2) pc[pw][r / 2] = make_ulonglong2(v[r], v[r + 1]);
+      pc[pw][GJ_NB / 2].x = pk2(w.x * rden, -w.y * rden);
+    }
+    int win = 0;
+    if (PW > 1) {
+      if (lane == 0) sh.pkey[q & 1][pw] = kmax;
+      bar_sync_n<GJ_BAR_STEP>(PW * 32);
+      kmax = sh.pkey[q & 1][0];
+#pragma unroll
+      for (int o = 1; o < PW; o++) {
+        const unsigned k = sh.pkey[q & 1][o];
+        win = k > kmax ? o : win;
+        kmax = k > kmax ? k : kmax;
+      }
+    } else {
+      __syncwarp();
+    }
+    const int kp = 127 - (int)(kmax & 127u);
+    const float2 d = upk2(pc[win][GJ_NB / 2].x);
+    float2 c[GJ_NB];
+#pragma unroll
+    for (int r = 0; r < GJ_NB; r += 2) {
+      const ulonglong2 t = pc[win][r / 2];
+      c[r] = upk2(t.x);
+      c[r + 1] = upk2(t.y);
+    }
+    const bool hit = j == kp;
+    if (hit) {
+      used = true;
+      mine = q;
+      sh.sig[i] = kp;
+      sh.sinv[kp] = i;
+      sh.kcol[buf][q] = kp;
+    }
+    // the pivot row times 1/pivot, then the other rows minus a(r, kp) times
+    // it; the pivot column starts from the unit column
+    const float2 x = hit ? make_float2(1.f, 0.f) : w;
+    const float2 o = make_float2(x.x * d.x - x.y * d.y, x.x * d.y + x.y * d.x);
+    v[q] = pk2(o.x, o.y);
+    const unsigned long long ps = pk2(o.y, -o.x);
+#pragma unroll
+    for (int rr = 1; rr < GJ_NB; rr++) {
+      const int r = (q + rr) % GJ_NB;  // the next pivot row first
+      v[r] = fma2(pk2(c[r].y, c[r].y), ps, fma2(pk2(-c[r].x, -c[r].x), v[q], hit ? 0ull : v[r]));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < GJ_NB; q += 2) *reinterpret_cast<ulonglong2 *>(&sh.p[buf][j][q]) = make_ulonglong2(v[q], v[q + 1]);
+  sh.slot[buf][j] = mine;
+}
+
+// u -= c p
+__device__ __forceinline__ void gj_fms(float2 &u, float2 c, float2 p) {
+  u.x = fmaf(-c.x, p.x, u.x);
+  u.y = fmaf(-c.x, p.y, u.y);
+  u.x = fmaf(c.y, p.y, u.x);
+  u.y = fmaf(-c.y, p.x, u.y);
+}
+
+static_assert(offsetof(GjShared<32>, slot) % 16 == 0 && offsetof(GjShared<64>, slot) % 16 == 0 &&
+                  offsetof(GjShared<96>, slot) % 16 == 0 && offsetof(GjShared<128>, slot) % 16 == 0 &&
+                  offsetof(GjShared<96>, p) % 16 == 0 && offsetof(GjShared<96>, pcol) % 16 == 0,
+              "16-byte shared loads");
+
+// RA rows a lane (N = 32 RA), W update warps, MINB blocks per SM
+template <int RA, int W, int MINB>
+__global__ void __launch_bounds__((W + RA) * 32, MINB) k_cgj32(const __grid_constant__ MatRef A,
+                                                            const __grid_constant__ MatRef X, int n, int nc,
+                                                            const int *__restrict__ act) {
+  constexpr int N = 32 * RA, T = W * 32, TALL = T + N;
   const int item = blockIdx.x, kk = item / nc, cc = item % nc;
   if (act && !act[item]) return;
-  const G32Job &J = jobs.j[blockIdx.y];
-  const int m = J.m, n = J.n, k = J.k;
-  __shared__ float2 As[32][64];  // [K index][row]
-  __shared__ float2 Bs[32][65];  // [K index][column], padded against store conflicts
-  const zd *a = mat_ptr(J.A, kk, cc), *b = mat_ptr(J.B, kk, cc);
-  const int lda = J.A.ld, ldb = J.B.ld;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // packed FP32 pairs: pr = (sum ar br, sum ar bi), pi = (sum ai br, sum ai bi)
-  // on the (br, bi) pair as it sits in shared memory; the product is
-  // (pr.x - pi.y, pr.y + pi.x)
-  unsigned long long pr[4][4], pi[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) pr[i][j] = pi[i][j] = 0ull;
-  for (int k0 = 0; k0 < k; k0 += 32) {
-    for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-      const int r = e & 63, q = e >> 6, col = k0 + q;
-      const zd v = (r < m && col < k) ? a[r + (long long)col * lda] : make_double2(0.0, 0.0);
-      As[q][r] = make_float2((float)v.x, (float)v.y);
+  extern __shared__ __align__(16) char gj_smem[];
+  GjShared<N> &sh = *reinterpret_cast<GjShared<N> *>(gj_smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, np = (n + GJ_NB - 1) / GJ_NB, ncols = np * GJ_NB;
+  if (w >= W) {  // the panel warps
+    const int j = threadIdx.x - T;
+    bool used = j >= n;
+    for (int p = 0; p < np; p++) {
+      bar_sync_n<GJ_BAR_RAW>(TALL);  // the rows of panel p are in p[p & 1]
+      gj_panel<N>(sh, p & 1, p * GJ_NB, n, j, used);
+      bar_arrive_n<GJ_BAR_PANEL>(TALL);
     }
-    for (int e = threadIdx.x; e < 32 * 64; e += 256) {
-      const int q = e & 31, c = e >> 5, row = k0 + q;
-      const zd v = (row < k && c < n) ? b[row + (long long)c * ldb] : make_double2(0.0, 0.0);
-      Bs[q][c] = make_float2((float)v.x, (float)v.y);
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int q = 0; q < 32; q++) {
-      unsigned long long bv[4];
+    return;
+  }
+  {
+    const zd *a = mat_ptr(A, kk, cc);
+    constexpr int LB = RA >= 3 ? 2 : 4;  // columns in flight
+    for (int j0 = w; j0 < N; j0 += LB * W) {
+      zd z[LB][RA];
 #pragma unroll
-      for (int j = 0; j < 4; j++) bv[j] = *reinterpret_cast<const unsigned long long *>(&Bs[q][tx + 16 * j]);
+      for (int e = 0; e < LB; e++)
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float2 a = As[q][ty + 16 * i];
-        const unsigned long long ar = pk2(a.x, a.x), ai = pk2(a.y, a.y);
+        for (int ia = 0; ia < RA; ia++) {
+          const int r = lane + 32 * ia, j = j0 + e * W;
+          z[e][ia] = r < n && j < n ? a[r + (long long)j * A.ld] : make_double2(r == j ? 1.0 : 0.0, 0.0);
+        }
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          pr[i][j] = fma2(ar, bv[j], pr[i][j]);
-          pi[i][j] = fma2(ai, bv[j], pi[i][j]);
+      for (int e = 0; e < LB; e++) {
+        const int j = j0 + e * W;
+        if (j >= N) break;
+#pragma unroll
+        for (int ia = 0; ia < RA; ia++) {
+          const unsigned long long v = pk2((float)z[e][ia].x, (float)z[e][ia].y);
+          sh.m[j][lane + 32 * ia] = v;
+          if (ia == 0 && lane < GJ_NB) {
+            sh.p[0][j][lane] = v;
+            sh.p[1][j][lane] = 0ull;  // (columns past ncols stay so)
+          }
         }
       }
     }
-    __syncthreads();
   }
-  zd *c = mat_ptr(J.C, kk, cc);
-  const int ldc = J.C.ld, mode = J.mode;
-  const zd *d = mode == 1 ? mat_ptr(J.D, kk, cc) : nullptr;
-  const int ldd = J.D.ld;
+  bar_arrive_n<GJ_BAR_RAW>(TALL);
+  for (int p = 0; p < np; p++) {
+    const int i0 = p * GJ_NB, buf = p & 1;
+    bar_sync_n<GJ_BAR_PANEL>(TALL);  // panel p factored, every earlier update finished
+    int kc[GJ_NB];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+    for (int q = 0; q < GJ_NB; q++) kc[q] = sh.kcol[buf][q];
+    if (p + 1 < np) {  // the next panel's rows: eight rows, four columns a warp
+      const int rn = lane & 7, r1 = i0 + GJ_NB + rn;
+      float2 cn[GJ_NB];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int r = ty + 16 * i, col = tx + 16 * j;
-      if (r < m && col < n) {
-        const float2 u = upk2(pr[i][j]), v = upk2(pi[i][j]);
-        const zd p = make_double2((double)(u.x - v.y), (double)(u.y + v.x));
-        zd o;
-        if (mode == 0) o = p;
-        else if (mode == 1) {
-          const zd dv = d[r + (long long)col * ldd];
-          o = make_double2(dv.x - p.x, dv.y - p.y);
-        } else o = make_double2(-p.x, -p.y);
-        c[r + (long long)col * ldc] = o;
+      for (int q = 0; q < GJ_NB; q++) cn[q] = upk2(sh.m[kc[q]][r1]);
+      for (int j = 4 * w + (lane >> 3); j < ncols; j += 4 * W) {
+        float2 u = upk2(sh.slot[buf][j] < 0 ? sh.m[j][r1] : 0ull);
+#pragma unroll
+        for (int q = 0; q < GJ_NB; q += 2) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(&sh.p[buf][j][q]);
+          gj_fms(u, cn[q], upk2(t.x));
+          gj_fms(u, cn[q + 1], upk2(t.y));
+        }
+        sh.p[buf ^ 1][j][rn] = pk2(u.x, u.y);
+      }
+      bar_arrive_n<GJ_BAR_RAW>(TALL);
+    }
+    float2 c[GJ_NB][RA];  // (of the panel's own rows too: they are overwritten below)
+#pragma unroll
+    for (int q = 0; q < GJ_NB; q++)
+#pragma unroll
+      for (int ia = 0; ia < RA; ia++) c[q][ia] = upk2(sh.m[kc[q]][lane + 32 * ia]);
+    bar_sync_n<GJ_BAR_MUL>(T);  // multipliers and next rows read: the matrix may change
+    for (int j0 = 4 * w; j0 < ncols; j0 += 4 * W) {
+      const int4 sl = *reinterpret_cast<const int4 *>(&sh.slot[buf][j0]);
+      const int sle[4] = {sl.x, sl.y, sl.z, sl.w};
+      if ((sl.x & sl.y & sl.z & sl.w) >= 0) {  // a column of K among them
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          if (sle[e] >= 0)
+#pragma unroll
+            for (int ia = 0; ia < RA; ia++) sh.m[j0 + e][lane + 32 * ia] = 0ull;
+      }
+      float2 u[4][RA];
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+#pragma unroll
+        for (int ia = 0; ia < RA; ia++) u[e][ia] = upk2(sh.m[j0 + e][lane + 32 * ia]);
+#pragma unroll
+      for (int q = 0; q < GJ_NB; q += 2)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(&sh.p[buf][j0 + e][q]);
+#pragma unroll
+          for (int ia = 0; ia < RA; ia++) gj_fms(u[e][ia], c[q][ia], upk2(t.x));
+#pragma unroll
+          for (int ia = 0; ia < RA; ia++) gj_fms(u[e][ia], c[q + 1][ia], upk2(t.y));
+        }
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+#pragma unroll
+        for (int ia = 0; ia < RA; ia++) sh.m[j0 + e][lane + 32 * ia] = pk2(u[e][ia].x, u[e][ia].y);
+      __syncwarp();
+      sh.m[j0 + (lane >> 3)][i0 + (lane & 7)] = sh.p[buf][j0 + (lane >> 3)][lane & 7];  // the panel's rows
+    }
+  }
+  bar_sync_n<GJ_BAR_MUL>(T);
+  // place (r, j) holds A^-1(sigma(r), sigma^-1(j))
+  zd *x = mat_ptr(X, kk, cc);
+#pragma unroll 4
+  for (int j = w; j < n; j += W) {
+    const unsigned long long *col = sh.m[sh.sig[j]];
+#pragma unroll
+    for (int ia = 0; ia < RA; ia++) {
+      const int r = lane + 32 * ia;
+      if (r < n) {
+        const float2 v = upk2(col[sh.sinv[r]]);
+        x[r + (long long)j * X.ld] = make_double2((double)v.x, (double)v.y);
       }
     }
-}
-
-static G32Job g32(int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D, int m, int n,
-                  int k) {
-  G32Job j;
-  j.A = A;
-  j.B = B;
-  j.C = C;
-  j.D = D;
-  j.m = m;
-  j.n = n;
-  j.k = k;
-  j.mode = mode;
-  return j;
-}
-
-// one or two products per launch
-static void cgemm32(const G32Job &j0, const G32Job *j1, int nc, const int *act, unsigned items, cudaStream_t st) {
-  G32Jobs js;
-  js.j[0] = j0;
-  js.j[1] = j1 ? *j1 : j0;
-  k_cgemm32<<<dim3(items, j1 ? 2 : 1), 256, 0, st>>>(js, nc, act);
-  SKKR_LAUNCHED();
+  }
 }
 
 // ------------------------------------------------------------------ host side
@@ -1332,10 +1351,8 @@ struct MixedWork {
                                        // IF bodies of captured further steps (device counts)
   cudaStream_t side = nullptr;         // captures the bodies of conditional graph nodes
   bool fuse_b = true;      // B operands formed inside the product (mixed_set_fused)
-  bool blocked = true;     // 2 x 2 block start of inverses above 64 rows (mixed_set_blocked)
 };
 
-void mixed_set_blocked(MixedWork *w, bool on) { w->blocked = on; }
 void mixed_set_fused(MixedWork *w, bool on) { w->fuse_b = on; }
 
 // the callers' streams are non-blocking: free the old buffer only once the
@@ -1708,7 +1725,8 @@ bool stream_capturing(cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 // Autotuned thread layout of the FP32 Gauss-Jordan.  A size class fixes the
-// columns per thread (16 RB >= n); the rows split over TY x RA threads.  Every
+// rows per lane (32 RA >= n); its layouts differ in the number of update
+// warps and in the blocks per SM.  Every
 // layout gives the same inverse bit for bit (each element takes the same
 // sequence of updates, the pivot search is deterministic), so the first
 // batch of each (size class, batch size) key times the layouts once on the
@@ -1716,23 +1734,27 @@ bool stream_capturing(cudaStream_t st) {
 // before a key is tuned takes the first layout.
 using GjLaunch = void (*)(const MatRef &, const MatRef &, int, int, const int *, unsigned, cudaStream_t);
 
-template <int TY, int RA, int RB, int MINB = 1>
+template <int RA, int W, int MINB>
 static void gj_launch(const MatRef &A, const MatRef &X, int n, int nc, const int *act, unsigned items,
                       cudaStream_t st) {
-  k_cgj32<TY, RA, RB, MINB><<<items, TY * 16, 0, st>>>(A, X, n, nc, act);
+  constexpr size_t smem = sizeof(GjShared<32 * RA>);
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(k_cgj32<RA, W, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_cgj32<RA, W, MINB><<<items, (W + RA) * 32, smem, st>>>(A, X, n, nc, act);
 }
 
 struct GjClass {
   int nmax;
   int nv;
-  GjLaunch f[3];
-  const char *name[3];
+  GjLaunch f[2];
+  const char *name[2];
 };
 
-static const GjClass GJ_CLASSES[3] = {
-    {32, 3, {gj_launch<16, 2, 2>, gj_launch<32, 1, 2>, gj_launch<8, 4, 2>}, {"16x2x2", "32x1x2", "8x4x2"}},
-    {64, 3, {gj_launch<16, 4, 4, 3>, gj_launch<32, 2, 4, 2>, gj_launch<64, 1, 4>}, {"16x4x4 (3/SM)", "32x2x4 (2/SM)", "64x1x4"}},
-    {128, 2, {gj_launch<32, 4, 8>, gj_launch<64, 2, 8>, nullptr}, {"32x4x8", "64x2x8", ""}},
+static const GjClass GJ_CLASSES[4] = {
+    {32, 2, {gj_launch<1, 4, 6>, gj_launch<1, 2, 8>}, {"4+1 warps", "2+1 warps"}},
+    {64, 2, {gj_launch<2, 4, 4>, gj_launch<2, 8, 3>}, {"4+2 warps", "8+2 warps"}},
+    {96, 2, {gj_launch<3, 6, 2>, gj_launch<3, 12, 1>}, {"6+3 warps", "12+3 warps"}},
+    {128, 2, {gj_launch<4, 8, 1>, gj_launch<4, 12, 1>}, {"8+4 warps", "12+4 warps"}},
 };
 
 namespace {
@@ -1743,7 +1765,7 @@ int g_tune_force = 0;                         // > 0: always layout g_tune_force
 
 static GjLaunch gj_choose(int n, long long items, const MatRef &A, const MatRef &X, int nc, const int *act,
                           cudaStream_t st) {
-  const int cls = n <= 32 ? 0 : n <= 64 ? 1 : 2;
+  const int cls = (n - 1) / 32;
   const GjClass &C = GJ_CLASSES[cls];
   std::lock_guard<std::mutex> lk(g_tune_mu);
   if (g_tune_force > 0) return C.f[std::min(g_tune_force - 1, C.nv - 1)];
@@ -1751,6 +1773,10 @@ static GjLaunch gj_choose(int n, long long items, const MatRef &A, const MatRef 
   const int bucket = items < 152 ? 0 : items < 608 ? 1 : 2;
   auto it = g_tuned.find({cls, bucket});
   if (it != g_tuned.end()) return C.f[it->second];
+  if (C.nv == 1) {
+    g_tuned[{cls, bucket}] = 0;
+    return C.f[0];
+  }
   if (stream_capturing(st)) return C.f[0];
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess) return C.f[0];
@@ -1803,42 +1829,6 @@ std::string gj_tune_report() {
   return r;
 }
 
-// The FP32 start of an inverse above 64 rows by the 2 x 2 block form: with
-// A = [[A11, A12], [A21, A22]], A11 64 x 64,
-//   X11 = A11^-1, U = X11 A12, S = A22 - A21 U, Y = S^-1, T = A21 X11,
-//   A^-1 = [[X11 - X12 T, X12], [-Y T, Y]],  X12 = -U Y,
-// the two diagonal inverses by the FP32 Gauss-Jordan (pivoting inside each
-// block) at 64 rows, where several matrices share an SM, and the six
-// products by k_cgemm32.  Without pivoting across the blocks the start is
-// a few times less accurate than the whole-matrix Gauss-Jordan on the
-// path's matrices; the Newton steps and their acceptance test are the same.
-// `scratch` holds n^2 elements per item (X11, U, S, T).
-static void block_start(const MatRef &A, const MatRef &X, int n, int nc, const int *act, unsigned items,
-                        zd *scratch, cudaStream_t st) {
-  const int b = 64, n2 = n - 64;
-  const long long MB = (long long)n * n;
-  auto sub = [&](const MatRef &M, int r, int c) { return mref_offset(M, r + (long long)c * M.ld); };
-  auto scr = [&](long long off, int ld) { return mref(scratch + off, (long long)nc * MB, MB, ld); };
-  const MatRef X11 = scr(0, b), U = scr((long long)b * b, b), S = scr((long long)b * b + (long long)b * n2, n2),
-               T = scr((long long)b * b + (long long)b * n2 + (long long)n2 * n2, n2);
-  const MatRef A11 = A, A12 = sub(A, 0, b), A21 = sub(A, b, 0), A22 = sub(A, b, b);
-  const MatRef Xa = X, X12 = sub(X, 0, b), X21 = sub(X, b, 0), X22 = sub(X, b, b);
-  const GjLaunch g1 = gj_choose(b, items, A11, X11, nc, act, st);
-  g1(A11, X11, b, nc, act, items, st);
-  SKKR_LAUNCHED();
-  const G32Job u = g32(0, X11, A12, U, U, b, n2, b), t = g32(0, A21, X11, T, T, n2, b, b);
-  cgemm32(u, &t, nc, act, items, st);                                  // U = X11 A12, T = A21 X11
-  cgemm32(g32(1, A21, U, S, A22, n2, n2, b), nullptr, nc, act, items, st);  // S = A22 - A21 U
-  // Y = S^-1 straight into its place in X (the layout autotuner may run its
-  // candidates on these operands: S is never overwritten)
-  const GjLaunch g2 = gj_choose(n2, items, S, X22, nc, act, st);
-  g2(S, X22, n2, nc, act, items, st);
-  SKKR_LAUNCHED();
-  const G32Job x12 = g32(2, U, X22, X12, X12, b, n2, n2), x21 = g32(2, X22, T, X21, X21, n2, b, n2);
-  cgemm32(x12, &x21, nc, act, items, st);                              // X12 = -U Y, X21 = -Y T
-  cgemm32(g32(1, X12, T, Xa, X11, b, b, n2), nullptr, nc, act, items, st);  // X11 - X12 T
-}
-
 // X = A^-1: FP32 Gauss-Jordan, then `newton` steps X += X (I - A X) with the
 // residual product at S = sres slices and the correction at S = scorr.  An
 // item is accepted when the residual before the last correction is at most
@@ -1868,13 +1858,8 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
   MatRef R = mref(w->rbuf, (long long)nc * MB, MB, n);
   if (inplace) launch_zaxpby(Ac, A, nullptr, 0, nullptr, 0, n, nk, nc, act, st);
   kstat_begin(KS_GJ, 8.0 * n * (double)n * n * (double)(act ? skkr_active_items(items) : items), st);
-  if (w->blocked && n > 64) {
-    block_start(Ac, X, n, nc, act, (unsigned)items, w->rbuf, st);
-  } else {
-    const GjLaunch gj = gj_choose(n, items, Ac, X, nc, act, st);
-    gj(Ac, X, n, nc, act, (unsigned)items, st);
-    SKKR_LAUNCHED();
-  }
+  gj_choose(n, items, Ac, X, nc, act, st)(Ac, X, n, nc, act, (unsigned)items, st);
+  SKKR_LAUNCHED();
   kstat_end(st);
   // A is split once (A slot 0) for the residuals of every Newton step
   if ((rc = mixed_split(w, 0, 0, sres, Ac, n, n, nk, nc, act, st))) return rc;
@@ -1975,8 +1960,8 @@ int wide_zgemm(MixedWork *w, int mode, const MatRef &A, const MatRef &B, const M
 // X = A^-1 to FP64 accuracy.  Up to 128 rows: mixed_zinv with eight-slice
 // residuals, four-slice corrections and the acceptance limit at 1e-9, whose
 // square is below FP64's rounding.  Above, and in `halves` (n even): the 2 x 2
-// block form of block_start with such inverses and products, then one Newton step on the
-// whole matrix, which also checks it.  What is not accepted is inverted by the
+// block form (X11 = A11^-1, U = X11 A12, T = A21 X11, S = A22 - A21 U, Y = S^-1) with
+// such inverses and products, then one Newton step on the whole matrix, which also checks it.  What is not accepted is inverted by the
 // FP64 Gauss-Jordan, as are odd sizes above 128.  30 inverses of n = 256:
 // 18.9 ms by k_zgj (one block, hence one SM, per matrix).
 int wide_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, bool halves, int nk, int nc, const int *act,
