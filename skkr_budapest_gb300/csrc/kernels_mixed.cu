@@ -1754,7 +1754,7 @@ static const GjClass GJ_CLASSES[4] = {
     {32, 2, {gj_launch<1, 4, 6>, gj_launch<1, 2, 8>}, {"4+1 warps", "2+1 warps"}},
     {64, 2, {gj_launch<2, 4, 4>, gj_launch<2, 8, 3>}, {"4+2 warps", "8+2 warps"}},
     {96, 2, {gj_launch<3, 6, 2>, gj_launch<3, 12, 1>}, {"6+3 warps", "12+3 warps"}},
-    {128, 2, {gj_launch<4, 8, 1>, gj_launch<4, 12, 1>}, {"8+4 warps", "12+4 warps"}},
+    {128, 2, {gj_launch<4, 12, 1>, gj_launch<4, 8, 1>}, {"12+4 warps", "8+4 warps"}},
 };
 
 namespace {
