@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <thread>
 #include <cstdlib>
@@ -2396,20 +2397,53 @@ extern "C" int skkr_gpu_surfgf_batch(int n, int batch, const double *ml, const d
 }
 
 // rsp-scf/phystau.f / nrsp-scf/phystau.f on the device
-__global__ void k_phys_mats(const zd *tinv, const zd *alpha, const int *lof, int nd, zd *lmat,
-                            zd *rmat, zd *cmat) {
-  for (int e = threadIdx.x + blockIdx.x * blockDim.x; e < nd * nd; e += blockDim.x * gridDim.x) {
-    const int a = e % nd, b = e / nd;
-    zd al = alpha[lof[a]], alp = alpha[lof[b]], t = tinv[e];
-    zd lv = zmul(al, t), rv = zmul(t, alp), cv = zmul(zmul(al, t), alp);
-    if (a == b) {
-      lv.x += 1.0;
-      rv.x += 1.0;
-      cv = zadd(al, cv);
+// (one block per row i: h = L(i, :) tau, then h R; PHYS_SEG threads share a
+// column's sum, each a stride of k, joined in a fixed order.  Row by row the
+// two products need no matrix in between, so that one launch does what two
+// k_phys_mats, two products and a subtraction did: 38 us of a single n = 32
+// block's time on the device, 7 now.)
+constexpr int PHYS_SEG = 4, PHYS_MAX = 64;
+__global__ void __launch_bounds__(PHYS_SEG *PHYS_MAX) k_phystau(const zd *__restrict__ tau, const zd *__restrict__ ti1,
+                                                               const zd *__restrict__ al1, const zd *__restrict__ ti2,
+                                                               const zd *__restrict__ al2, const int *__restrict__ lof,
+                                                               int nd, bool sub, zd *__restrict__ out) {
+  __shared__ zd v[PHYS_MAX], part[PHYS_SEG][PHYS_MAX];
+  const int i = blockIdx.x, j = threadIdx.x % PHYS_MAX, seg = threadIdx.x / PHYS_MAX;
+  const zd ai = al1[lof[i]];
+  if (seg == 0 && j < nd) {
+    zd l = zmul(ai, ti1[i + j * nd]);
+    if (i == j) l.x += 1.0;
+    v[j] = l;
+  }
+  __syncthreads();
+  const zd aj = j < nd ? al2[lof[j]] : make_double2(0.0, 0.0);
+  for (int pass = 0; pass < 2; pass++) {  // L(i, :) tau, then that times R
+    zd acc = make_double2(0.0, 0.0);
+    if (j < nd)
+#pragma unroll 4
+      for (int k = seg; k < nd; k += PHYS_SEG) {
+        zd m = pass ? zmul(ti2[k + j * nd], aj) : tau[k + j * nd];
+        if (pass && k == j) m.x += 1.0;
+        zfma(acc, v[k], m);
+      }
+    part[seg][j] = acc;
+    __syncthreads();
+    if (seg == 0) {
+      zd h = part[0][j];
+#pragma unroll
+      for (int s = 1; s < PHYS_SEG; s++) h = zadd(h, part[s][j]);
+      v[j] = h;
     }
-    lmat[e] = lv;
-    rmat[e] = rv;
-    cmat[e] = cv;
+    __syncthreads();
+  }
+  if (seg == 0 && j < nd) {
+    zd o = v[j];
+    if (sub) {  // - (alpha delta + alpha t^-1 alpha)
+      zd c = zmul(zmul(ai, ti1[i + j * nd]), aj);
+      if (i == j) c = zadd(ai, c);
+      o = make_double2(o.x - c.x, o.y - c.y);
+    }
+    out[i + j * nd] = o;
   }
 }
 
@@ -2436,40 +2470,85 @@ static int phys_basis(int mode, int lmax, int ld, int *nd, int *nal, std::vector
   return SKKR_OK;
 }
 
+// tau <- L tau R (- C for one layer, tinv2 null): every operand in one host
+// block, one copy each way, and the device block from a small pool of the
+// device's (8 cudaMalloc and cudaFree a call cost 0.2 ms, several times the
+// work): at most PHYS_POOL_KEEP bytes stay with it between calls.
+constexpr unsigned long long PHYS_POOL_KEEP = 4ull << 20;
+static int phys_pool(cudaMemPool_t *pool) {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = pools.find(dev);
+  if (it == pools.end()) {
+    cudaMemPoolProps pr = {};
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    cudaMemPool_t p;
+    CK(cudaMemPoolCreate(&p, &pr));
+    unsigned long long keep = PHYS_POOL_KEEP;  // (a 64-bit attribute)
+    const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(p);
+      CK(e);
+    }
+    it = pools.emplace(dev, p).first;
+  }
+  *pool = it->second;
+  return SKKR_OK;
+}
+
+static int phys_run(int nd, int nal, const std::vector<int> &lof, double *tau, const double *tinv1,
+                    const double *alpha1, const double *tinv2, const double *alpha2, int ld) {
+  const size_t MB = (size_t)nd * nd;
+  const bool pair = tinv2 != nullptr;
+  // tau, t1^-1 (, t2^-1), alpha1 (, alpha2), l of the basis; then the result
+  const size_t nz = MB * (pair ? 3 : 2) + (size_t)nal * (pair ? 2 : 1), in = nz * sizeof(zd) + nd * sizeof(int),
+               out = (in + 255) / 256 * 256;
+  std::vector<zd> host(nz + (nd * sizeof(int) + sizeof(zd) - 1) / sizeof(zd));
+  auto put = [&](size_t at, const double *src) {
+    for (int c = 0; c < nd; c++) memcpy(&host[at + (size_t)c * nd], src + 2 * (size_t)c * ld, nd * sizeof(zd));
+  };
+  size_t at = 0;
+  put(at, tau);
+  put(at += MB, tinv1);
+  if (pair) put(at += MB, tinv2);
+  at += MB;
+  memcpy(&host[at], alpha1, nal * sizeof(zd));
+  if (pair) memcpy(&host[at + nal], alpha2, nal * sizeof(zd));
+  memcpy((char *)host.data() + nz * sizeof(zd), lof.data(), nd * sizeof(int));
+  cudaMemPool_t pool;
+  CKR(phys_pool(&pool));
+  void *q = nullptr;
+  const cudaError_t e = cudaMallocFromPoolAsync(&q, out + MB * sizeof(zd), pool, 0);
+  if (e != cudaSuccess) {
+    g_last_error = std::string("cudaMallocFromPoolAsync: ") + cudaGetErrorString(e);
+    return SKKR_ERR_NOMEM;
+  }
+  zd *d = (zd *)q, *O = (zd *)((char *)q + out);
+  auto run = [&]() -> int {
+    CK(cudaMemcpy(d, host.data(), in, cudaMemcpyHostToDevice));
+    const zd *t1 = d + MB, *t2 = pair ? t1 + MB : t1, *a1 = t2 + MB, *a2 = pair ? a1 + nal : a1;
+    k_phystau<<<nd, PHYS_SEG * PHYS_MAX>>>(d, t1, a1, t2, a2, (const int *)(d + nz), nd, !pair, O);
+    SKKR_LAUNCHED();
+    CK(cudaGetLastError());
+    return download_mats(tau, O, 1, nd, ld);
+  };
+  const int rc = run();
+  cudaFreeAsync(q, 0);
+  return rc;
+}
+
 extern "C" int skkr_gpu_phystau(int mode, int lmax, double *tau, const double *tinv,
                                 const double *alpha, int ld) {
   if (!tau || !tinv || !alpha) return SKKR_ERR_ARG;
   int nd, nal;
   std::vector<int> lof;
   CKR(phys_basis(mode, lmax, ld, &nd, &nal, lof));
-  const long long MB = (long long)nd * nd;
-  Scoped s;
-  zd *T, *Ti, *Al, *Lm, *Rm, *Cm, *H;
-  int *Lo;
-  CKR(s.alloc(&T, MB));
-  CKR(s.alloc(&Ti, MB));
-  CKR(s.alloc(&Al, nal));
-  CKR(s.alloc(&Lm, MB));
-  CKR(s.alloc(&Rm, MB));
-  CKR(s.alloc(&Cm, MB));
-  CKR(s.alloc(&H, MB));
-  CKR(s.alloc(&Lo, nd));
-  CKR(upload_mats(T, tau, 1, nd, ld));
-  CKR(upload_mats(Ti, tinv, 1, nd, ld));
-  CK(cudaMemcpy(Al, alpha, nal * sizeof(zd), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(Lo, lof.data(), nd * sizeof(int), cudaMemcpyHostToDevice));
-  k_phys_mats<<<4, 256>>>(Ti, Al, Lo, nd, Lm, Rm, Cm);
-  SKKR_LAUNCHED();
-  // tripmt(lmat, tau, rmat): (lmat tau) rmat ; then tau - cmat
-  launch_zgemm(0, mref(Lm, 0, 0, nd), mref(T, 0, 0, nd), mref(H, 0, 0, nd), mref(H, 0, 0, nd),
-               mref(H, 0, 0, nd), nd, nd, nd, 1, 1, nullptr, 0);
-  launch_zgemm(0, mref(H, 0, 0, nd), mref(Rm, 0, 0, nd), mref(T, 0, 0, nd), mref(T, 0, 0, nd),
-               mref(T, 0, 0, nd), nd, nd, nd, 1, 1, nullptr, 0);
-  MatRef Tm = mref(T, 0, 0, nd), Cmm = mref(Cm, 0, 0, nd);
-  launch_zaxpby(Tm, Tm, &Cmm, -1.0, nullptr, 0, nd, 1, 1, nullptr, 0);
-  CK(cudaDeviceSynchronize());
-  CK(cudaGetLastError());
-  return download_mats(tau, T, 1, nd, ld);
+  return phys_run(nd, nal, lof, tau, tinv, alpha, nullptr, nullptr, ld);
 }
 
 extern "C" int skkr_gpu_phystau2(int mode, int lmax, double *tau, const double *tinv1,
@@ -2479,40 +2558,9 @@ extern "C" int skkr_gpu_phystau2(int mode, int lmax, double *tau, const double *
   int nd, nal;
   std::vector<int> lof;
   CKR(phys_basis(mode, lmax, ld, &nd, &nal, lof));
-  const long long MB = (long long)nd * nd;
-  Scoped s;
-  zd *T, *Ti1, *Ti2, *Al1, *Al2, *Lm, *Rm, *Sc, *Cm, *H;
-  int *Lo;
-  CKR(s.alloc(&T, MB));
-  CKR(s.alloc(&Ti1, MB));
-  CKR(s.alloc(&Ti2, MB));
-  CKR(s.alloc(&Al1, nal));
-  CKR(s.alloc(&Al2, nal));
-  CKR(s.alloc(&Lm, MB));
-  CKR(s.alloc(&Rm, MB));
-  CKR(s.alloc(&Sc, MB));
-  CKR(s.alloc(&Cm, MB));
-  CKR(s.alloc(&H, MB));
-  CKR(s.alloc(&Lo, nd));
-  CKR(upload_mats(T, tau, 1, nd, ld));
-  CKR(upload_mats(Ti1, tinv1, 1, nd, ld));
-  CKR(upload_mats(Ti2, tinv2, 1, nd, ld));
-  CK(cudaMemcpy(Al1, alpha1, nal * sizeof(zd), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(Al2, alpha2, nal * sizeof(zd), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(Lo, lof.data(), nd * sizeof(int), cudaMemcpyHostToDevice));
   // lmat = 1 + alpha1 tinv1 from the row layer, rmat = 1 + tinv2 alpha2 from
-  // the column layer (the other two outputs of each launch are scratch)
-  k_phys_mats<<<4, 256>>>(Ti1, Al1, Lo, nd, Lm, Sc, Cm);
-  SKKR_LAUNCHED();
-  k_phys_mats<<<4, 256>>>(Ti2, Al2, Lo, nd, Sc, Rm, Cm);
-  SKKR_LAUNCHED();
-  launch_zgemm(0, mref(Lm, 0, 0, nd), mref(T, 0, 0, nd), mref(H, 0, 0, nd), mref(H, 0, 0, nd),
-               mref(H, 0, 0, nd), nd, nd, nd, 1, 1, nullptr, 0);
-  launch_zgemm(0, mref(H, 0, 0, nd), mref(Rm, 0, 0, nd), mref(T, 0, 0, nd), mref(T, 0, 0, nd),
-               mref(T, 0, 0, nd), nd, nd, nd, 1, 1, nullptr, 0);
-  CK(cudaDeviceSynchronize());
-  CK(cudaGetLastError());
-  return download_mats(tau, T, 1, nd, ld);
+  // the column layer
+  return phys_run(nd, nal, lof, tau, tinv1, alpha1, tinv2, alpha2, ld);
 }
 
 extern "C" int skkr_gpu_layer_dos(int mode, int lmax, int nlay, const double *tau, int ld,
