@@ -247,7 +247,9 @@ __device__ __forceinline__ void store1(const int (&dg)[S], int wshift, uint16_t 
 // tiles transposed through shared memory, each thread taking four
 // consecutive columns of one row (8-byte stores of every slice) when K is a
 // multiple of four, one element otherwise.
-template <int S, int DB>
+// H (n <= 64, see k_ozaki): row 64 + r of A' is [Im A, Re A] and row r
+// [Re A, -Im A].
+template <int S, int DB, int H>
 __global__ void __launch_bounds__(256) k_split_a(MatRef A, int n, int K, int nc, const int *__restrict__ act,
                                                  __nv_bfloat16 *__restrict__ out, int Mp, int Kp,
                                                  int *__restrict__ sigma) {
@@ -274,7 +276,8 @@ __global__ void __launch_bounds__(256) k_split_a(MatRef A, int n, int K, int nc,
     for (int q = 0; q < 8; q++) mm = red[q][lane] > mm ? red[q][lane] : mm;
     const int es = scale_exp(mm);
     sc[lane] = es;
-    if (r0 + lane < Mp) sigma[(long long)item * Mp + r0 + lane] = es;
+    if (r0 + lane < (H ? MT / 2 : Mp)) sigma[(long long)item * Mp + r0 + lane] = es;
+    if (H && r0 + lane < MT / 2) sigma[(long long)item * Mp + MT / 2 + r0 + lane] = es;
   }
   __syncthreads();
   const long long sstride = (long long)Mp * Kp;
@@ -299,7 +302,11 @@ __global__ void __launch_bounds__(256) k_split_a(MatRef A, int n, int K, int nc,
         uint32_t wr[S][2], wi[S][2];
         slice4<S, DB>(re, im, sc[q], 0, wr, wi);
         store_words<S>(wr, 0u, base + tiled(r, kpos(col, 0), Mp), sstride);
-        store_words<S>(wi, 0u, base + tiled(r, kpos(col, 1), Mp), sstride);
+        store_words<S>(wi, H ? 0x80008000u : 0u, base + tiled(r, kpos(col, 1), Mp), sstride);
+        if (H) {
+          store_words<S>(wi, 0u, base + tiled(MT / 2 + r, kpos(col, 0), Mp), sstride);
+          store_words<S>(wr, 0u, base + tiled(MT / 2 + r, kpos(col, 1), Mp), sstride);
+        }
       }
     } else {
       for (int q = w; q < 32; q += 8) {
@@ -311,7 +318,11 @@ __global__ void __launch_bounds__(256) k_split_a(MatRef A, int n, int K, int nc,
           slice_digits<S, DB>(v.x, es, dr);
           slice_digits<S, DB>(v.y, es, di);
           store1<S, DB>(dr, 0, 0, base + tiled(r, kpos(col, 0), Mp), sstride);
-          store1<S, DB>(di, 0, 0, base + tiled(r, kpos(col, 1), Mp), sstride);
+          store1<S, DB>(di, 0, H ? 0x8000 : 0, base + tiled(r, kpos(col, 1), Mp), sstride);
+          if (H) {
+            store1<S, DB>(di, 0, 0, base + tiled(MT / 2 + r, kpos(col, 0), Mp), sstride);
+            store1<S, DB>(dr, 0, 0, base + tiled(MT / 2 + r, kpos(col, 1), Mp), sstride);
+          }
         }
       }
     }
@@ -326,7 +337,8 @@ __global__ void __launch_bounds__(256) k_split_a(MatRef A, int n, int K, int nc,
 // lane takes four consecutive rows k (8-byte stores) when K is a multiple of
 // four, one row otherwise; each digit is formed once and stored twice, -Im
 // with its sign bit flipped.
-template <int S, int DB>
+// H (n <= 64): row j of B'^T is [Re B(:,j), Im B(:,j)].
+template <int S, int DB, int H>
 __global__ void __launch_bounds__(256, 3) k_split_b(MatRef B, int n, int K, int nc, const int *__restrict__ act,
                                                  __nv_bfloat16 *__restrict__ out, int Np, int Kp,
                                                  int *__restrict__ tau) {
@@ -362,6 +374,11 @@ __global__ void __launch_bounds__(256, 3) k_split_b(MatRef B, int n, int K, int 
       }
       uint32_t wr[S][2], wi[S][2];
       slice4<S, DB>(re, im, es, 16, wr, wi);
+      if (H) {
+        store_words<S>(wr, 0u, base + tiled(j, kpos(k, 0), Np), sstride);
+        store_words<S>(wi, 0u, base + tiled(j, kpos(k, 1), Np), sstride);
+        continue;
+      }
       store_words<S>(wr, 0u, base + tiled(2 * j, kpos(k, 0), Np), sstride);
       store_words<S>(wi, 0x80008000u, base + tiled(2 * j, kpos(k, 1), Np), sstride);
       store_words<S>(wi, 0u, base + tiled(2 * j + 1, kpos(k, 0), Np), sstride);
@@ -373,6 +390,11 @@ __global__ void __launch_bounds__(256, 3) k_split_b(MatRef B, int n, int K, int 
       int dr[S], di[S];
       slice_digits<S, DB>(v.x, es, dr);
       slice_digits<S, DB>(v.y, es, di);
+      if (H) {
+        store1<S, DB>(dr, 16, 0, base + tiled(j, kpos(k, 0), Np), sstride);
+        store1<S, DB>(di, 16, 0, base + tiled(j, kpos(k, 1), Np), sstride);
+        continue;
+      }
       store1<S, DB>(dr, 16, 0, base + tiled(2 * j, kpos(k, 0), Np), sstride);
       store1<S, DB>(di, 16, 0x8000, base + tiled(2 * j, kpos(k, 1), Np), sstride);
       store1<S, DB>(di, 16, 0, base + tiled(2 * j + 1, kpos(k, 0), Np), sstride);
@@ -484,7 +506,7 @@ struct OzShared {
   uint32_t tmem_base;
   volatile int failed;
   volatile int a_issued, raw_issued;      // k-blocks asked for (counts over all tiles)
-  int col_exp[OZ_EXP_RING][NT / 2];       // column scale exponents of each tile's complex columns
+  short col_exp[OZ_EXP_RING][NT];         // column scale exponents of each tile's complex columns
 };
 
 // the warp waits for a phase of a barrier; false (for the whole warp) once
@@ -498,10 +520,16 @@ __device__ __forceinline__ bool oz_warp_wait(OzShared &sh, uint64_t *bar, uint32
   return ok != 0;
 }
 
-// n rows x 32 columns of an operand's tile towards L2, one column per lane
+// n rows of an operand's tile's columns towards L2, one column per lane
 __device__ __forceinline__ void oz_prefetch(const zd *p, int ld, int rows, int cols) {
-  const int lane = threadIdx.x & 31;
-  if (lane < cols) bulk_prefetch_l2(p + (long long)lane * ld, (uint32_t)rows * (uint32_t)sizeof(zd));
+  for (int c = threadIdx.x & 31; c < cols; c += 32)
+    bulk_prefetch_l2(p + (long long)c * ld, (uint32_t)rows * (uint32_t)sizeof(zd));
+}
+
+// raw blocks (32 columns each) of a k-block of fused B
+template <int H>
+__device__ __forceinline__ int oz_raw_passes(const OzArgs &g) {
+  return H && g.n > 32 ? 2 : 1;
 }
 
 // The scale role (warp 2, fused B only): the exponents of each tile's 32
@@ -513,26 +541,28 @@ __device__ __forceinline__ void oz_prefetch(const zd *p, int ld, int rows, int c
 // again when the role returns to it: it runs at most four tiles ahead of the
 // conversion, the conversion at most four k-blocks, hence five tiles, ahead of
 // the MMAs, and those wait for the epilogue of the tile oz_bufs before.
+template <int H>
 __device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
+  constexpr int NC = H ? NT : NT / 2;  // complex columns of a tile
   const int lane = threadIdx.x & 31;
   auto prefetch_b = [&](const TileWalk &w) {
-    const int item = w.item(), j0 = w.nt() * (NT / 2);
+    const int item = w.item(), j0 = w.nt() * NC;
     if (w.valid())
       oz_prefetch(mat_ptr(g.B, item / g.nc, item % g.nc) + (long long)j0 * g.B.ld, g.B.ld, g.K,
-                  g.n - j0 < NT / 2 ? g.n - j0 : NT / 2);
+                  g.n - j0 < NC ? g.n - j0 : NC);
   };
   TileWalk wp(g);
   prefetch_b(wp);
   wp.step();
   prefetch_b(wp);
   for (TileWalk w(g); w.valid(); w.step()) {
-    const int item = w.item(), j0 = w.nt() * (NT / 2), nj = g.n - j0 < NT / 2 ? g.n - j0 : NT / 2;
+    const int item = w.item(), j0 = w.nt() * NC, nj = g.n - j0 < NC ? g.n - j0 : NC;
     if (wp.valid()) wp.step();
     prefetch_b(wp);
     if (!oz_warp_wait(sh, &sh.sc_empty[w.i % OZ_SCALE_RING], ((w.i / OZ_SCALE_RING) - 1) & 1, w.i < OZ_SCALE_RING))
       break;
     const zd *b = mat_ptr(g.B, item / g.nc, item % g.nc) + (long long)j0 * g.B.ld;
-    int mine = 0;
+    int mine = 0, mine1 = 0;  // columns lane and 32 + lane
 #pragma unroll 1
     for (int c0 = 0; c0 < nj; c0 += 8) {
       unsigned m[8];
@@ -561,9 +591,11 @@ __device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
       for (int c = 0; c < 8; c++) {
         const unsigned t = __reduce_max_sync(0xffffffffu, m[c]);
         if (lane == c0 + c && lane < nj) mine = scale_exp((unsigned long long)t << 32);
+        if (H && lane + 32 == c0 + c && lane + 32 < nj) mine1 = scale_exp((unsigned long long)t << 32);
       }
     }
-    sh.col_exp[w.i % OZ_EXP_RING][lane] = mine;
+    sh.col_exp[w.i % OZ_EXP_RING][lane] = (short)mine;
+    if (H) sh.col_exp[w.i % OZ_EXP_RING][lane + 32] = (short)mine1;
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.sc_full[w.i % OZ_SCALE_RING]);
   }
@@ -576,43 +608,52 @@ __device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
 // flipped sign bits).  Each thread orders its stores before the tensor core's
 // reads (proxy fence); lane 0, after the warp's barrier, arrives on the
 // stage's full barrier.  (Values outside the matrix arrive as zeros.)
-template <int S, int DB, int NB, int NRAW>
+// H: 64 columns of one row each, in passes of 32 columns that each take a raw
+// block; two stores a value.
+template <int S, int DB, int NB, int NRAW, int H>
 __device__ __forceinline__ void oz_convert(const OzArgs &g, OzShared &sh, unsigned char *sb0, const unsigned char *raw) {
   const int cw = (threadIdx.x >> 5) - OZ_CONV0, lane = threadIdx.x & 31;
   const int nkb = g.kblocks, jl = 8 * (cw & 3) + (lane >> 2), kq = 4 * (lane & 3);
-  const int r = 2 * jl;
+  const int r = H ? jl : 2 * jl, npass = oz_raw_passes<H>(g);
   const uint32_t o0 = sw64_off(r, kq), o1 = sw64_off(r, kq + 16), o2 = sw64_off(r + 1, kq),
                  o3 = sw64_off(r + 1, kq + 16);
   // this thread's 16-byte values in a raw block: box kq / 8, row jl, chunks kq % 8 .. +3 XORed with jl % 8
   const unsigned char *src = raw + (kq >> 3) * (OZ_RAW_BYTES / 2) + jl * 128;
   for (TileWalk w(g); w.valid(); w.step()) {
     if (!oz_warp_wait(sh, &sh.sc_full[w.i % OZ_SCALE_RING], (w.i / OZ_SCALE_RING) & 1)) return;
-    const int es = sh.col_exp[w.i % OZ_EXP_RING][jl];
     for (int kb = cw >> 2; kb < nkb; kb += oz_conv_groups(S)) {
-      const int kc = w.i * nkb + kb, st = kc % NB, rr = kc % NRAW;
-      if (!oz_warp_wait(sh, &sh.raw_full[rr], (kc / NRAW) & 1)) return;
-      double re[4], im[4];
+      const int kc = w.i * nkb + kb, st = kc % NB;
+#pragma unroll 1
+      for (int pass = 0; pass < npass; pass++) {
+        const int rc = kc * npass + pass, rr = rc % NRAW, es = sh.col_exp[w.i % OZ_EXP_RING][jl + 32 * pass];
+        if (!oz_warp_wait(sh, &sh.raw_full[rr], (rc / NRAW) & 1)) return;
+        double re[4], im[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const zd v = *reinterpret_cast<const zd *>(src + rr * OZ_RAW_BYTES + ((((kq & 7) + e) ^ (jl & 7)) << 4));
-        re[e] = v.x;
-        im[e] = v.y;
-      }
-      uint32_t wr[S][2], wi[S][2];
-      if constexpr (DB == 8) slice4b<S>(re, im, es, wr, wi);
-      else slice4<S, DB>(re, im, es, 16, wr, wi);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.raw_empty[rr]);
-      // the stores come after the tensor core's reads of the stage
-      if (!oz_warp_wait(sh, &sh.b_empty[st], ((kc / NB) - 1) & 1, kc < NB)) return;
-      unsigned char *sb = sb0 + st * (S * OZ_B_SLICE);
+        for (int e = 0; e < 4; e++) {
+          const zd v = *reinterpret_cast<const zd *>(src + rr * OZ_RAW_BYTES + ((((kq & 7) + e) ^ (jl & 7)) << 4));
+          re[e] = v.x;
+          im[e] = v.y;
+        }
+        uint32_t wr[S][2], wi[S][2];
+        if constexpr (DB == 8) slice4b<S>(re, im, es, wr, wi);
+        else slice4<S, DB>(re, im, es, 16, wr, wi);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.raw_empty[rr]);
+        // the stores come after the tensor core's reads of the stage
+        if (pass == 0 && !oz_warp_wait(sh, &sh.b_empty[st], ((kc / NB) - 1) & 1, kc < NB)) return;
+        unsigned char *sb = sb0 + st * (S * OZ_B_SLICE) + pass * (32 * KB * 2);
 #pragma unroll
-      for (int p = 0; p < S; p++) {
-        unsigned char *tp = sb + p * OZ_B_SLICE;
-        *reinterpret_cast<uint2 *>(tp + o0) = make_uint2(wr[p][0], wr[p][1]);
-        *reinterpret_cast<uint2 *>(tp + o1) = make_uint2(wi[p][0] ^ 0x80008000u, wi[p][1] ^ 0x80008000u);
-        *reinterpret_cast<uint2 *>(tp + o2) = make_uint2(wi[p][0], wi[p][1]);
-        *reinterpret_cast<uint2 *>(tp + o3) = make_uint2(wr[p][0], wr[p][1]);
+        for (int p = 0; p < S; p++) {
+          unsigned char *tp = sb + p * OZ_B_SLICE;
+          *reinterpret_cast<uint2 *>(tp + o0) = make_uint2(wr[p][0], wr[p][1]);
+          if constexpr (H) {
+            *reinterpret_cast<uint2 *>(tp + o1) = make_uint2(wi[p][0], wi[p][1]);
+          } else {
+            *reinterpret_cast<uint2 *>(tp + o1) = make_uint2(wi[p][0] ^ 0x80008000u, wi[p][1] ^ 0x80008000u);
+            *reinterpret_cast<uint2 *>(tp + o2) = make_uint2(wi[p][0], wi[p][1]);
+            *reinterpret_cast<uint2 *>(tp + o3) = make_uint2(wr[p][0], wr[p][1]);
+          }
+        }
       }
       // every lane's stores visible to the tensor core, then one arrival per warp
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -652,7 +693,9 @@ __device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint3
     const zd *src = rd_c ? pc : pd;
     const long long sld = rd_c ? g.C.ld : g.D.ld;
     // the column scales: of the scale role (fused B), or of the split
-    const int *ce = FB ? sh.col_exp[w.i % OZ_EXP_RING] + half * 16 : g.tau + (long long)item * g.n + j0;
+    auto ce = [&](int q) {
+      return FB ? (int)sh.col_exp[w.i % OZ_EXP_RING][half * 16 + q] : g.tau[(long long)item * g.n + j0 + q];
+    };
     zd old[NO];
     auto load_old = [&](const zd *src, long long sld, int q0) {  // columns q0 .. q0 + NO - 1
 #pragma unroll
@@ -669,7 +712,7 @@ __device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint3
     };
     // the level sums in FP64; a row of A or a column of B that holds an infinity or a NaN has no digits
     auto value = [&](long long ar, long long ai, int q) {
-      const int tj = ce[q];
+      const int tj = ce(q);
       zd val = make_double2(fix_to_double(ar, erow + tj), fix_to_double(ai, erow + tj));
       if (sig == SCALE_NONFINITE || tj == SCALE_NONFINITE) val = make_double2(nan, nan);
       return val;
@@ -755,6 +798,123 @@ __device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint3
   }
 }
 
+// The epilogue role for stacked operands (H): rows 0-63 of the tile hold the
+// real, rows 64-127 the imaginary parts, a TMEM column is one complex column;
+// a thread updates one part of 32 outputs.  (The two parts of a row come from
+// different warps: their 8-byte accesses meet in the cache.)
+template <int S, int DB, int FB>
+__device__ __forceinline__ void oz_epilogue_h(const OzArgs &g, OzShared &sh, uint32_t tbase) {
+  constexpr int NBUF = oz_bufs(S), CH = S <= 6 ? 8 : 4;  // columns per TMEM load
+  constexpr bool EARLY = NBUF == 1;                      // hand the accumulators back before the rounding
+  constexpr int NA = EARLY ? 32 : CH, NO = 8;  // sums held, old values in a batch
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quarter = warp & 3, half = (warp - OZ_EPI0) >> 2;
+  const int mode = g.mode, part = quarter >> 1, row = (quarter & 1) * 32 + lane, j0 = half * 32;
+  const int nq = row < g.n ? g.n - j0 : 0;  // columns of this thread's row inside the matrix
+  const bool rd = mode == 1 || mode == 5 || mode == 2 || mode == 3, rd_c = mode == 1 || mode == 5;
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  for (TileWalk w(g); w.valid(); w.step()) {
+    const int item = w.item(), kk = item / g.nc, cc = item % g.nc, buf = w.i % NBUF;
+    const int sig = row < g.n ? g.sigma[(long long)item * MT + part * (MT / 2) + row] : 0;
+    const int erow = sig - 2 * (DB - 1) - DB * (S - 1 < 5 ? S - 1 : 5);
+    auto at = [&](const MatRef &M) {
+      return reinterpret_cast<double *>(mat_ptr(M, kk, cc) + row + (long long)j0 * M.ld) + part;
+    };
+    double *pc = at(g.C), *pd = at(g.D), *pe = at(g.E);
+    const double *src = rd_c ? pc : pd;
+    const long long sld = 2ll * (rd_c ? g.C.ld : g.D.ld), eld = 2ll * g.E.ld, old_ld = 2ll * (mode == 2 ? g.D.ld : g.C.ld);
+    double *out = mode == 2 ? pd : pc;
+    auto ce = [&](int q) {
+      return FB ? (int)sh.col_exp[w.i % OZ_EXP_RING][j0 + q] : g.tau[(long long)item * g.n + j0 + q];
+    };
+    if (rd) {
+      // the next tile's old values towards L2: 32 columns x 512 bytes, shared with the warp of the other part
+      TileWalk wn = w;
+      wn.step();
+      if (wn.valid()) {
+        const int in = wn.item(), rn = (quarter & 1) * 32 + 8 * (lane & 3);
+        const MatRef &M = rd_c ? g.C : g.D;
+        const zd *p = mat_ptr(M, in / g.nc, in % g.nc) + rn;
+        const zd *pe2 = mat_ptr(g.E, in / g.nc, in % g.nc) + rn;
+#pragma unroll
+        for (int q = 0; q < 16; q += 8) {
+          const int j = j0 + 16 * part + q + (lane >> 2);
+          if (rn < g.n && j < g.n) {
+            prefetch_l2(p + (long long)j * M.ld);
+            if (mode == 2) prefetch_l2(pe2 + (long long)j * g.E.ld);
+          }
+        }
+      }
+    }
+    long long acc[NA];
+    double old[NO];
+    auto load_old = [&](const double *p, long long ld, int q0) {  // columns q0 .. q0 + NO - 1
+#pragma unroll
+      for (int q = 0; q < NO; q++)
+        if (q0 + q < nq) old[q] = p[(q0 + q) * ld];
+    };
+    auto emit = [&](int q0) {  // columns q0 .. q0 + NO - 1 into C (mode 2: into D)
+#pragma unroll
+      for (int q = 0; q < NO; q++)
+        if (q0 + q < nq) {
+          const int tj = ce(q0 + q);
+          double val = fix_to_double(acc[(q0 + q) % NA], erow + tj);
+          if (sig == SCALE_NONFINITE || tj == SCALE_NONFINITE) val = nan;
+          const double unit = part == 0 && row == j0 + q0 + q ? 1.0 : 0.0;
+          out[(q0 + q) * old_ld] = mode == 0 ? val : mode == 4 ? unit - val : mode == 5 ? old[q] + val : old[q] - val;
+          acc[(q0 + q) % NA] = __double_as_longlong(val);  // for E
+        }
+    };
+    auto emit_e = [&](int q0) {
+#pragma unroll
+      for (int q = 0; q < NO; q++)
+        if (q0 + q < nq) pe[(q0 + q) * eld] = old[q] - __longlong_as_double(acc[(q0 + q) % NA]);
+    };
+    if (!EARLY && rd) load_old(src, sld, 0);
+    if (!oz_warp_wait(sh, &sh.acc_full[buf], (w.i / NBUF) & 1)) break;
+    tc_fence_after();
+    const uint32_t ta = tbase + ((uint32_t)(quarter * 32) << 16) + buf * 256 + half * 32;
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += CH) {
+      uint32_t v[S][CH];
+#pragma unroll
+      for (int l = 0; l < S; l++) {
+        if constexpr (CH == 8) tmem_ld8(ta + l * NT + c0, v[l]);
+        else tmem_ld4(ta + l * NT + c0, v[l]);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int t = 0; t < CH; t++) acc[(c0 + t) % NA] = levels_sum<S, DB, CH>(v, t);
+      if constexpr (!EARLY) {
+        emit(c0);
+        if (mode == 2) {
+          load_old(pe, eld, c0);
+          emit_e(c0);
+        }
+        if (rd && c0 + CH < 32) load_old(src, sld, c0 + CH);
+        __syncwarp();
+      }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
+    if constexpr (EARLY) {
+#pragma unroll
+      for (int q0 = 0; q0 < 32; q0 += NO) {
+        if (rd) load_old(src, sld, q0);
+        emit(q0);
+      }
+      if (mode == 2) {
+#pragma unroll
+        for (int q0 = 0; q0 < 32; q0 += NO) {
+          load_old(pe, eld, q0);
+          emit_e(q0);
+        }
+      }
+    }
+  }
+}
+
 // Sliced product, persistent: one CTA per SM walks its output tiles (128 rows
 // x 32 complex columns) with the roles below running side by side, so that
 // the loads, the conversion of B and the rounding of one tile hide behind
@@ -780,7 +940,14 @@ __device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint3
 // FB = 0: B tiles by TMA from the staged B'; FB = 1: B fused, its tiles
 // formed by the conversion role from the FP64 B, which tmB then maps (g.B is
 // the same operand).
-template <int S, int DB, int FB>
+// H = 1 (up to 64 rows): the tile is the whole product, with the real and the
+// imaginary parts of A stacked, [Re A, -Im A; Im A, Re A] (64 + 64 rows)
+// times [Re B; Im B] (one row of B'^T, one accumulator column per complex
+// column).  The other form would fill half the rows of every tile and form
+// every digit of B four times instead of twice; the integers summed are the
+// same, so are the results bit for bit.  1640 products of n = 54: staged B, six
+// slices 276 -> 156 us; fused B, seven slices 418 -> 209, three 311 -> 183.
+template <int S, int DB, int FB, int H>
 __global__ void __launch_bounds__(oz_threads(S), 1) k_ozaki(const __grid_constant__ CUtensorMap tmA,
                                                          const __grid_constant__ CUtensorMap tmB,
                                                          const __grid_constant__ OzArgs g) {
@@ -891,32 +1058,34 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_ozaki(const __grid_constan
       umma_commit(&sh.done);
     }
   } else if (warp == 2) {
-    if constexpr (FB > 0) oz_scales(g, sh);
+    if constexpr (FB > 0) oz_scales<H>(g, sh);
   } else if (warp == 3) {
     // fused B: the FP64 k-blocks of B into their ring
     if (FB > 0 && lane == 0) {
+      const int npass = oz_raw_passes<H>(g);
       int rc = 0;
       for (TileWalk w(g); w.valid() && !sh.failed; w.step()) {
         const int kk = w.item() / g.nc, cc = w.item() % g.nc, j0 = w.nt() * (NT / 2);
         const int mc = map_at(g.B, cc);
-        for (int kb = 0; kb < nkb; kb++, rc++) {
-          const int r = rc % NRAW;
+        for (int kp = 0; kp < nkb * npass; kp++, rc++) {
+          const int r = rc % NRAW, kb = kp / npass, jp = j0 + (kp % npass) * 32;
           if (sh.failed || (rc >= NRAW && !mbar_wait(&sh.raw_empty[r], ((rc / NRAW) - 1) & 1))) {
             sh.failed = 1;
             break;
           }
           mbar_expect_tx(&sh.raw_full[r], OZ_RAW_BYTES);
           unsigned char *dst = raw + r * OZ_RAW_BYTES;
-          tma_load_4d(dst, &tmB, 32 * kb, j0, mc, kk, &sh.raw_full[r]);
-          tma_load_4d(dst + OZ_RAW_BYTES / 2, &tmB, 32 * kb + 16, j0, mc, kk, &sh.raw_full[r]);
+          tma_load_4d(dst, &tmB, 32 * kb, jp, mc, kk, &sh.raw_full[r]);
+          tma_load_4d(dst + OZ_RAW_BYTES / 2, &tmB, 32 * kb + 16, jp, mc, kk, &sh.raw_full[r]);
           sh.raw_issued = rc + 1;
         }
       }
     }
   } else if (warp < OZ_CONV0) {
-    oz_epilogue<S, DB, FB>(g, sh, tbase);
+    if constexpr (H) oz_epilogue_h<S, DB, FB>(g, sh, tbase);
+    else oz_epilogue<S, DB, FB>(g, sh, tbase);
   } else if constexpr (FB > 0) {
-    oz_convert<S, DB, NB, NRAW>(g, sh, sB, raw);
+    oz_convert<S, DB, NB, NRAW, H>(g, sh, sB, raw);
   }
   __syncthreads();
   // every MMA issued is complete (bounded wait) before the accumulators go
@@ -1453,11 +1622,15 @@ int mixed_error_flag(MixedWork *w) {
   return h;
 }
 
+// up to 64 rows the real and imaginary parts of A are stacked in one tile
+// (k_ozaki's H; depths of the eight-bit digits)
+static bool oz_stacked(int n, int K) { return n <= MT / 2 && K <= 128; }
+
 // dims of the staged real problem for complex n x K times K x n
 static void oz_dims(int n, int K, int *Mp, int *Np, int *Kp, int *mtiles, int *ntiles, int *kblocks) {
   *mtiles = (n + MT - 1) / MT;
   *Mp = *mtiles * MT;
-  *ntiles = (2 * n + NT - 1) / NT;
+  *ntiles = oz_stacked(n, K) ? 1 : (2 * n + NT - 1) / NT;
   *Np = *ntiles * NT;
   *kblocks = (2 * K + KB - 1) / KB;
   *Kp = *kblocks * KB;
@@ -1470,7 +1643,7 @@ static int oz_digits(int K) { return K <= 128 ? 8 : 7; }
 // side 1 with fuse_b: the slot only records B (the product reads it when it
 // runs: B must not change in between, which every caller keeps); `real`
 // (an operand several products read) splits it all the same
-template <int S, int DB>
+template <int S, int DB, int H>
 static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int K, int nk, int nc,
                    const int *act, cudaStream_t st, bool real = false) {
   int Mp, Np, Kp, mtiles, ntiles, kblocks;
@@ -1508,28 +1681,28 @@ static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int
   if (side == 0) {
     dim3 ga((n + 31) / 32, items);
     kstat_begin(KS_OTHER, split_bytes, st);
-    k_split_a<S, DB><<<ga, 256, 0, st>>>(M, n, K, nc, act, (__nv_bfloat16 *)sg.p, Mp, Kp, sg.scale);
+    k_split_a<S, DB, H><<<ga, 256, 0, st>>>(M, n, K, nc, act, (__nv_bfloat16 *)sg.p, Mp, Kp, sg.scale);
   } else {
     dim3 gb((n + 7) / 8, items);
     kstat_begin(KS_OTHER, 2.0 * split_bytes, st);
-    k_split_b<S, DB><<<gb, 256, 0, st>>>(M, n, K, nc, act, (__nv_bfloat16 *)sg.p, Np, Kp, sg.scale);
+    k_split_b<S, DB, H><<<gb, 256, 0, st>>>(M, n, K, nc, act, (__nv_bfloat16 *)sg.p, Np, Kp, sg.scale);
   }
   kstat_end(st);
   SKKR_LAUNCHED();
   return 0;
 }
 
-template <int S, int DB, int FB>
+template <int S, int DB, int FB, int H>
 static int oz_launch(const CUtensorMap &ma, const CUtensorMap &mb, const OzArgs &g, cudaStream_t st) {
   const size_t smem = oz_smem_bytes(S, FB > 0);
   static const cudaError_t set =  // once per process (thread-safe static initialisation)
-      cudaFuncSetAttribute(k_ozaki<S, DB, FB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_ozaki<S, DB, FB, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (set != cudaSuccess) return SKKR_ERR_CUDA;
-  k_ozaki<S, DB, FB><<<std::min(g.tiles, sm_count()), oz_threads(S), smem, st>>>(ma, mb, g);
+  k_ozaki<S, DB, FB, H><<<std::min(g.tiles, sm_count()), oz_threads(S), smem, st>>>(ma, mb, g);
   return 0;
 }
 
-template <int S, int DB>
+template <int S, int DB, int H>
 static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const MatRef &D, const MatRef &E,
                   int n, int K, int nk, int nc, const int *act, cudaStream_t st) {
   if (get_encoder()) return SKKR_ERR_CUDA;
@@ -1547,7 +1720,7 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   // whose strides no tensor map takes
   if (B.fused && (mref_overlap(B.src, C, nk, nc, n) || mref_overlap(B.src, D, nk, nc, n) ||
                   mref_overlap(B.src, E, nk, nc, n) || !make_raw_map(&mb, B.src, n, K, nk, nc))) {
-    const int rc = split_s<S, DB>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
+    const int rc = split_s<S, DB, H>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
     if (rc) return rc;
   }
   if (make_map(&ma, A.p, Mp, items * S * kblocks, MT)) return SKKR_ERR_CUDA;
@@ -1574,26 +1747,29 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   kstat_begin2(KS_OZAKI, (double)(S * (S + 1) / 2) * 8.0 * n * (double)n * K * (double)active,
                8.0 * n * (double)n * K * (double)active, st);
   g.tiles = (int)(items * mtiles * ntiles);
-  const int rc = B.fused ? oz_launch<S, DB, 1>(ma, mb, g, st) : oz_launch<S, DB, 0>(ma, mb, g, st);
+  const int rc = B.fused ? oz_launch<S, DB, 1, H>(ma, mb, g, st) : oz_launch<S, DB, 0, H>(ma, mb, g, st);
   kstat_end(st);
   if (rc) return rc;
   SKKR_LAUNCHED();
   return 0;
 }
 
-// f<S, DB>(...) for S = 3..8 and the digit base of the depth
-#define OZ_DISPATCH(S, K, f, ...)                                    \
-  do {                                                               \
-    const bool d8 = oz_digits(K) == 8;                               \
-    switch (S) {                                                     \
-      case 3: return d8 ? f<3, 8>(__VA_ARGS__) : f<3, 7>(__VA_ARGS__); \
-      case 4: return d8 ? f<4, 8>(__VA_ARGS__) : f<4, 7>(__VA_ARGS__); \
-      case 5: return d8 ? f<5, 8>(__VA_ARGS__) : f<5, 7>(__VA_ARGS__); \
-      case 6: return d8 ? f<6, 8>(__VA_ARGS__) : f<6, 7>(__VA_ARGS__); \
-      case 7: return d8 ? f<7, 8>(__VA_ARGS__) : f<7, 7>(__VA_ARGS__); \
-      case 8: return d8 ? f<8, 8>(__VA_ARGS__) : f<8, 7>(__VA_ARGS__); \
-      default: return SKKR_ERR_ARG;                                  \
-    }                                                                \
+// f<S, DB, H>(...) for S = 3..8, the digit base of the depth and the form of the size
+#define OZ_CASE(S, f, ...)                                                      \
+  case S:                                                                       \
+    return stacked ? f<S, 8, 1>(__VA_ARGS__) : d8 ? f<S, 8, 0>(__VA_ARGS__) : f<S, 7, 0>(__VA_ARGS__);
+#define OZ_DISPATCH(S, n, K, f, ...)                                            \
+  do {                                                                          \
+    const bool d8 = oz_digits(K) == 8, stacked = oz_stacked(n, K);              \
+    switch (S) {                                                                \
+      OZ_CASE(3, f, __VA_ARGS__)                                                \
+      OZ_CASE(4, f, __VA_ARGS__)                                                \
+      OZ_CASE(5, f, __VA_ARGS__)                                                \
+      OZ_CASE(6, f, __VA_ARGS__)                                                \
+      OZ_CASE(7, f, __VA_ARGS__)                                                \
+      OZ_CASE(8, f, __VA_ARGS__)                                                \
+      default: return SKKR_ERR_ARG;                                             \
+    }                                                                           \
   } while (0)
 
 int mixed_split(MixedWork *w, int side, int slot, int S, const MatRef &M, int n, int K, int nk, int nc,
@@ -1601,13 +1777,13 @@ int mixed_split(MixedWork *w, int side, int slot, int S, const MatRef &M, int n,
   if (n < 1 || n > 256 || K < 1 || K > 256 || nk * (long long)nc > 65535 || slot < 0 ||
       slot >= MIXED_SLOTS || (side != 0 && side != 1))
     return SKKR_ERR_ARG;
-  OZ_DISPATCH(S, K, split_s, w, side, slot, M, n, K, nk, nc, act, st, reused);
+  OZ_DISPATCH(S, n, K, split_s, w, side, slot, M, n, K, nk, nc, act, st, reused);
 }
 
 int mixed_gemm_staged(MixedWork *w, int mode, int S, int sa, int sb, const MatRef &C, const MatRef &D,
                       const MatRef &E, int n, int K, int nk, int nc, const int *act, cudaStream_t st) {
   if (sa < 0 || sa >= MIXED_SLOTS || sb < 0 || sb >= MIXED_SLOTS) return SKKR_ERR_ARG;
-  OZ_DISPATCH(S, K, gemm_s, w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
+  OZ_DISPATCH(S, n, K, gemm_s, w, mode, sa, sb, C, D, E, n, K, nk, nc, act, st);
 }
 
 int mixed_zgemm_k(MixedWork *w, int mode, int S, const MatRef &A, const MatRef &B, const MatRef &C,
