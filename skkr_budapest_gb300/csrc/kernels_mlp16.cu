@@ -46,7 +46,8 @@ __device__ __forceinline__ void fma2(unsigned long long &c, unsigned long long a
 // shared tile feeds sixteen multiply-adds, done as packed pairs of columns, and
 // the next k step's tiles are loaded while this one is multiplied.  Bound by
 // the FP32 pipe and shared-memory reads; 4096 x 256 by 256 x 256: 52.8 us with
-// strided scalar reads and no prefetch.
+// strided scalar reads and no prefetch, 34 now.  (Taken back for no gain: 128 x
+// 64 tiles of 8 x 4 outputs a thread, k steps of 32.)
 template <typename TB>
 __global__ void __launch_bounds__(GT) k_gemm32(const float *__restrict__ A, long long sam, long long sak,
                                                const TB *__restrict__ B, long long sbk, long long sbn, int M, int N,
@@ -130,13 +131,13 @@ __global__ void k_split_reduce(const float *__restrict__ part, int nsplit, long 
 }
 
 // db[j] = sum_r dZ[r][j], rows in order: 32 columns per block; eight warps bring
-// 256 rows at a time into shared memory, the next ones on their way while one
-// warp adds (a column's additions stay one chain in row order; reading rows
-// one by one in that chain, one or two blocks in all, took 355 us at
-// 4096 x 256).
-constexpr int CS_ROWS = 256;
-__global__ void __launch_bounds__(256) k_colsum(const float *__restrict__ dZ, int n, int dout, float *__restrict__ db) {
-  __shared__ float sh[CS_ROWS][32];
+// 256 rows at a time into one of two shared buffers, two steps ahead of the
+// ninth warp, which adds (a column's additions stay one chain in row order:
+// 4096 dependent additions are 8 us).  4096 x 256: 355 us with rows read one
+// by one in that chain, 41 with one buffer and the adder among the loaders, 21 now.
+constexpr int CS_ROWS = 256, CS_BYTES = 2 * CS_ROWS * 32 * (int)sizeof(float);
+__global__ void __launch_bounds__(288) k_colsum(const float *__restrict__ dZ, int n, int dout, float *__restrict__ db) {
+  extern __shared__ float cs_sh[];  // [2][CS_ROWS][32]
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, j = blockIdx.x * 32 + tx;
   float v[CS_ROWS / 8], s = 0.f;
   auto fetch = [&](int r0) {
@@ -146,20 +147,34 @@ __global__ void __launch_bounds__(256) k_colsum(const float *__restrict__ dZ, in
       v[q] = (r < n && j < dout) ? dZ[(long long)r * dout + j] : 0.f;
     }
   };
-  fetch(0);
-  for (int r0 = 0; r0 < n; r0 += CS_ROWS) {
+  auto put = [&](int c) {
 #pragma unroll
-    for (int q = 0; q < CS_ROWS / 8; q++) sh[ty + 8 * q][tx] = v[q];
-    __syncthreads();
-    if (r0 + CS_ROWS < n) fetch(r0 + CS_ROWS);
-    if (ty == 0) {
-      const int rows = min(CS_ROWS, n - r0);
-#pragma unroll 16
-      for (int q = 0; q < rows; q++) s += sh[q][tx];
+    for (int q = 0; q < CS_ROWS / 8; q++) cs_sh[((c & 1) * CS_ROWS + ty + 8 * q) * 32 + tx] = v[q];
+  };
+  const int nc = (n + CS_ROWS - 1) / CS_ROWS;
+  if (ty < 8) {
+    fetch(0);
+    put(0);
+    fetch(CS_ROWS);
+  }
+  __syncthreads();
+  for (int c = 0; c < nc; c++) {
+    if (ty == 8) {
+      const float *p = cs_sh + (c & 1) * CS_ROWS * 32 + tx;
+      const int rows = min(CS_ROWS, n - c * CS_ROWS);
+      if (rows == CS_ROWS) {
+#pragma unroll 32
+        for (int q = 0; q < CS_ROWS; q++) s += p[q * 32];
+      } else {
+        for (int q = 0; q < rows; q++) s += p[q * 32];
+      }
+    } else if (c + 1 < nc) {
+      put(c + 1);
+      fetch((c + 2) * CS_ROWS);
     }
     __syncthreads();
   }
-  if (ty == 0 && j < dout) db[j] = s;
+  if (ty == 8 && j < dout) db[j] = s;
 }
 
 // per row: squared error over the outputs on rows with sel[r] == want (sel
@@ -280,7 +295,10 @@ void mlp16_wgrad(const float *H, const float *dZ, int n, int din, int dout, floa
   const int nz = (n + kchunk - 1) / kchunk;
   k_split_reduce<<<grid1((long long)din * dout), 256, 0, st>>>(part, nz, (long long)din * dout, g);
   SKKR_LAUNCHED();
-  k_colsum<<<(dout + 31) / 32, 256, 0, st>>>(dZ, n, dout, g + (long long)din * dout);
+  static const cudaError_t set =  // once per process (thread-safe static initialisation)
+      cudaFuncSetAttribute(k_colsum, cudaFuncAttributeMaxDynamicSharedMemorySize, CS_BYTES);
+  (void)set;  // (a failure shows as the launch's)
+  k_colsum<<<(dout + 31) / 32, 288, CS_BYTES, st>>>(dZ, n, dout, g + (long long)din * dout);
   SKKR_LAUNCHED();
 }
 
