@@ -532,12 +532,49 @@ __device__ __forceinline__ int oz_raw_passes(const OzArgs &g) {
   return H && g.n > 32 ? 2 : 1;
 }
 
+// Scale exponents of the columns c0 .. c0 + 7 of B (nj columns from b) over the
+// whole depth: column c0 + lane % 8's in every lane, 0 past the last.
+__device__ __forceinline__ int oz_exps8(const OzArgs &g, const zd *b, int c0, int nj) {
+  const int lane = threadIdx.x & 31;
+  unsigned m[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) m[c] = 0;
+#pragma unroll 1
+  for (int kc = 0; kc < g.K; kc += 128) {
+    // indices past the end repeat the last one: every load is valid and
+    // all of them are in flight together
+    unsigned v[8][8];
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const uint32_t *q = reinterpret_cast<const uint32_t *>(b + min(kc + lane + 32 * e, g.K - 1) +
+                                                               (long long)min(c0 + c, nj - 1) * g.B.ld);
+        v[c][2 * e] = load_u32(q + 1);
+        v[c][2 * e + 1] = load_u32(q + 3);
+      }
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+#pragma unroll
+      for (int e = 0; e < 8; e++) m[c] = max(m[c], v[c][e] & 0x7FFFFFFFu);
+  }
+  int mine = 0;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const unsigned t = __reduce_max_sync(0xffffffffu, m[c]);
+    if ((lane & 7) == c && c0 + c < nj) mine = scale_exp((unsigned long long)t << 32);
+  }
+  return mine;
+}
+
 // The scale role (warp 2, fused B only): the exponents of each tile's 32
 // columns of B over the whole depth K, into the ring the conversion and the
 // epilogue read, with the columns of B two tiles ahead started towards L2.
 // Only the exponent field of a value matters (scale_exp), so the maxima run on
 // the upper words, and only those are loaded (64 loads of a lane in flight:
-// the role's pace is its load latency).  A ring slot of exponents is free
+// the role's pace is its load latency).  The first tile's are the conversion
+// warps' own work, which have nothing else yet: four warps at once (30
+// products of n = 128, one tile an SM, eight slices: 49 -> 44 us).  A ring slot of exponents is free
 // again when the role returns to it: it runs at most four tiles ahead of the
 // conversion, the conversion at most four k-blocks, hence five tiles, ahead of
 // the MMAs, and those wait for the epilogue of the tile oz_bufs before.
@@ -555,7 +592,11 @@ __device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
   prefetch_b(wp);
   wp.step();
   prefetch_b(wp);
-  for (TileWalk w(g); w.valid(); w.step()) {
+  if (wp.valid()) wp.step();
+  prefetch_b(wp);
+  TileWalk w(g);
+  if (w.valid()) w.step();
+  for (; w.valid(); w.step()) {
     const int item = w.item(), j0 = w.nt() * NC, nj = g.n - j0 < NC ? g.n - j0 : NC;
     if (wp.valid()) wp.step();
     prefetch_b(wp);
@@ -565,39 +606,13 @@ __device__ __forceinline__ void oz_scales(const OzArgs &g, OzShared &sh) {
     int mine = 0, mine1 = 0;  // columns lane and 32 + lane
 #pragma unroll 1
     for (int c0 = 0; c0 < nj; c0 += 8) {
-      unsigned m[8];
-#pragma unroll
-      for (int c = 0; c < 8; c++) m[c] = 0;
-#pragma unroll 1
-      for (int kc = 0; kc < g.K; kc += 128) {
-        // indices past the end repeat the last one: every load is valid and
-        // all of them are in flight together
-        unsigned v[8][8];
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const uint32_t *q = reinterpret_cast<const uint32_t *>(b + min(kc + lane + 32 * e, g.K - 1) +
-                                                                   (long long)min(c0 + c, nj - 1) * g.B.ld);
-            v[c][2 * e] = load_u32(q + 1);
-            v[c][2 * e + 1] = load_u32(q + 3);
-          }
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-#pragma unroll
-          for (int e = 0; e < 8; e++) m[c] = max(m[c], v[c][e] & 0x7FFFFFFFu);
-      }
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const unsigned t = __reduce_max_sync(0xffffffffu, m[c]);
-        if (lane == c0 + c && lane < nj) mine = scale_exp((unsigned long long)t << 32);
-        if (H && lane + 32 == c0 + c && lane + 32 < nj) mine1 = scale_exp((unsigned long long)t << 32);
-      }
+      const int e = oz_exps8(g, b, c0, nj);
+      if ((lane & ~7) == (c0 & 31)) (H && c0 >= 32 ? mine1 : mine) = e;
     }
     sh.col_exp[w.i % OZ_EXP_RING][lane] = (short)mine;
     if (H) sh.col_exp[w.i % OZ_EXP_RING][lane + 32] = (short)mine1;
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sh.sc_full[w.i % OZ_SCALE_RING]);
+    if (lane < 4) mbar_arrive(&sh.sc_full[w.i % OZ_SCALE_RING]);  // (as the four conversion warps for the first tile)
   }
 }
 
@@ -620,6 +635,17 @@ __device__ __forceinline__ void oz_convert(const OzArgs &g, OzShared &sh, unsign
   // this thread's 16-byte values in a raw block: box kq / 8, row jl, chunks kq % 8 .. +3 XORed with jl % 8
   const unsigned char *src = raw + (kq >> 3) * (OZ_RAW_BYTES / 2) + jl * 128;
   for (TileWalk w(g); w.valid(); w.step()) {
+    if (w.i == 0 && cw < 4) {  // the first tile's scales: eight columns a warp (and a pass)
+      const int j0 = w.nt() * (H ? NT : NT / 2), nj = min(g.n - j0, H ? NT : NT / 2);
+      const zd *b = mat_ptr(g.B, w.item() / g.nc, w.item() % g.nc) + (long long)j0 * g.B.ld;
+#pragma unroll 1
+      for (int c0 = 8 * cw; c0 < 32 * npass; c0 += 32) {
+        const int e = oz_exps8(g, b, c0, nj);
+        if (lane < 8) sh.col_exp[0][c0 + lane] = (short)e;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.sc_full[0]);
+    }
     if (!oz_warp_wait(sh, &sh.sc_full[w.i % OZ_SCALE_RING], (w.i / OZ_SCALE_RING) & 1)) return;
     for (int kb = cw >> 2; kb < nkb; kb += oz_conv_groups(S)) {
       const int kc = w.i * nkb + kb, st = kc % NB;
@@ -979,7 +1005,7 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_ozaki(const __grid_constan
       mbar_init(&sh.raw_empty[i], 4);
     }
     for (int i = 0; i < OZ_SCALE_RING; i++) {
-      mbar_init(&sh.sc_full[i], 1);
+      mbar_init(&sh.sc_full[i], 4);
       mbar_init(&sh.sc_empty[i], 4 * oz_conv_groups(S));
     }
     for (int i = 0; i < NBUF; i++) {
