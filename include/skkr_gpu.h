@@ -35,6 +35,8 @@ extern "C" {
 /* NONREL: lm basis (nrsp-scf); REL: (kappa,mu) (rsp-scf); BDG: electron
  * (kappa,mu) block then hole block, 4 (lmax+1)^2 per site (skkr_dbogo_bsf) */
 enum skkr_mode { SKKR_NONREL = 0, SKKR_REL = 1, SKKR_BDG = 2 };
+/* SKKR_MIXED: split precision (the accuracy rules of skkr_gpu_set_mixed_policy);
+ * principal layers of up to 27 rows run in FP64 there too, which is faster. */
 enum skkr_precision { SKKR_FP64 = 0, SKKR_MIXED = 1 };
 
 enum skkr_error {

@@ -865,8 +865,17 @@ static int stage_slices(const skkr_ctx *c) {
   return c->sz.precision == SKKR_MIXED ? c->slices_res : WIDE_SLICES;
 }
 
+// Blocks of up to SMALL_ROWS rows run on the FP64 pipe in split-precision
+// contexts too: its kernels follow the size, a sliced product pays a 128-row
+// tile and an inverse eight launches.  506 items, product / inverse in us, FP64
+// against six slices: 18 rows 30 / 71 against 61 / 297, 24 rows 59 / 102
+// against 70 / 307, 27 rows 77 / 184 against 76 / 321, 32 rows 119 / 237 against
+// 76 / 323 (six products and one inverse an iteration).  Energies of the plain
+// interface (18 rows, 253 k): 25.0 -> 59.8 thousand (E, k) points a second.
+constexpr int SMALL_ROWS = 27;
 static bool use_mixed(const skkr_ctx *c, bool decimation) {
   if (c->sz.precision != SKKR_MIXED || c->force_fp64) return false;
+  if (c->n <= SMALL_ROWS) return false;
   // decimation near the real axis stays in FP64 (default: within 2e-4 Ry)
   const bool dec_fp64 = std::fabs(c->ce.y) < c->dec_fp64_im;
   if (decimation && dec_fp64) return false;
