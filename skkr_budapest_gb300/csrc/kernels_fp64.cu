@@ -284,7 +284,8 @@ __global__ void __launch_bounds__(256) k_zgemm(MatRef A, MatRef B, MatRef C, Mat
 // the SMs.  The FP64 pipe bounds both forms (about two multiply-adds a clock
 // per SM): an 18-row block fills 324 of 352 lanes here against 324 of 1024
 // outputs of a 32 x 32 tile, and one 32-row product takes 16 SMs instead of
-// one (36.6 us).  Every output is summed in the same order (same bits).
+// one.  506 products of 18 rows 62 -> 21 us (pipe floor 20), one of 32 rows
+// 36.6 -> 3.  Every output is summed in the same order (same bits).
 constexpr int ZF_ROWS = 64, ZF_K = 32;
 template <int MODE>
 __global__ void __launch_bounds__(256) k_zgemm_flat(MatRef A, MatRef B, MatRef C, MatRef D, MatRef E, int M, int N,
@@ -462,8 +463,8 @@ __device__ __forceinline__ double zmag(zd v, bool far) { return far ? hypot(v.x,
 // one block barrier.  The FP64 pipe bounds it (n^2 complex multiply-adds a
 // step, about half a clock each per SM), so the layouts follow n in steps of
 // eight columns and warps without a row of the matrix only keep the barriers.
-// 506 matrices of 18 rows: 212 us, 24 of 32 rows: 200 us by k_zgj, whose steps
-// take four barriers and pass over global memory.
+// 506 matrices of 18 rows: 212 -> 61 us, 24 of 32 rows: 200 -> 86, against
+// k_zgj, whose steps take four barriers and pass over global memory.
 template <int LW, int TY, int RA, int RB>
 __device__ __forceinline__ void zgj_stage(const zd (&m)[RA][RB], int row, unsigned used, int tx, unsigned gmask,
                                           zd *prow, int *kp_out) {
@@ -692,7 +693,7 @@ void launch_add_tblocks(const MatRef &out, const MatRef &in, const MatRef &t, in
 
 // One block per matrix, a warp per column, eight loads of a lane in flight
 // (one 256-thread block with a division per element: 42 us for any number of
-// 128-row matrices up to one per SM).  The FP64 pipe's two multiply-adds per
+// 128-row matrices up to one per SM; 15 now).  The FP64 pipe's two multiply-adds per
 // element set the floor: 8 us per 128-row matrix and SM.
 __global__ void __launch_bounds__(1024) k_fnorm(MatRef A, int n, int nc, const int *__restrict__ act, double *out) {
   const int item = blockIdx.x;
@@ -889,7 +890,7 @@ void launch_extract_pairs(const MatRef &W, int lk, int nl, int rowlay0, int coll
 // do not depend on the element: the block forms those of 128 k points at a
 // time, one per thread, in shared memory (a sine and cosine per element and k
 // point took 3.97 ms for 192 pairs, 8 operations and 36 k points of 32-row
-// blocks, of which eight FP64 multiply-adds per element are 0.74).
+// blocks, 1.29 now; eight FP64 multiply-adds per element are 0.74).
 constexpr int PAIR_T = 128;
 __global__ void __launch_bounds__(PAIR_T) k_pair_sum(const zd *__restrict__ tauf, int nkc, int nc, int nintfc, int lk2,
                                                      const int *__restrict__ cls_of_g, int ngeff,
