@@ -1027,23 +1027,27 @@ static int run_decimation(skkr_ctx *c, int k0, int nkc, const std::vector<int> &
     MatRef &bc = odd ? b0 : b1, &bn = odd ? b1 : b0;
     CKR(eng_inv(c, mx, eps, y1, false, n, nkc, nc, act));              // y1 = eps^-1
     if (staged) {
-      // tensor-core engines: each operand split once (B slots 1-3: y1,
-      // alfa, beta; A slots 1-4: alfa, beta, P, Q) for the six products
+      // tensor-core engines: U = y1 alfa and V = y1 beta (in P and Q) serve two
+      // products each, so that five operands are split (A slots 1-3: y1,
+      // alfa, beta; B slots 1 and 4: U, V) and alfa and beta enter U and V
+      // unsplit.  By (alfa y1) alfa and so on it were seven splits: energies of
+      // 128 rows 17.5 -> 17.3 ms (210 k), with eight slices 8.6 -> 8.3 (55 k),
+      // 54 rows 26.0 -> 25.6 (820 k); the errors against 64 bits are the same.
       MixedWork *w = c->mw;
       const int S = mx ? slices_for(c) : WIDE_SLICES;
-      CKR(mixed_split(w, 1, 1, S, y1, n, n, nkc, nc, act, st, true));
-      CKR(mixed_split(w, 0, 1, S, ac, n, n, nkc, nc, act, st));
-      CKR(mixed_split(w, 0, 2, S, bc, n, n, nkc, nc, act, st));
-      CKR(mixed_gemm_staged(w, 0, S, 1, 1, P, P, P, n, n, nkc, nc, act, st));        // P = alfa y1
-      CKR(mixed_gemm_staged(w, 0, S, 2, 1, Q, Q, Q, n, n, nkc, nc, act, st));        // Q = beta y1
-      CKR(mixed_split(w, 1, 2, S, ac, n, n, nkc, nc, act, st, true));
-      CKR(mixed_split(w, 1, 3, S, bc, n, n, nkc, nc, act, st, true));
-      CKR(mixed_split(w, 0, 3, S, P, n, n, nkc, nc, act, st));
-      CKR(mixed_split(w, 0, 4, S, Q, n, n, nkc, nc, act, st));
-      CKR(mixed_gemm_staged(w, 0, S, 3, 2, an, an, an, n, n, nkc, nc, act, st));     // alfa' = P alfa
-      CKR(mixed_gemm_staged(w, 0, S, 4, 3, bn, bn, bn, n, n, nkc, nc, act, st));     // beta' = Q beta
-      CKR(mixed_gemm_staged(w, 2, S, 3, 3, P, eps, x, n, n, nkc, nc, act, st));      // eps, x -= P beta
-      CKR(mixed_gemm_staged(w, 1, S, 4, 2, eps, eps, eps, n, n, nkc, nc, act, st));  // eps -= Q alfa
+      CKR(mixed_split(w, 0, 1, S, y1, n, n, nkc, nc, act, st));
+      CKR(mixed_split(w, 1, 2, S, ac, n, n, nkc, nc, act, st));
+      CKR(mixed_split(w, 1, 3, S, bc, n, n, nkc, nc, act, st));
+      CKR(mixed_gemm_staged(w, 0, S, 1, 2, P, P, P, n, n, nkc, nc, act, st));        // U = y1 alfa
+      CKR(mixed_gemm_staged(w, 0, S, 1, 3, Q, Q, Q, n, n, nkc, nc, act, st));        // V = y1 beta
+      CKR(mixed_split(w, 0, 2, S, ac, n, n, nkc, nc, act, st));
+      CKR(mixed_split(w, 0, 3, S, bc, n, n, nkc, nc, act, st));
+      CKR(mixed_split(w, 1, 1, S, P, n, n, nkc, nc, act, st, true));
+      CKR(mixed_split(w, 1, 4, S, Q, n, n, nkc, nc, act, st, true));
+      CKR(mixed_gemm_staged(w, 0, S, 2, 1, an, an, an, n, n, nkc, nc, act, st));     // alfa' = alfa U
+      CKR(mixed_gemm_staged(w, 0, S, 3, 4, bn, bn, bn, n, n, nkc, nc, act, st));     // beta' = beta V
+      CKR(mixed_gemm_staged(w, 2, S, 2, 4, P, eps, x, n, n, nkc, nc, act, st));      // eps, x -= alfa V
+      CKR(mixed_gemm_staged(w, 1, S, 3, 1, eps, eps, eps, n, n, nkc, nc, act, st));  // eps -= beta U
     } else {
       CKR(eng_gemm(c, mx, 0, ac, y1, P, P, P, n, nkc, nc, act));        // P = alfa y1
       CKR(eng_gemm(c, mx, 0, bc, y1, Q, Q, Q, n, nkc, nc, act));        // Q = beta y1
