@@ -489,6 +489,8 @@ extern "C" int skkr_gpu_create(const skkr_sizes *sizes, skkr_ctx **out) {
   return SKKR_OK;
 }
 
+static void phys_pool_trim(int dev);
+
 extern "C" int skkr_gpu_destroy(skkr_ctx *c) {
   if (!c) return SKKR_OK;
   DBuf *all[] = {&c->gR, &c->rvec, &c->rstart, &c->blkmap_d, &c->xk, &c->wk, &c->lg, &c->rg,
@@ -507,6 +509,7 @@ extern "C" int skkr_gpu_destroy(skkr_ctx *c) {
     delete sl;
   }
   if (c->st) cudaStreamDestroy(c->st);
+  phys_pool_trim(c->dev);
   delete c;
   return SKKR_OK;
 }
@@ -2516,16 +2519,24 @@ static int phys_basis(int mode, int lmax, int ld, int *nd, int *nal, std::vector
 // tau <- L tau R (- C for one layer, tinv2 null): every operand in one host
 // block, one copy each way, and the device block from a small pool of the
 // device's (8 cudaMalloc and cudaFree a call cost 0.2 ms, several times the
-// work): at most PHYS_POOL_KEEP bytes stay with it between calls.
+// work): at most PHYS_POOL_KEEP bytes stay with it between calls, until a
+// context of the device is destroyed.
 constexpr unsigned long long PHYS_POOL_KEEP = 4ull << 20;
+static std::mutex g_phys_mu;
+static std::map<int, cudaMemPool_t> g_phys_pools;  // by device
+
+static void phys_pool_trim(int dev) {
+  std::lock_guard<std::mutex> lk(g_phys_mu);
+  auto it = g_phys_pools.find(dev);
+  if (it != g_phys_pools.end()) cudaMemPoolTrimTo(it->second, 0);
+}
+
 static int phys_pool(cudaMemPool_t *pool) {
-  static std::mutex mu;
-  static std::map<int, cudaMemPool_t> pools;
   int dev = 0;
   CK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = pools.find(dev);
-  if (it == pools.end()) {
+  std::lock_guard<std::mutex> lk(g_phys_mu);
+  auto it = g_phys_pools.find(dev);
+  if (it == g_phys_pools.end()) {
     cudaMemPoolProps pr = {};
     pr.allocType = cudaMemAllocationTypePinned;
     pr.location.type = cudaMemLocationTypeDevice;
@@ -2538,7 +2549,7 @@ static int phys_pool(cudaMemPool_t *pool) {
       cudaMemPoolDestroy(p);
       CK(e);
     }
-    it = pools.emplace(dev, p).first;
+    it = g_phys_pools.emplace(dev, p).first;
   }
   *pool = it->second;
   return SKKR_OK;
