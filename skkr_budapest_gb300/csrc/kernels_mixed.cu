@@ -1498,17 +1498,6 @@ size_t oz_smem_bytes(int S, bool fused) {
   return (size_t)oz_ring_bytes(S, fused) + (fused ? (size_t)oz_raw_stages(S) * OZ_RAW_BYTES : 0) + 1024;
 }
 
-int sm_count() {
-  static const int n = []() {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1)
-      return 152;
-    return v;
-  }();
-  return n;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1528,6 +1517,8 @@ struct Stage {
   MatRef src;
 };
 
+constexpr int OZ_FORMS = 6 * 2 * 3;  // k_ozaki's instances: slices, staged or fused B, digit base or stacked
+
 struct MixedWork {
   Stage A[MIXED_SLOTS], B[MIXED_SLOTS];
   zd *acopy = nullptr, *rbuf = nullptr, *big = nullptr;
@@ -1545,6 +1536,11 @@ struct MixedWork {
   unsigned long long *nref = nullptr;  // [0] inverses that took further Newton steps, [1] kernels run by the
                                        // IF bodies of captured further steps (device counts)
   cudaStream_t side = nullptr;         // captures the bodies of conditional graph nodes
+  // of the device this context lives on: its SMs, and which forms of k_ozaki
+  // have had their shared memory limit raised (a kernel's attributes belong to
+  // the device that is current when they are set, and end with its context)
+  int sms = 0;
+  bool smem_set[OZ_FORMS] = {};
   bool fuse_b = true;      // B operands formed inside the product (mixed_set_fused)
 };
 
@@ -1573,11 +1569,14 @@ static int grow(void **p, size_t *cap, size_t bytes, bool zero) {
 MixedWork *mixed_create() {
   std::lock_guard<std::recursive_mutex> lk(skkr_device_mutex());
   MixedWork *w = new MixedWork();
+  int dev = 0;
   if (cudaMalloc(&w->err, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&w->dmax, sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&w->nfb, sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&w->cnt, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&w->nref, 2 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || w->sms < 1 ||
       cudaStreamCreateWithFlags(&w->side, cudaStreamNonBlocking) != cudaSuccess) {
     void *ps[] = {w->err, w->dmax, w->nfb, w->cnt, w->nref};
     for (void *p : ps)
@@ -1719,12 +1718,15 @@ static int split_s(MixedWork *w, int side, int slot, const MatRef &M, int n, int
 }
 
 template <int S, int DB, int FB, int H>
-static int oz_launch(const CUtensorMap &ma, const CUtensorMap &mb, const OzArgs &g, cudaStream_t st) {
+static int oz_launch(MixedWork *w, const CUtensorMap &ma, const CUtensorMap &mb, const OzArgs &g, cudaStream_t st) {
   const size_t smem = oz_smem_bytes(S, FB > 0);
-  static const cudaError_t set =  // once per process (thread-safe static initialisation)
-      cudaFuncSetAttribute(k_ozaki<S, DB, FB, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (set != cudaSuccess) return SKKR_ERR_CUDA;
-  k_ozaki<S, DB, FB, H><<<std::min(g.tiles, sm_count()), oz_threads(S), smem, st>>>(ma, mb, g);
+  bool &set = w->smem_set[((S - 3) * 2 + (FB > 0)) * 3 + (H ? 2 : DB - 7)];
+  if (!set &&
+      cudaFuncSetAttribute(k_ozaki<S, DB, FB, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess)
+    return SKKR_ERR_CUDA;
+  set = true;
+  k_ozaki<S, DB, FB, H><<<std::min(g.tiles, w->sms), oz_threads(S), smem, st>>>(ma, mb, g);
   return 0;
 }
 
@@ -1773,7 +1775,7 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   kstat_begin2(KS_OZAKI, (double)(S * (S + 1) / 2) * 8.0 * n * (double)n * K * (double)active,
                8.0 * n * (double)n * K * (double)active, st);
   g.tiles = (int)(items * mtiles * ntiles);
-  const int rc = B.fused ? oz_launch<S, DB, 1, H>(ma, mb, g, st) : oz_launch<S, DB, 0, H>(ma, mb, g, st);
+  const int rc = B.fused ? oz_launch<S, DB, 1, H>(w, ma, mb, g, st) : oz_launch<S, DB, 0, H>(w, ma, mb, g, st);
   kstat_end(st);
   if (rc) return rc;
   SKKR_LAUNCHED();

@@ -295,9 +295,8 @@ void mlp16_wgrad(const float *H, const float *dZ, int n, int din, int dout, floa
   const int nz = (n + kchunk - 1) / kchunk;
   k_split_reduce<<<grid1((long long)din * dout), 256, 0, st>>>(part, nz, (long long)din * dout, g);
   SKKR_LAUNCHED();
-  static const cudaError_t set =  // once per process (thread-safe static initialisation)
-      cudaFuncSetAttribute(k_colsum, cudaFuncAttributeMaxDynamicSharedMemorySize, CS_BYTES);
-  (void)set;  // (a failure shows as the launch's)
+  // on each call, as the attribute is the current device's (a failure shows as the launch's)
+  cudaFuncSetAttribute(k_colsum, cudaFuncAttributeMaxDynamicSharedMemorySize, CS_BYTES);
   k_colsum<<<(dout + 31) / 32, 288, CS_BYTES, st>>>(dZ, n, dout, g + (long long)din * dout);
   SKKR_LAUNCHED();
 }

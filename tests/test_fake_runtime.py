@@ -1,0 +1,59 @@
+"""The library's host code against a CUDA runtime of the host (harness/
+fake_cudart.cpp, preloaded; CPU): what depends on the device that is current,
+and what a call returns when a kernel reports a failure.  Kernels do not run,
+so nothing here looks at numbers."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from skkr_budapest_gb300 import build, native
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HEAD = """
+import ctypes, dataclasses
+import numpy as np
+from skkr_budapest_gb300 import api, native
+from skkr_budapest_gb300 import workloads as W
+rt = ctypes.CDLL(None)
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    if not os.path.exists(native.LIB_PATH):
+        build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include", "-o", so,
+                    os.path.join(ROOT, "tests", "harness", "fake_cudart.cpp")], check=True)
+
+    def go(code):
+        r = subprocess.run([sys.executable, "-c", HEAD + code], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                           env=dict(os.environ, LD_PRELOAD=so))
+        assert r.returncode == 0 and "done" in r.stdout, (r.stdout[-500:], r.stderr[-2000:])
+    return go
+
+
+@pytest.mark.parametrize("n", [20, 100, 200])  # stacked tiles, 8-bit and 7-bit digits
+def test_products_launch_on_every_device_of_the_process(run, n):
+    run("""
+a = np.ones((2, %d, %d), complex)
+for dev in (0, 1, 0, 2):
+    rt.cudaSetDevice(dev)
+    for s in range(3, 9):
+        native.zgemm_batch(a, a, precision="mixed", slices=s)
+assert rt.fake_launches() > 0
+print("done")
+""" % (n, n))
+
+
+def test_training_launches_on_every_device_of_the_process(run):
+    run("""
+layers = [(np.ones((5, 9), np.float32), np.zeros(9, np.float32))]
+for dev in (0, 1):
+    rt.cudaSetDevice(dev)
+    native.mlp16_train(layers, np.ones((40, 5), np.float32), np.ones((40, 9), np.float32), np.ones(40, np.uint8), 2,
+                       1e-3, 1e-4, eval_every=0)
+print("done")
+""")
