@@ -1586,6 +1586,19 @@ static int redo_dominant_k(skkr_ctx *c, int itcpa, const std::vector<int> &lcls,
   return SKKR_OK;
 }
 
+// A tensor-core kernel whose bounded wait ran out leaves its tiles unwritten
+// and raises the context's error word: the call's results are not returned.
+// (The word is cleared when the next call starts.)
+static int check_waits(skkr_ctx *c) {
+  if (!c->mw || c->err_code != 0) return SKKR_OK;
+  CK(cudaStreamSynchronize(c->st));
+  if (mixed_error_flag(c->mw) != 0) {
+    g_last_error = "tensor-core kernel: bounded wait expired";
+    c->err_code = SKKR_ERR_CUDA;
+  }
+  return SKKR_OK;
+}
+
 // Off-diagonal tau of the interface for cluster embedding
 // (skkr_dbogo_bsf/rsp-scf/cpacoord_ksave.f:638-660, 760-840): one k loop of
 // the staged energy with its current t^-1 -- G(k), decimation, the full
@@ -1711,8 +1724,11 @@ extern "C" int skkr_gpu_tauij(skkr_ctx *c, int npair, const int *pairs, const do
       launch_zgemm(0, T1m, Rm, T2m, T2m, T2m, lk, lk, lk, npair, ng, nullptr, st);
       launch_gsum(T2 + side * accn, ng, lk, npair, T1 + side * accn, st);
     }
-    CKR(get_mats(tau_ij, T1, npair, lk, ld, st));
-    CKR(get_mats(tau_ji, T1 + accn, npair, lk, ld, st));
+    CKR(check_waits(c));
+    if (!c->err_code) {
+      CKR(get_mats(tau_ij, T1, npair, lk, ld, st));
+      CKR(get_mats(tau_ji, T1 + accn, npair, lk, ld, st));
+    }
   }
   CK(cudaStreamSynchronize(st));
   CK(cudaGetLastError());
@@ -1979,13 +1995,7 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   c->inv_refined = 0;
   if (c->sz.precision == SKKR_MIXED)
     CKR(mixed_resid_read(c->mw, &c->max_resid, &c->inv_fallbacks, &c->inv_refined, st));
-  if (c->mw && c->err_code == 0) {
-    int f = mixed_error_flag(c->mw);
-    if (f != 0) {
-      g_last_error = "tensor-core kernel: bounded wait expired";
-      c->err_code = SKKR_ERR_CUDA;
-    }
-  }
+  CKR(check_waits(c));
   CK(cudaEventRecord(ev1, st));
   CK(cudaStreamSynchronize(st));
   CK(cudaGetLastError());

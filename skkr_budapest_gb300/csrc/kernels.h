@@ -133,7 +133,7 @@ int wide_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, bool halves
 // running maximum of the accepted Newton residual norms and the count of
 // inverses redone in FP64 (device scalars), and the count of inverses that
 // took further Newton steps (host): reset asynchronously, read with a
-// stream synchronisation
+// stream synchronisation.  The reset clears the error word (mixed_error_flag) too
 int mixed_resid_reset(MixedWork *w, cudaStream_t st);
 int mixed_resid_read(MixedWork *w, double *out, long long *fallbacks, long long *refined, cudaStream_t st);
 

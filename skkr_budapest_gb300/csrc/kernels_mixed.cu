@@ -1593,7 +1593,8 @@ MixedWork *mixed_create() {
 }
 
 int mixed_resid_reset(MixedWork *w, cudaStream_t st) {
-  return (cudaMemsetAsync(w->dmax, 0, sizeof(unsigned long long), st) == cudaSuccess &&
+  return (cudaMemsetAsync(w->err, 0, sizeof(int), st) == cudaSuccess &&
+          cudaMemsetAsync(w->dmax, 0, sizeof(unsigned long long), st) == cudaSuccess &&
           cudaMemsetAsync(w->nfb, 0, sizeof(unsigned long long), st) == cudaSuccess &&
           cudaMemsetAsync(w->nref, 0, 2 * sizeof(unsigned long long), st) == cudaSuccess)
              ? 0

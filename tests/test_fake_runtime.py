@@ -57,3 +57,27 @@ for dev in (0, 1):
                        1e-3, 1e-4, eval_every=0)
 print("done")
 """)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_an_expired_wait_fails_the_call_it_happened_in(run, precision):
+    """tauij and the energy return the CUDA error and leave the caller's
+    arrays alone; the call after them starts from a clear word."""
+    run("""
+ep = W.energy_problem(dataclasses.replace(W.plain_fcc(nset=1), pl=4), 8)   # 36 rows: tensor-core engines
+ctx = api.Context.for_problem(ep, %r)
+ctx.set_graphs(False)   # (the host runtime has no graphs)
+def tauij():
+    r = ctx.tauij(ep, [(0, 0, 0, 1)], [1.0, 0.0], [0.0, 1.0], np.zeros((ep.nintfc, 2)), np.eye(2).reshape(1, 4)
+                  .repeat(len(ep.lg), 0), check=False)
+    assert not r["tau_ij"].any()
+    return r["status"]
+def energy():
+    return ctx.cpacoord(ep, check=False)["status"]
+for call in (tauij, energy):
+    rt.fake_expire_waits(1)
+    assert call() == -2 and "bounded wait" in native.last_error(), call
+    rt.fake_expire_waits(0)
+    assert tauij() == 0
+print("done")
+""" % precision)
