@@ -1211,14 +1211,6 @@ struct GjShared {
   int sig[N], sinv[N];
 };
 
-// 1/x to an ulp without the branches of the rounded reciprocal (0 and the
-// infinite: NaN, as good a mark of a lost start)
-__device__ __forceinline__ float gj_rcp(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
-}
-
 // Eight Gauss-Jordan steps on the panel of rows i0 .. i0 + 7, column j in this
 // thread.  Each warp proposes the best pivot of its 32 columns together with
 // its column and reciprocal, so that a step takes one barrier of the panel
@@ -1244,7 +1236,7 @@ __device__ __forceinline__ void gj_panel(GjShared<N> &sh, int buf, int i0, int n
     unsigned key = mm >= 0.f ? ((__float_as_uint(mm) | 0x80000000u) & ~127u) | inv : 128u | inv;
     key = used ? 0u : key;
     key = i < n ? key : j == i ? 0xFFFFFF80u | inv : 0u;
-    const float rden = gj_rcp(mm);
+    const float rden = __frcp_rn(mm);
     unsigned kmax = __reduce_max_sync(0xFFFFFFFFu, key);
     ulonglong2(&pc)[PW][GJ_NB / 2 + 1] = sh.pcol[q & 1];
     if (key == kmax && key != 0u) {
