@@ -424,8 +424,14 @@ __device__ __forceinline__ int level_int(uint32_t v, int l) {
 }
 // The weighted sum of the S levels of one output in units of level
 // min(S - 1, 5) (weight 2^(-5 DB) of level 0 at most: 62 bits hold it, as
-// |N_0| <= 2^22); deeper levels are rounded into that unit.  32 x 32 + 64 bit
-// multiply-adds with constant powers of two.
+// |N_0| <= 2^22); seven slices round level 6 into that unit.  Eight, which
+// stand for FP64, keep what the levels 6 and 7 add: the lowest bit tells the
+// unit, 1 for level 6 while the sum stays below 2^55 units of level 5 (it then
+// fits there), 0 for level 5 above, where a double's last place is eight of
+// them.  In level 5's unit throughout, an output far below sigma_i tau_j lost
+// digits that its slices hold: 2^-55 sigma_i tau_j, now 2^-60; 110 products of
+// n = 128 take 67.2 us as before with staged B, 75 for 70 with fused B.  32 x
+// 32 + 64 bit multiply-adds with constant powers of two.
 template <int S, int DB, int W>
 __device__ __forceinline__ long long levels_sum(const uint32_t (&v)[S][W], int t) {
   constexpr int B1 = 1 << DB, B2 = 1 << (2 * DB);
@@ -439,9 +445,15 @@ __device__ __forceinline__ long long levels_sum(const uint32_t (&v)[S][W], int t
     long long lo = (long long)level_int<DB>(v[3][t], 3) * B2 +
                    ((long long)level_int<DB>(v[4][t], 4) * B1 + level_int<DB>(v[5][t], 5));
     if constexpr (S == 7) lo += (level_int<DB>(v[6][t], 6) + B1 / 2) >> DB;
-    if constexpr (S == 8)
-      lo += ((long long)level_int<DB>(v[6][t], 6) * B1 + level_int<DB>(v[7][t], 7) + B2 / 2) >> (2 * DB);
-    return (hi << (3 * DB)) + lo;
+    const long long sum = (hi << (3 * DB)) + lo;
+    if constexpr (S < 8) return sum;
+    // level 6 with level 7 rounded into it; the sum's upper word decides the unit.  (Both
+    // values, then the choice: chosen terms cost twice the spilled registers.)
+    const int low = level_int<DB>(v[6][t], 6) + ((level_int<DB>(v[7][t], 7) + B1 / 2) >> DB);
+    const bool small = (unsigned)((int)(sum >> 32) + (1 << 23) - 1) < (1u << 24) - 2u;
+    const long long fine = (sum << DB) + ((low + 1) | 1);
+    const long long coarse = (sum + ((low + B1) >> DB)) & ~1ll;
+    return small ? fine : coarse;
   }
 }
 // round-to-nearest-even double of a * 2^e from integer operations only (the
@@ -462,6 +474,12 @@ __device__ __forceinline__ double fix_to_double(long long a, int e) {
   r = bx >= 2046 ? 0x7FF0000000000000ull : r;
   r = (a == 0 || bx < 0) ? 0ull : r;
   return __longlong_as_double((long long)(sign | r));
+}
+// levels_sum's value, e the exponent of level min(S - 1, 5)'s unit
+template <int S, int DB>
+__device__ __forceinline__ double level_value(long long a, int e) {
+  if constexpr (S < 8) return fix_to_double(a, e);
+  return fix_to_double(a & ~1ll, e - ((a & 1) ? DB : 0));
 }
 
 // byte offset of bf16 (row r, column t < 32) in a K-major tile of 64-byte rows
@@ -739,7 +757,7 @@ __device__ __forceinline__ void oz_epilogue(const OzArgs &g, OzShared &sh, uint3
     // the level sums in FP64; a row of A or a column of B that holds an infinity or a NaN has no digits
     auto value = [&](long long ar, long long ai, int q) {
       const int tj = ce(q);
-      zd val = make_double2(fix_to_double(ar, erow + tj), fix_to_double(ai, erow + tj));
+      zd val = make_double2(level_value<S, DB>(ar, erow + tj), level_value<S, DB>(ai, erow + tj));
       if (sig == SCALE_NONFINITE || tj == SCALE_NONFINITE) val = make_double2(nan, nan);
       return val;
     };
@@ -884,7 +902,7 @@ __device__ __forceinline__ void oz_epilogue_h(const OzArgs &g, OzShared &sh, uin
       for (int q = 0; q < NO; q++)
         if (q0 + q < nq) {
           const int tj = ce(q0 + q);
-          double val = fix_to_double(acc[(q0 + q) % NA], erow + tj);
+          double val = level_value<S, DB>(acc[(q0 + q) % NA], erow + tj);
           if (sig == SCALE_NONFINITE || tj == SCALE_NONFINITE) val = nan;
           const double unit = part == 0 && row == j0 + q0 + q ? 1.0 : 0.0;
           out[(q0 + q) * old_ld] = mode == 0 ? val : mode == 4 ? unit - val : mode == 5 ? old[q] + val : old[q] - val;
@@ -2135,14 +2153,21 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
 
 // ---------------------------------------------------------------------------
 // FP64 products and inverses on the tensor cores.  Eight slices of eight bits
-// hold a 64-bit fixed-point value per element (exact for every element down
-// to 2^-11 of its row's or column's largest, the others to 2^-64 of it), so a
-// product errs by less than the FP64 pipe's own rounding of its 2K terms.  The
+// hold a 64-bit fixed-point value per element, in units of 2^-63 of its row's
+// (A) or column's (B) scale sigma_i, tau_j (the power of two above its
+// largest), and the slice pairs past level 7 are left out.  An output errs by
+//   2^-53 |C_ij| + 2^-60 sigma_i tau_j
+// at a depth of 128 (the second term as a root mean square over digits;
+// 2^-53 sigma_i tau_j if every digit left out were the largest and of one
+// sign), where FP64's own 2K roundings are relative to sum_k |a_ik| |b_kj|.
+// That sum is of the order of sigma_i tau_j for operands of even scale, and
+// the error is below FP64's; it is far below it where a row's large elements
+// meet a column's small ones, and there the error is above FP64's.  The
 // depth is cut into `halves` above 128, where the level sums would leave
 // FP32's integers, and for BdG blocks (electron-first layout): each half then
 // has its own row and column scales, so that the O(Delta) electron-hole blocks
-// keep their own relative precision beside the diagonal ones.  590 products of n = 128: 8.01 ms on the FP64 pipe (99.5 % of its
-// rate), 0.29 ms here; relative Frobenius error 5e-16 either way.
+// keep their own relative precision beside the diagonal ones.  590 products of
+// n = 128: 8.01 ms on the FP64 pipe (99.5 % of its rate), 0.29 ms here.
 int wide_zgemm(MixedWork *w, int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D,
                const MatRef &E, int n, bool halves, int nk, int nc, const int *act, cudaStream_t st) {
   if (n <= 128 && !halves) return mixed_zgemm(w, mode, WIDE_SLICES, A, B, C, D, E, n, nk, nc, act, st);
