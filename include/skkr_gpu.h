@@ -35,7 +35,10 @@ extern "C" {
 /* NONREL: lm basis (nrsp-scf); REL: (kappa,mu) (rsp-scf); BDG: electron
  * (kappa,mu) block then hole block, 4 (lmax+1)^2 per site (skkr_dbogo_bsf) */
 enum skkr_mode { SKKR_NONREL = 0, SKKR_REL = 1, SKKR_BDG = 2 };
-/* SKKR_MIXED: split precision (the accuracy rules of skkr_gpu_set_mixed_policy);
+/* SKKR_FP64: FP64 throughout.  Principal layers above 32 rows run on the tensor
+ * cores with eight BF16 slices per operand where their scales allow it
+ * (skkr_gpu_set_fp64_pipe).
+ * SKKR_MIXED: split precision (the accuracy rules of skkr_gpu_set_mixed_policy);
  * principal layers of up to 27 rows run in FP64 there too, which is faster. */
 enum skkr_precision { SKKR_FP64 = 0, SKKR_MIXED = 1 };
 
@@ -138,6 +141,19 @@ int skkr_gpu_destroy(skkr_ctx *ctx);
  * the tau2d products alone does not repay the splits and the peak redo. */
 int skkr_gpu_set_mixed_policy(skkr_ctx *ctx, double dec_fp64_im, double near_im, int slices_near,
                               double dominant_frac);
+
+/* FP64 arithmetic above 32 rows: FP64 contexts and the FP64 parts of
+ * split-precision ones (decimation near the axis, peaks redone).  on = 0 (the
+ * default): products and inverses on the tensor cores, eight BF16 slices per
+ * operand (64-bit fixed point, exact sums).  An element of a product C = A B
+ * then errs by 2^-53 |C_ij| + 2^-60 sigma_i tau_j (root mean square at a depth
+ * of 128), with sigma_i, tau_j the largest elements of A's row and B's column,
+ * instead of the roundings of its terms; a phase whose diagonal blocks
+ * t^-1 - G have rows or columns that spread over more than 2^9 (strongly
+ * graded channels), where that would cost digits, runs on the FP64 pipe by
+ * itself.  on != 0: the FP64 pipe (IEEE multiply-adds, Gauss-Jordan
+ * elimination) always, some five to ten times slower. */
+int skkr_gpu_set_fp64_pipe(skkr_ctx *ctx, int on);
 
 /* Standard Newton steps X += X (I - A X) after the FP32 Gauss-Jordan start of
  * every split-precision inverse (1..3, default 2).  The acceptance test is

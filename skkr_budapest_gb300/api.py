@@ -71,6 +71,12 @@ class Context:
         result bit for bit (skkr_gpu_set_fused_split)."""
         N._check(N.lib().skkr_gpu_set_fused_split(self.h, 1 if on else 0), "skkr_gpu_set_fused_split")
 
+    def set_fp64_pipe(self, on=True):
+        """FP64 arithmetic above 32 rows on the FP64 pipe always, instead of
+        on the tensor cores where the blocks' scales allow it
+        (skkr_gpu_set_fp64_pipe)."""
+        N._check(N.lib().skkr_gpu_set_fp64_pipe(self.h, 1 if on else 0), "skkr_gpu_set_fp64_pipe")
+
     def set_graphs(self, on=True):
         """Decimation loop as one CUDA graph launch per k chunk (the default)
         or one host-driven iteration at a time (skkr_gpu_set_graphs)."""

@@ -372,6 +372,9 @@ struct skkr_ctx {
   int slices_near = 7;
   double dominant_frac = 1.0e-2; // k points carrying more of |sum_k tau_k| are redone in FP64
   bool force_fp64 = false;       // set while such a k point is redone
+  bool fp64_pipe = false;        // FP64 parts on the FP64 pipe at any size (skkr_gpu_set_fp64_pipe)
+  bool pipe = false;             // the same for the phase that runs (choose_engine)
+  DBuf spread;                   // [0] spread of the diagonal blocks of a phase
   DBuf knorm;                    // [nk] norms of the k-resolved tau contributions
   long long k_fp64 = 0;          // k points redone in FP64 in this run
   skkr_reduce_fn red_fn = nullptr;  // host allreduce of tauc for a k-split energy
@@ -497,7 +500,7 @@ extern "C" int skkr_gpu_destroy(skkr_ctx *c) {
                  &c->conc, &c->tcat, &c->tab, &c->trot, &c->trtmp, &c->pnorm, &c->G, &c->sspo,
                  &c->pool, &c->jobs, &c->dec, &c->decf, &c->deci, &c->tauw, &c->tauk, &c->S,
                  &c->T1, &c->T2, &c->tauc, &c->cpa, &c->cpan, &c->cpaact, &c->decctl, &c->knorm,
-                 &c->redd};
+                 &c->redd, &c->spread};
   for (DBuf *b : all) b->release();
   c->kd.release();
   c->kblk.release();
@@ -808,7 +811,19 @@ static int check_slot_quirk(const skkr_ctx *c) {
 // / inverse in us, pipe against tensor cores: 27 rows 167 / 362 against 162 /
 // 598, 36 rows 385 / 893 against 218 / 794.
 constexpr int WIDE_ROWS = 32;
-static bool wide_engine(const skkr_ctx *c) { return c->n > WIDE_ROWS && c->mw != nullptr; }
+// Their error is relative to the largest elements of an operand's rows and
+// columns, FP64's to the terms of each sum: the same for blocks of even scale,
+// not where the rows of t^-1 + G grow steeply with l and those of its inverse
+// shrink with them.  Blocks whose rows or columns spread over more than
+// 2^WIDE_SPREAD stay on the FP64 pipe (choose_engine).  Restated on the host
+// with the f (d) channel of t^-1 scaled up, errors of tau against long double,
+// eight slices / FP64 elimination: the whole tau 1.2e-16 ... 1.3e-15 / 5e-16
+// ... 4e-15 at any spread; the median element, spread 2^5 4.4e-16 / 8.6e-16,
+// 2^8.8 8.6e-16 / 1.5e-15 (128 rows) and 2.0e-15 / 7e-16 (54 rows, the worst
+// system), 2^10 3.2e-15 / 7.5e-16, 2^15 6e-14 / 7e-16.  The package's systems
+// lie between 2^2 and 2^8.6.
+constexpr int WIDE_SPREAD = 9;
+static bool wide_engine(const skkr_ctx *c) { return c->n > WIDE_ROWS && c->mw != nullptr && !c->pipe; }
 
 // electron-first principal-layer layout: BdG on the tensor-core engines
 static int ehsplit(const skkr_ctx *c) {
@@ -862,6 +877,24 @@ static int eng_inv(skkr_ctx *c, bool mixed, const MatRef &A, const MatRef &X, bo
   }
   if (!inplace) launch_zaxpby(X, A, nullptr, 0, nullptr, 0, n, nk, nc, act, c->st);
   launch_zgj(X, n, nk, nc, act, c->st);
+  return SKKR_OK;
+}
+
+// The engine of a phase in FP64 (decimation or tau2d of a chunk of k points) by
+// its diagonal blocks: measure(launch) calls launch(blocks, nk, nc) for them.
+// One read of the blocks and one synchronisation (rel 128 rows, 55 k: 0.1 of
+// 8.6 ms).
+template <class Measure>
+static int choose_engine(skkr_ctx *c, bool mixed, const Measure &measure) {
+  c->pipe = c->fp64_pipe;
+  if (mixed || !wide_engine(c)) return SKKR_OK;
+  unsigned far = 0;
+  CKR(c->spread.ensure(sizeof(far)));
+  CK(cudaMemsetAsync(c->spread.p, 0, sizeof(far), c->st));
+  measure([&](const MatRef &m, int nk, int nc) { launch_spread(m, c->n, nk, nc, c->spread.as<unsigned>(), c->st); });
+  CK(cudaMemcpyAsync(&far, c->spread.p, sizeof(far), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  c->pipe = far > (unsigned)WIDE_SPREAD << 20;
   return SKKR_OK;
 }
 
@@ -1020,6 +1053,7 @@ static int run_decimation(skkr_ctx *c, int k0, int nkc, const std::vector<int> &
   }
   const int itermax = std::max(c->sz.itermaxl, c->sz.itermaxr);
   const bool mx = use_mixed(c, true);
+  CKR(choose_engine(c, mx, [&](auto &&spread) { spread(eps, nkc, nc); }));
   // products by whole operands of one depth: split each operand once
   const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
   // products by the two halves of the depth (as eng_gemm runs them)
@@ -1214,6 +1248,21 @@ static int tau2d_sweeps(skkr_ctx *c, int k0, int nkc, const std::vector<int> &ic
   launch_zaxpby(pair(YY(0), -1), Ys, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
   launch_zaxpby(pair(XX(nprc - 1), -1), Xs, nullptr, 0, nullptr, 0, n, nkc, nc, nullptr, st);
   const bool mx = use_mixed(c, false);
+  // the diagonal blocks of several PLs per batch: at most as many classes as
+  // the chunk size and the split staging count on
+  const int group = std::max(1, std::min(nprc, 2 * c->ngeff / nc));
+  auto many = [&](int b0, int np) {  // class q nc + s: buffer b0 + q of class s
+    int map[SKKR_MAPN];
+    for (int q = 0; q < np; q++)
+      for (int s = 0; s < nc; s++) map[q * nc + s] = s * nbuf + b0 + q;
+    return mref_map(Wb, (long long)nc * nbuf * MB, MB, n, map, np * nc);
+  };
+  CKR(choose_engine(c, mx, [&](auto &&spread) {
+    for (int p = 0; p < nprc; p += group) {
+      const int np = std::min(group, nprc - p);
+      spread(many(T00(p), np), nkc, np * nc);
+    }
+  }));
   // tensor-core engines: the pairs (M10, M01) on the left and (M01, M10) on
   // the right enter every step, so they are split once (A slot 1, B slot 1);
   // the per-step operands use slot 2
@@ -1249,18 +1298,10 @@ static int tau2d_sweeps(skkr_ctx *c, int k0, int nkc, const std::vector<int> &ic
       CKR(eng_gemm(c, mx, 0, vm, Mr, o, o, o, n, nkc, nc2, nullptr));
     }
   }
-  // tau(p,p) = (T00 - XX - YY)^-1, several PLs per batch: at most as many
-  // classes as the chunk size and the split staging count on
-  const int group = std::max(1, std::min(nprc, 2 * c->ngeff / nc));
+  // tau(p,p) = (T00 - XX - YY)^-1
   for (int p0 = 0; p0 < nprc; p0 += group) {
     const int np = std::min(group, nprc - p0), ng = np * nc;
-    auto many = [&](int b0) {  // class q nc + s: buffer b0 + q of class s
-      int map[SKKR_MAPN];
-      for (int q = 0; q < np; q++)
-        for (int s = 0; s < nc; s++) map[q * nc + s] = s * nbuf + b0 + q;
-      return mref_map(Wb, (long long)nc * nbuf * MB, MB, n, map, ng);
-    };
-    const MatRef t = many(T00(p0)), xx = many(XX(p0)), yy = many(YY(p0));
+    const MatRef t = many(T00(p0), np), xx = many(XX(p0), np), yy = many(YY(p0), np);
     launch_zaxpby(t, t, &xx, -1.0, &yy, -1.0, n, nkc, ng, nullptr, st);
     CKR(eng_inv(c, mx, t, xx, false, n, nkc, ng, nullptr));
   }
@@ -1776,6 +1817,12 @@ extern "C" int skkr_gpu_set_inverse_start(skkr_ctx *c, int) { return c ? SKKR_OK
 extern "C" int skkr_gpu_set_fused_split(skkr_ctx *c, int on) {
   if (!c) return SKKR_ERR_ARG;
   c->fused_b = on != 0;
+  return SKKR_OK;
+}
+
+extern "C" int skkr_gpu_set_fp64_pipe(skkr_ctx *c, int on) {
+  if (!c) return SKKR_ERR_ARG;
+  c->fp64_pipe = on != 0;
   return SKKR_OK;
 }
 

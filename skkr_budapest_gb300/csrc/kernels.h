@@ -38,6 +38,11 @@ void launch_add_tblocks(const MatRef &out, const MatRef &in, const MatRef &t, in
 // Frobenius norms of items -> out[k*nc+c]
 void launch_fnorm(const MatRef &a, int n, int nk, int nc, const int *act, double *out,
                   cudaStream_t st);
+// *out = max(*out, spread) over items: how far the largest elements of the rows
+// (or of the columns) of a matrix lie apart, in 2^-20 of a factor of two;
+// n <= SPREAD_ROWS
+constexpr int SPREAD_ROWS = 256;
+void launch_spread(const MatRef &a, int n, int nk, int nc, unsigned *out, cudaStream_t st);
 // decimation state update (surfgf.f:81-96)
 void launch_dec_state(const double *err, int *act, int *stat, int *iters, int nitems, int iter,
                       int itermax, double errmax, cudaStream_t st);

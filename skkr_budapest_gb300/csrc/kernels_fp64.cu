@@ -730,6 +730,58 @@ void launch_fnorm(const MatRef &a, int n, int nk, int nc, const int *act, double
   SKKR_LAUNCHED();
 }
 
+// How far the rows, and the columns, of a matrix spread: the ratio of the
+// largest to the smallest of their largest elements, as the difference of the
+// doubles' upper words (2^20 a factor of two, linear in between; a zero row or a
+// NaN counts as far), the largest over the items.  One block per matrix, a
+// warp per column, a lane's row maxima in registers: one read of the matrix
+// (55 matrices of 128 rows from DRAM 12 us, 30 of 256 rows 28).
+__global__ void __launch_bounds__(1024) k_spread(MatRef A, int n, int nc, unsigned *out) {
+  constexpr int RL = SPREAD_ROWS / 32;
+  __shared__ unsigned rmax[SPREAD_ROWS], cmax[SPREAD_ROWS];
+  const int item = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const zd *a = mat_ptr(A, item / nc, item % nc);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) rmax[i] = 0u;
+  __syncthreads();
+  unsigned r[RL];
+#pragma unroll
+  for (int i = 0; i < RL; i++) r[i] = 0u;
+  for (int c = w; c < n; c += nw) {
+    unsigned m = 0u;
+#pragma unroll
+    for (int i = 0; i < RL; i++)
+      if (lane + 32 * i < n) {
+        const zd v = a[lane + 32 * i + (long long)c * A.ld];
+        const unsigned h = max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
+        r[i] = max(r[i], h);
+        m = max(m, h);
+      }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) cmax[c] = m;
+  }
+#pragma unroll
+  for (int i = 0; i < RL; i++)
+    if (lane + 32 * i < n) atomicMax(&rmax[lane + 32 * i], r[i]);
+  __syncthreads();
+  if (w < 2) {  // warp 0 the rows, warp 1 the columns
+    const unsigned *p = w ? cmax : rmax;
+    unsigned lo = 0xFFFFFFFFu, hi = 0u;
+    for (int i = lane; i < n; i += 32) {
+      lo = min(lo, p[i]);
+      hi = max(hi, p[i]);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) atomicMax(out, hi >= 0x7FF00000u ? 0xFFFFFFFFu : hi - lo);
+  }
+}
+
+void launch_spread(const MatRef &a, int n, int nk, int nc, unsigned *out, cudaStream_t st) {
+  if (nk <= 0 || nc <= 0 || n <= 0) return;
+  k_spread<<<nk * nc, 32 * std::min(32, std::max(2, n)), 0, st>>>(a, n, nc, out);
+  SKKR_LAUNCHED();
+}
+
 // surfgf.f:81-104: stop when err < errmax or iter > itermax; error > 1e10
 // is "enormous"; leaving with iter > itermax is the itermax failure.
 __global__ void k_dec_state(const double *err, int *act, int *stat, int *iters, int nitems, int iter,

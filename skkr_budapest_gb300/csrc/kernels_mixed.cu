@@ -2162,7 +2162,8 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
 // sign), where FP64's own 2K roundings are relative to sum_k |a_ik| |b_kj|.
 // That sum is of the order of sigma_i tau_j for operands of even scale, and
 // the error is below FP64's; it is far below it where a row's large elements
-// meet a column's small ones, and there the error is above FP64's.  The
+// meet a column's small ones, and there the error is above FP64's: callers
+// keep strongly graded blocks on the FP64 pipe (choose_engine in capi.cu).  The
 // depth is cut into `halves` above 128, where the level sums would leave
 // FP32's integers, and for BdG blocks (electron-first layout): each half then
 // has its own row and column scales, so that the O(Delta) electron-hole blocks
