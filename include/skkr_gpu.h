@@ -100,14 +100,15 @@ typedef struct {
   int max_dec_iters;          /* largest decimation iteration count */
   long long dec_iters_total;  /* summed decimation iterations */
   long long gpu_launches;     /* kernels launched by this call */
-  double max_refine_resid;    /* mixed precision: largest accepted Newton residual |I - AX|_F
-                                 (before the last correction) */
+  double max_refine_resid;    /* inverses on the tensor cores (mixed precision, FP64 above 32 rows):
+                                 largest accepted Newton residual |I - AX|_F (before the last
+                                 correction; at most 1e-6, FP64 1e-9) */
   double run_ms;              /* device time of the call (CUDA events on the library stream) */
-  long long inv_fallbacks;    /* mixed precision: inverses whose residual stayed above 1e-6
-                                 and were redone in FP64 */
+  long long inv_fallbacks;    /* of those, inverses whose residual stayed above that and were
+                                 redone by the FP64 elimination */
   long long k_fp64;           /* mixed precision: k points redone in FP64 (dominant contributions) */
-  long long inv_refined;      /* mixed precision: inverses that took further Newton steps (residual
-                                 above 1e-6 after the standard steps, below 1/2) */
+  long long inv_refined;      /* of those, inverses that took further Newton steps (residual above
+                                 that after the standard steps, below 1/2) */
   double alg_flops;           /* FP64-equivalent algorithmic work of the call in the reference's
                                  operation count, U = 8 n_PL^3 real FLOP per block operation:
                                  (9 it + 3) U per lead decimation of `it` iterations (surfgf.f,

@@ -2040,8 +2040,7 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
   trace_point("after CPA loop");
   c->inv_fallbacks = 0;
   c->inv_refined = 0;
-  if (c->sz.precision == SKKR_MIXED)
-    CKR(mixed_resid_read(c->mw, &c->max_resid, &c->inv_fallbacks, &c->inv_refined, st));
+  if (c->mw) CKR(mixed_resid_read(c->mw, &c->max_resid, &c->inv_fallbacks, &c->inv_refined, st));
   CKR(check_waits(c));
   CK(cudaEventRecord(ev1, st));
   CK(cudaStreamSynchronize(st));
