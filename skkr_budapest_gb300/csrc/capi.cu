@@ -1267,8 +1267,6 @@ static int tau2d_sweeps(skkr_ctx *c, int k0, int nkc, const std::vector<int> &ic
   // the right enter every step, so they are split once (A slot 1, B slot 1);
   // the per-step operands use slot 2
   const bool staged = !ehsplit(c) && (mx || (wide_engine(c) && n <= 128));
-  // products by the two halves of the depth (as eng_gemm runs them)
-  const bool halved = mx ? ehsplit(c) != 0 : wide_engine(c) && (n > 128 || ehsplit(c));
   MixedWork *w = c->mw;
   const int S = mx ? slices_for(c) : WIDE_SLICES, nc2 = 2 * nc;
   const MatRef Ml = pool(c->idx10, c->idx01), Mr = pool(c->idx01, c->idx10);
