@@ -84,9 +84,13 @@ inline MatRef mref_map(zd *base, long long sk, long long sc, int ld, const int *
   return r;
 }
 
-// element range [lo, hi) of an operand's nk x nc items (`cols` columns of at
-// most ld rows each), relative to its base
-inline void mref_span(const MatRef &m, int nk, int nc, int cols, long long *lo, long long *hi) {
+// elements from the first to past the last of `rows` x `cols` (rows 0: all ld)
+inline long long mref_extent(const MatRef &m, int rows, int cols) {
+  return (long long)(cols - 1) * m.ld + (rows > 0 ? rows : m.ld);
+}
+// element range [lo, hi) of an operand's nk x nc items (`cols` columns of
+// `rows` rows each), relative to its base
+inline void mref_span(const MatRef &m, int nk, int nc, int cols, int rows, long long *lo, long long *hi) {
   long long mn = 0, mx = 0;
   for (int c = 0; c < nc && c < SKKR_MAPN; c++) {
     const long long o = (long long)m.map[c] * m.sc;
@@ -95,22 +99,23 @@ inline void mref_span(const MatRef &m, int nk, int nc, int cols, long long *lo, 
   }
   const long long ks = (long long)(nk - 1) * m.sk;
   *lo = mn + std::min(0LL, ks);
-  *hi = mx + std::max(0LL, ks) + (long long)cols * m.ld;
+  *hi = mx + std::max(0LL, ks) + mref_extent(m, rows, cols);
 }
 // whether two operands' items may share an element: no when their ranges
 // are apart; when both sit on the same lattice of item offsets (equal sk, sc
 // and ld, and each item's classes within one sk), exactly when an item of one
-// and an item of the other, of the same or a neighbouring k, are closer than a
-// footprint of cols x ld elements
-inline bool mref_overlap(const MatRef &a, const MatRef &b, int nk, int nc, int cols) {
+// and an item of the other, of the same or a neighbouring k, are closer than
+// the extent of the first of them (cols columns; rows_a, rows_b rows of them,
+// 0: all ld.  A depth half, which starts h rows into its matrix, ends with it)
+inline bool mref_overlap(const MatRef &a, const MatRef &b, int nk, int nc, int cols, int rows_a = 0, int rows_b = 0) {
   long long la, ha, lb, hb;
-  mref_span(a, nk, nc, cols, &la, &ha);
-  mref_span(b, nk, nc, cols, &lb, &hb);
+  mref_span(a, nk, nc, cols, rows_a, &la, &ha);
+  mref_span(b, nk, nc, cols, rows_b, &lb, &hb);
   const uintptr_t a0 = (uintptr_t)(a.base + la), a1 = (uintptr_t)(a.base + ha);
   const uintptr_t b0 = (uintptr_t)(b.base + lb), b1 = (uintptr_t)(b.base + hb);
   if (!(a0 < b1 && b0 < a1)) return false;
   if (a.sk != b.sk || a.sc != b.sc || a.ld != b.ld) return true;
-  const long long fp = (long long)cols * a.ld;
+  const long long fa = mref_extent(a, rows_a, cols), fb = mref_extent(b, rows_b, cols), fp = std::max(fa, fb);
   const long long d = ((long long)(intptr_t)((uintptr_t)b.base - (uintptr_t)a.base)) / (long long)sizeof(zd);
   // distances of item pairs are d + (k2 - k1) sk + (map_b - map_a) sc
   long long lo = 0, hi = 0;
@@ -128,7 +133,7 @@ inline bool mref_overlap(const MatRef &a, const MatRef &b, int nk, int nc, int c
     for (int j = 0; j < nc && j < SKKR_MAPN; j++)
       for (int dk = nk > 1 ? -1 : 0; dk <= (nk > 1 ? 1 : 0); dk++) {
         const long long o = d + dk * sk + (long long)(b.map[j] - a.map[i]) * a.sc;
-        if (o < fp && o > -fp) return true;
+        if (o < fa && o > -fb) return true;
       }
   return false;
 }

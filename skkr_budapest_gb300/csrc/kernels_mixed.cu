@@ -1757,8 +1757,8 @@ static int gemm_s(MixedWork *w, int mode, int sa, int sb, const MatRef &C, const
   // a fused B that the product writes over (C, D or E) is split first, so
   // that no CTA reads an element another one has already replaced; so is one
   // whose strides no tensor map takes
-  if (B.fused && (mref_overlap(B.src, C, nk, nc, n) || mref_overlap(B.src, D, nk, nc, n) ||
-                  mref_overlap(B.src, E, nk, nc, n) || !make_raw_map(&mb, B.src, n, K, nk, nc))) {
+  auto over = [&](const MatRef &out) { return mref_overlap(B.src, out, nk, nc, n, K, n); };
+  if (B.fused && (over(C) || over(D) || over(E) || !make_raw_map(&mb, B.src, n, K, nk, nc))) {
     const int rc = split_s<S, DB, H>(w, 1, sb, B.src, n, K, nk, nc, act, st, true);
     if (rc) return rc;
   }

@@ -14,3 +14,11 @@ extern "C" int overlap_maps_eval(long long offa, const int *mapa, long long offb
              ? 1
              : 0;
 }
+
+// operands of rows_a and rows_b rows, identity maps
+extern "C" int overlap_rows_eval(long long offa, int rows_a, long long offb, int rows_b, long long sk, long long sc,
+                                 int ld, int nk, int nc, int cols) {
+  static zd pool[1];
+  return mref_overlap(mref(pool + offa, sk, sc, ld), mref(pool + offb, sk, sc, ld), nk, nc, cols, rows_a, rows_b) ? 1
+                                                                                                                 : 0;
+}

@@ -1,6 +1,7 @@
 """The aliasing test of the sliced products for operands that pick buffers by
 class maps of their own, as the batched tau2d sweeps do (pairs of buffers,
-several principal layers as classes), against a brute-force intersection
+several principal layers as classes), and for operands of fewer rows than
+their leading dimension (depth halves), against a brute-force intersection
 (CPU)."""
 import ctypes
 import os
@@ -21,9 +22,12 @@ def overlap(tmp_path_factory):
     ll, i, p = ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p
     L.overlap_maps_eval.argtypes = [ll, p, ll, p, ll, ll, i, i, i, i]
 
+    L.overlap_rows_eval.argtypes = [ll, i, ll, i, ll, ll, i, i, i, i]
+
     def go(offa, mapa, offb, mapb, sk, sc, ld, nk, n):
         a, b = (np.ascontiguousarray(m, np.int32) for m in (mapa, mapb))
         return L.overlap_maps_eval(offa, a.ctypes.data, offb, b.ctypes.data, sk, sc, ld, nk, len(a), n)
+    go.rows = L.overlap_rows_eval
     return go
 
 
@@ -71,3 +75,30 @@ def test_never_apart_when_sharing(overlap):
         true = bool(_elems(o1, m1, sk, sc, ld, nk, n) & _elems(o2, m2, sk, sc, ld, nk, n))
         if true:
             assert overlap(o1, m1, o2, m2, sk, sc, ld, nk, n) == 1, (o1, m1, o2, m2, sk, sc, ld, nk, n)
+
+
+def test_depth_halves_end_with_their_matrix(overlap):
+    """The two halves of every buffer of an item against every whole buffer: apart from all but their own, the
+    last buffer's second half from the next item's first buffer too."""
+    n, nbuf, nc, nk = 4, 3, 2, 3
+    MB = n * n
+    for b1 in range(nbuf):
+        for half in (0, n // 2):
+            for b2 in range(nbuf):
+                got = overlap.rows(b1 * MB + half, n // 2, b2 * MB, n, nc * nbuf * MB, nbuf * MB, n, nk, nc, n)
+                assert got == (b1 == b2)
+
+
+def test_row_ranges_are_never_apart_when_sharing(overlap):
+    rng = np.random.default_rng(6)
+    for _ in range(600):
+        n = int(rng.integers(1, 5))
+        ra, rb = (int(rng.integers(1, n + 1)) for _ in range(2))
+        ld = n + int(rng.integers(0, 3))
+        nk, nc = int(rng.integers(1, 4)), int(rng.integers(1, 4))
+        sc, sk = int(rng.integers(0, 2 * n * ld)), int(rng.integers(0, 6 * n * ld))
+        o1, o2 = (int(rng.integers(0, 40)) for _ in range(2))
+        el = [{o + k * sk + c * sc + j * ld + q for k in range(nk) for c in range(nc) for j in range(n) for q in range(r)}
+              for o, r in ((o1, ra), (o2, rb))]
+        if el[0] & el[1]:
+            assert overlap.rows(o1, ra, o2, rb, sk, sc, ld, nk, nc, n) == 1, (o1, ra, o2, rb, sk, sc, ld, nk, nc, n)
