@@ -1996,6 +1996,7 @@ extern "C" int skkr_gpu_run(skkr_ctx *c, skkr_status *status) {
     }
     if (!c->err_code && use_mixed(c, false) && c->dominant_frac > 0.0)
       CKR(redo_dominant_k(c, itcpa, lcls, rcls, icls));
+    if (c->red_fn || c->red_dev_fn) CKR(check_waits(c));  // (before this rank's sum joins the others')
     if (c->err_code) {
       if (c->red_fn || c->red_dev_fn) reduce_tauc(c, true);  // tell the other ranks before returning
       break;

@@ -81,3 +81,24 @@ for call in (tauij, energy):
     assert tauij() == 0
 print("done")
 """ % precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_rank_with_an_expired_wait_tells_the_others(run, precision):
+    """Its sum does not join theirs: the flag goes into the reduction instead."""
+    run("""
+ep = W.energy_problem(dataclasses.replace(W.plain_fcc(nset=1), pl=4), 8)
+ctx = api.Context.for_problem(ep, %r)
+ctx.set_graphs(False)
+flags = []
+def reduce(buf):
+    flags.append(buf[-1])
+ctx.set_reduce(reduce)
+rt.fake_expire_waits(1)
+assert ctx.cpacoord(ep, check=False)["status"] == -2 and flags == [1.0], flags
+rt.fake_expire_waits(0)
+flags.clear()
+ctx.cpacoord(ep, check=False)
+assert flags[0] == 0.0
+print("done")
+""" % precision)
