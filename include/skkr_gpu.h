@@ -150,7 +150,7 @@ int skkr_gpu_set_mixed_policy(skkr_ctx *ctx, double dec_fp64_im, double near_im,
  * then errs by 2^-53 |C_ij| + 2^-60 sigma_i tau_j (root mean square at a depth
  * of 128), with sigma_i, tau_j the largest elements of A's row and B's column,
  * instead of the roundings of its terms; a phase whose diagonal blocks
- * t^-1 - G have rows or columns that spread over more than 2^9 (strongly
+ * t^-1 - G have rows or columns that spread over more than 2^10 (strongly
  * graded channels), where that would cost digits, runs on the FP64 pipe by
  * itself.  on != 0: the FP64 pipe (IEEE multiply-adds, Gauss-Jordan
  * elimination) always, some five to ten times slower. */

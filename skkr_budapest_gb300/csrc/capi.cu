@@ -813,16 +813,16 @@ static int check_slot_quirk(const skkr_ctx *c) {
 constexpr int WIDE_ROWS = 32;
 // Their error is relative to the largest elements of an operand's rows and
 // columns, FP64's to the terms of each sum: the same for blocks of even scale,
-// not where the rows of t^-1 + G grow steeply with l and those of its inverse
+// not where the rows of t^-1 - G grow steeply with l and those of its inverse
 // shrink with them.  Blocks whose rows or columns spread over more than
-// 2^WIDE_SPREAD stay on the FP64 pipe (choose_engine).  Restated on the host
-// with the f (d) channel of t^-1 scaled up, errors of tau against long double,
-// eight slices / FP64 elimination: the whole tau 1.2e-16 ... 1.3e-15 / 5e-16
-// ... 4e-15 at any spread; the median element, spread 2^5 4.4e-16 / 8.6e-16,
-// 2^8.8 8.6e-16 / 1.5e-15 (128 rows) and 2.0e-15 / 7e-16 (54 rows, the worst
-// system), 2^10 3.2e-15 / 7.5e-16, 2^15 6e-14 / 7e-16.  The package's systems
-// lie between 2^2 and 2^8.6.
-constexpr int WIDE_SPREAD = 9;
+// 2^WIDE_SPREAD stay on the FP64 pipe (choose_engine).  Error of tau at single
+// k points of seven systems against long double, the highest channel of t^-1
+// scaled up step by step, slices over pipe: the whole tau 0.8 ... 1.02 at any
+// spread; median element / 90th percentile up to 2^8.6 0.4 ... 1.02 / 0.25 ...
+// 1.0, 2^9.1 ... 2^9.8 (the worst two) 1.06 / 1.13, 2^11 ... 2^12 1.3 / 3.1,
+// 2^15 5 / 41.  The package's systems lie between 2^2 and 2^9.2 (a well near a
+// resonance).
+constexpr int WIDE_SPREAD = 10;
 static bool wide_engine(const skkr_ctx *c) { return c->n > WIDE_ROWS && c->mw != nullptr && !c->pipe; }
 
 // electron-first principal-layer layout: BdG on the tensor-core engines
