@@ -39,7 +39,8 @@ enum skkr_mode { SKKR_NONREL = 0, SKKR_REL = 1, SKKR_BDG = 2 };
  * cores with eight BF16 slices per operand where their scales allow it
  * (skkr_gpu_set_fp64_pipe).
  * SKKR_MIXED: split precision (the accuracy rules of skkr_gpu_set_mixed_policy);
- * principal layers of up to 27 rows run in FP64 there too, which is faster. */
+ * principal layers of up to 27 rows run in FP64 there too, which is faster.
+ * Above 128 rows its inverses run on the FP64 pipe: SKKR_FP64 is faster there. */
 enum skkr_precision { SKKR_FP64 = 0, SKKR_MIXED = 1 };
 
 enum skkr_error {
@@ -152,7 +153,8 @@ int skkr_gpu_set_mixed_policy(skkr_ctx *ctx, double dec_fp64_im, double near_im,
  * instead of the roundings of its terms; a phase whose diagonal blocks
  * t^-1 - G have rows or columns that spread over more than 2^10 (strongly
  * graded channels), where that would cost digits, runs on the FP64 pipe by
- * itself.  on != 0: the FP64 pipe (IEEE multiply-adds, Gauss-Jordan
+ * itself.  Results below the normal range of a double are 0 on the tensor
+ * cores.  on != 0: the FP64 pipe (IEEE multiply-adds, Gauss-Jordan
  * elimination) always, some five to ten times slower. */
 int skkr_gpu_set_fp64_pipe(skkr_ctx *ctx, int on);
 
@@ -172,7 +174,7 @@ int skkr_gpu_set_inverse_start(skkr_ctx *ctx, int blocked);
 
 /* The B operand of every split-precision product: on
  * != 0 (the default) the product reads B in FP64 and forms its BF16 slices in
- * shared memory, tile by tile, with the warps that later run the epilogue; 0
+ * shared memory, tile by tile, by warps of their own; 0
  * splits B into a staging buffer first and loads its tiles by TMA.  Both give
  * the same slices, hence the same result bit for bit. */
 int skkr_gpu_set_fused_split(skkr_ctx *ctx, int on);

@@ -972,9 +972,10 @@ __device__ __forceinline__ void oz_epilogue_h(const OzArgs &g, OzShared &sh, uin
 // arithmetic at half the FP32 rate); fused B, seven slices 391 -> 258 us,
 // three slices 280 -> 164 us (conversion, likewise integer arithmetic);
 // R = I - AX and X += XR of the Newton step 422 + 316 -> 258 + 187 us.
-// More epilogue or conversion warps do not pay where they cost registers: 20
-// warps with 96 registers spill the six-slice epilogue's 64-bit sums (187 ->
-// 244 us); neither does redistributing registers with setmaxnreg (291 us).
+// The 64-bit sums that the epilogue holds from five slices on spill 80 to 170
+// bytes a thread at 128 registers (H = 0).  More epilogue or conversion warps
+// do not pay where they cost registers: 20 warps with 96 spill more (six
+// slices 187 -> 244 us); neither does redistributing registers with setmaxnreg (291 us).
 // Every level p + q has its own accumulator (64 TMEM columns each), so that
 // every level sum stays an exact integer while its bound allows (levels 0..3
 // always), and the slices of B lie side by side in a stage: A_p against up
@@ -2163,12 +2164,14 @@ int mixed_zinv(MixedWork *w, const MatRef &A, const MatRef &X, int n, int nk, in
 // That sum is of the order of sigma_i tau_j for operands of even scale, and
 // the error is below FP64's; it is far below it where a row's large elements
 // meet a column's small ones, and there the error is above FP64's: callers
-// keep strongly graded blocks on the FP64 pipe (choose_engine in capi.cu).  The
+// keep strongly graded blocks on the FP64 pipe (choose_engine in capi.cu).
+// (The sums of levels 4 to 7 leave FP32's exact integers only where nearly all
+// digits are the largest and of one sign, by a unit of that level.)  The
 // depth is cut into `halves` above 128, where the level sums would leave
 // FP32's integers, and for BdG blocks (electron-first layout): each half then
 // has its own row and column scales, so that the O(Delta) electron-hole blocks
 // keep their own relative precision beside the diagonal ones.  590 products of
-// n = 128: 8.01 ms on the FP64 pipe (99.5 % of its rate), 0.29 ms here.
+// n = 128: 8.01 ms on the FP64 pipe (99.5 % of its rate), 0.28 ms staged, 0.30 fused.
 int wide_zgemm(MixedWork *w, int mode, const MatRef &A, const MatRef &B, const MatRef &C, const MatRef &D,
                const MatRef &E, int n, bool halves, int nk, int nc, const int *act, cudaStream_t st) {
   if (n <= 128 && !halves) return mixed_zgemm(w, mode, WIDE_SLICES, A, B, C, D, E, n, nk, nc, act, st);
