@@ -1,8 +1,8 @@
 """B operands formed in the product against staged ones, bit for bit, in
 energies whose block rows are no multiple of 16 and that do run on the tensor
 cores (28 rows and more with split precision, 33 and more in FP64): the
-stacked tiles up to 64 rows and the plain ones above, with the oracle as the
-judge of the numbers."""
+stacked tiles up to 64 rows and the plain ones above; the numbers against the
+oracle."""
 import dataclasses
 
 import numpy as np
